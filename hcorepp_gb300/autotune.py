@@ -6,8 +6,7 @@ Knobs (all schedule / routing choices; results are the same up to rounding order
   wy_min   reflectors a side needs for the tensor-core WY Q application (plain form; hcgb_set_tuning)
   oz_min   outputs a factor product needs to go to the FP64-accurate tensor-core kernel (hcgb_set_tuning)
   graph    the whole multiply captured once as a CUDA graph and replayed (hcgb_set_graph)
-  precond  core columns from which the plain form's core SVD runs FP32 preconditioning sweeps first
-           (hcgb_set_precond)
+  precond  core columns from which the core SVD finds its rotations in FP32 sweeps (hcgb_set_precond)
 
 `tune()` times candidates on the caller's own multiply by coordinate descent (one knob at a time,
 the others at their current best), restoring C before every trial.  `python -m hcorepp_gb300.autotune`
@@ -23,12 +22,12 @@ import os
 import numpy as np
 
 CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning_cache.json")
-DEFAULT = {"groups": 8, "wy_min": 48, "oz_min": 2048, "graph": 0, "precond": 1 << 30}
+DEFAULT = {"groups": 8, "wy_min": 48, "oz_min": 2048, "graph": 0, "precond": 16}
 CANDIDATES = {"groups": [4, 8, 16], "wy_min": [32, 48, 96, 1 << 30], "oz_min": [512, 1024, 2048, 4096],
               "graph": [0, 1], "precond": [16, 32, 64, 1 << 30]}
 ORDER = ["groups", "wy_min", "oz_min", "graph", "precond"]
-# The float-float form applies Q in float-float panels on every side (no WY form) and has no FP32
-# preconditioning, so wy_min and precond do not act on it.
+# The float-float form applies Q in float-float panels on every side (no WY form), so wy_min does not act on
+# it; precond is tuned on the plain form, whose cores it shares.
 FORM_KNOBS = {"mixed_ff48": ["groups", "oz_min", "graph"]}
 
 

@@ -47,12 +47,42 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 // two teams of one CTA never wait for each other.
 template <int NTH>
 struct Team {
-    static constexpr int nth = NTH;
+    static constexpr int nth = NTH, ctas = 1;
     int tid, bar;
     __device__ __forceinline__ int warp() const { return tid >> 5; }
     __device__ __forceinline__ static constexpr int nw() { return NTH >> 5; }
+    __device__ __forceinline__ static constexpr int warps_per_cta() { return NTH >> 5; }
     __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NTH) : "memory"); }
 };
+
+// The NTH threads of each CTA of a thread-block cluster of CTAS as one team: threads are numbered through
+// the cluster and sync() is the cluster's barrier, which also orders their global and distributed
+// shared memory.  rank: this CTA's in the cluster.
+template <int NTH, int CTAS>
+struct ClusterTeam {
+    static constexpr int nth = NTH * CTAS, ctas = CTAS, cta_threads = NTH;
+    int tid, rank;
+    __device__ __forceinline__ int warp() const { return tid >> 5; }
+    __device__ __forceinline__ static constexpr int nw() { return (NTH * CTAS) >> 5; }
+    __device__ __forceinline__ static constexpr int warps_per_cta() { return NTH >> 5; }
+    __device__ __forceinline__ void sync() const {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    }
+};
+
+__device__ __forceinline__ int cluster_rank() {
+    int r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Address, in the generic space, of shared-memory object p of the cluster's CTA `rank`.
+template <class T>
+__device__ __forceinline__ T *cluster_map(T *p, int rank) {
+    T *q;
+    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
+    return q;
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -175,7 +205,7 @@ struct Params {
     int oz;          // 1: large factor products on the 16-bit tensor cores (FP64-accurate splitting)
     int oz_min;      // outputs a product needs to go to the tensor cores (OZ_MIN_OUTPUTS by default)
     int wy_min;      // reflectors a side needs for the WY Q application (WY_MIN_REFLECTORS by default)
-    int precond_min; // plain form: Jacobi columns a core needs for the FP32 preconditioning sweeps
+    int precond_min; // Jacobi columns a core needs for the FP32 preconditioning sweeps
     int sk_pct;      // learned form: sketch an update only when its sketch (with probes) is at most
                      // this percentage of its stack width
 };
@@ -184,10 +214,9 @@ struct Params {
 // which pays for the sketch products and its own QR; wider sketches cost more than they save.
 constexpr int SKETCH_MAX_PCT = 50;
 
-// Default of Params::precond_min: off.  Measured on the 32 x 32-tile nb = 512 multiply, the FP32
-// preconditioning sweeps cut the FP64 sweeps from ~4.7 to ~3 but cost more than they save
-// (918-925 ms per multiply from 16, 32 or 64 core columns on, 844 ms off).
-constexpr int PRECOND_MIN_COLS = 1 << 30;
+// Default of Params::precond_min: a 16-column core is about where the single-precision sweeps and the corrections
+// cost what the FP64 sweeps do (25 columns: 400 kcycles against 930; 15 columns: 250 either way).
+constexpr int PRECOND_MIN_COLS = 16;
 
 // ---- launchers (stream-ordered, asynchronous) ----
 void launch_plan(const DevUpdate *ups, int n, double alpha, double beta, Workspace ws, Params p, GemmJob *jobs,

@@ -5,15 +5,19 @@
 // CompressedTile<T>::Gemm (src/operators/concrete/Compressed.cpp:441-527, :597-599) and the
 // host-synchronising rank scan of the CUDA backend (src/kernels/cuda/CudaKernels.cu:656-697).
 //
-// One team per update (a whole 512-thread CTA for a core that does not fit half the shared
-// memory, else half a CTA).  M = R_U R_V^T on DMMA; Householder QR with column pivoting of M,
+// One team per update: a quarter or half of a CTA, or a cluster of CTAs for a core that does not fit half the
+// shared memory.  M = R_U R_V^T on DMMA; Householder QR with column pivoting of M,
 // stopped once the remaining columns lie far below the truncation threshold; one-sided Jacobi on
-// the rk columns of X = R^T (round-robin parallel ordering, 4-32 lanes per column pair, scaled
-// rotations, tracked norms) until every pair is orthogonal to working precision: X J = W,
-// sigma_j = ||w_j||.  The right factor is XV = P W_r (= V_r Sigma_r) and the left one
-// U = M XV Sigma^-2 (= U_r), so the rotations never need accumulating.  The pivoted QR and the
-// sweeps run in FP64 (plain form) or float-float (mixed form).  The rank rule is the reference's
-// (omp/kernels.cpp:82-104) applied to the sorted sigma.
+// the rk columns of X = R^T until every pair is orthogonal to working precision: X J = W,
+// sigma_j = ||w_j||, found in single precision and finished in FP64 (jacobi_precond; small cores by FP64 sweeps
+// alone).  The right factor is XV = P W_r (= V_r Sigma_r) and the left one U = M XV Sigma^-2 (= U_r).
+// The pivoted QR runs in FP64 (plain form, wide cores) or float-float (mixed form).  The rank rule is the
+// reference's (omp/kernels.cpp:82-104) applied to the sorted sigma.
+//
+// Measured (1.06 TFLOP/s FP64 pipe): the sweeps of a 200-column core of stack width 215 took 72,500 kcycles
+// on one SM, 4,970 on its cluster of eight; of a 25-column core 930, now 400, four to an SM; the pivoted QR
+// 9,970 -> 2,140 and 274 -> 229.
+#include <algorithm>
 #include <cfloat>
 
 #include "internal.cuh"
@@ -24,7 +28,10 @@ namespace hcgb {
 namespace {
 
 constexpr int SVD_THREADS = 512;
-constexpr float PRECOND_TOL32 = 1e-6f;
+constexpr int WIDE_CTAS = 8;              // CTAs of a wide update's cluster
+constexpr int WIDE_CLUSTERS = 19;         // clusters of a launch (152 SMs / 8)
+constexpr int WIDE_POOL_DOUBLES = 16640;  // shared memory of a CTA for a pair of column blocks (130 KB)
+constexpr float PRECOND_TOL32 = 1e-6f;  // above the rounding of a single-precision cosine
 constexpr int PRECOND_MAX_SWEEPS = 12;
 constexpr int SVD_RED_DOUBLES = 64, SVD_REDI_INTS = 128;  // reduction area (up to 32 warps)
 constexpr int SVD_AUX_FIXED = 1 + SVD_RED_DOUBLES + SVD_REDI_INTS / 2;  // aux = 6 kmax + this
@@ -300,179 +307,6 @@ __device__ void jacobi(const TM &tm, double *X, int ldx, int rows, int ncols, do
 }
 
 // Lane-group / register-tile choice for a column length: G lanes per pair, RPL rows per lane.
-// ---------------------------------------------------------------------------------------------
-// Float-float Jacobi (mixed form): the columns, the tracked squared norms and the scales d, 1/d are
-// all float-float values, so neither the rows nor the per-pair bookkeeping touch the FP64 pipe.
-// Same method as jacobi_sweep (round-robin ordering, scaled rotations, tracked norms); the rotation
-// tangent is a float (any tangent gives an exact rotation once cos = 1/sqrt(1 + t^2) is formed to
-// float-float accuracy, which one Newton step on the float reciprocal square root does).
-// ---------------------------------------------------------------------------------------------
-template <int G, int RPL, class TM>
-__device__ int jacobi_sweep_df(const TM &tm, df *X, int ldx, int rows, int ncols, df *nrm, df *ds, df *dv, float tol, float tiny,
-                               int n2) {
-    static_assert(G >= 4, "a pair's bookkeeping is spread over four lanes of its group");
-    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
-    constexpr int PPW = 32 / G;
-    const int gl = lane % G, grp = lane / G;
-    const int npairs = n2 / 2;
-    const int nchunks = (npairs + PPW - 1) / PPW;
-    int rotations = 0;
-    for (int t = 0; t < n2 - 1; t++) {
-        for (int ch = warp; ch < nchunks; ch += nw) {
-            const int pp = ch * PPW + grp;
-            int i = 0, j = 0;
-            bool act = pp < npairs;
-            if (act) {
-                jacobi_pair(t, pp, n2, i, j);
-                act = i < ncols && j < ncols;
-            }
-            df *x = X + (size_t) (act ? i : 0) * ldx;
-            df *y = X + (size_t) (act ? j : 0) * ldx;
-            df xr[RPL], yr[RPL];
-            df_acc ca{0.f, 0.f};
-#pragma unroll
-            for (int q = 0; q < RPL; q++) {
-                xr[q] = yr[q] = df_f(0.f);
-                if (G * q < rows) {
-                    const int r = gl + G * q;
-                    if (act && r < rows) {
-                        xr[q] = x[r];
-                        yr[q] = y[r];
-                    }
-                    df_acc_fma(ca, xr[q], yr[q]);
-                }
-            }
-            const df c = group_sum(df_acc_value(ca), G);
-            df a = df_f(0.f), b = df_f(0.f), di = df_f(1.f), dj = df_f(1.f);
-            if (act) {
-                a = nrm[i];
-                b = nrm[j];
-                di = ds[i];
-                dj = ds[j];
-            }
-            const df cd = df_mul(df_mul(c, di), dj);  // true inner product
-            // |c| / sqrt(a b) > tol, in float (all quantities well inside the float range)
-            const bool rot = act && a.h > tiny && b.h > tiny && fabsf(cd.h) * rsqrtf(a.h) * rsqrtf(b.h) > tol;
-            if (rot) {
-                const float num = df_add(b, -a).h, den = 2.f * cd.h;
-                const float zf = num / den;
-                const float tt = fabsf(zf) > 1.0e18f ? 0.5f / zf
-                                                     : copysignf(1.0f, zf) / (fabsf(zf) + sqrtf(fmaf(zf, zf, 1.0f)));
-                const df q = df_add(df_f(1.f), df_mul(df_f(tt), df_f(tt)));
-                const df cs = df_rsqrt(q);
-                const df dvi = dv[i], dvj = dv[j];
-                const df t1 = df_mul(df_mul(df_f(tt), dj), dvi), t2 = df_mul(df_mul(df_f(tt), di), dvj);
-                const df mt1 = -t1;
-#pragma unroll
-                for (int q2 = 0; q2 < RPL; q2++) {
-                    if (G * q2 < rows) {
-                        const int r = gl + G * q2;
-                        if (r < rows) {
-                            x[r] = df_fma(mt1, yr[q2], xr[q2]);
-                            y[r] = df_fma(t2, xr[q2], yr[q2]);
-                        }
-                    }
-                }
-                // the pair's bookkeeping spread over the first four lanes of its group (as the FP64
-                // sweep's pair_bookkeeping): each evaluates the same float-float operations on
-                // operands it selects, which shortens the dependent chain one lane would otherwise run
-                {
-                    const bool second = gl & 1, norm_lane = gl < 2;
-                    const int col = second ? j : i;
-                    // lanes 0 / 1: norm a - t cd, b + t cd; lanes 2 / 3: scale d cs
-                    const df m1 = norm_lane ? (second ? df_f(tt) : df_f(-tt)) : (second ? dj : di);
-                    const df prod = df_mul(m1, norm_lane ? cd : cs);
-                    const df v = norm_lane ? df_add(second ? b : a, prod) : prod;
-                    const df w = df_mul(second ? dvj : dvi, df_mul(q, cs));  // inverse scale, lanes 0 / 1
-                    if (norm_lane) {
-                        nrm[col] = v;
-                        dv[col] = w;
-                    } else if (gl < 4) {
-                        ds[col] = v;
-                    }
-                }
-                if (gl == 0) rotations++;
-            }
-        }
-        tm.sync();
-    }
-    return rotations;
-}
-
-template <int G, int RPL, class TM>
-__device__ void jacobi_df(const TM &tm, df *X, int ldx, int rows, int ncols, df *nrm, df *ds, df *dv, int *s_rot, float *s_amax,
-                          int *sweeps_out, bool *converged_out, float tol, int max_sweeps) {
-    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
-    const float noise = 3.5527137e-15f * (float) (rows > 1 ? rows : 1);  // 2^-48 rows
-    const int n2 = ncols + (ncols & 1);
-    int sweeps = 0;
-    bool converged = ncols < 2;
-    for (int jj = tm.tid; jj < ncols; jj += tm.nth) ds[jj] = dv[jj] = df_f(1.f);
-    tm.sync();
-    // Exact squared norms; the scales of the previous sweep are folded into the columns.
-    auto fold_and_norms = [&](float &amax) {
-        for (int jj = warp; jj < ncols; jj += nw) {
-            df *col = X + (size_t) jj * ldx;
-            const df d = ds[jj];
-            const bool scale = d.h != 1.f || d.l != 0.f;
-            df sq = df_f(0.f);
-            for (int r = lane; r < rows; r += 32) {
-                df v = col[r];
-                if (scale) {
-                    v = df_mul(v, d);
-                    col[r] = v;
-                }
-                sq = df_fma(v, v, sq);
-            }
-            sq = group_sum(sq, 32);
-            __syncwarp();
-            if (lane == 0) {
-                nrm[jj] = sq;
-                ds[jj] = dv[jj] = df_f(1.f);
-            }
-            amax = fmaxf(amax, sq.h);
-        }
-    };
-    while (!converged && sweeps < max_sweeps) {
-        if (tm.tid == 0) {
-            *s_rot = 0;
-            *s_amax = 0.f;
-        }
-        tm.sync();
-        float amax = 0.f;
-        fold_and_norms(amax);
-        if (lane == 0) atomicMax(reinterpret_cast<int *>(s_amax), __float_as_int(amax));  // amax >= 0
-        tm.sync();
-        const float tiny = *s_amax * noise * noise;
-        const int rot = jacobi_sweep_df<G, RPL>(tm, X, ldx, rows, ncols, nrm, ds, dv, tol, tiny, n2);
-        if (rot) atomicAdd(s_rot, rot);
-        tm.sync();
-        sweeps++;
-        converged = (*s_rot == 0);
-        tm.sync();
-    }
-    float amax = 0.f;
-    fold_and_norms(amax);  // a sweep limit can leave scales unfolded
-    tm.sync();
-    *sweeps_out = sweeps;
-    *converged_out = converged;
-}
-
-template <int MAXRPL, class TM>
-__device__ void jacobi_df_dispatch(const TM &tm, df *X, int ldx, int rows, int ncols, df *nrm, df *ds, df *dv, int *s_rot,
-                                   float *s_amax, int *sweeps, bool *conv, float tol, int max_sweeps) {
-    // (A looped sweep like the FP64 form's measured slower here, 296 vs 192 ms of core per multiply:
-    // the float-float form is not bound by per-pair instructions on a scarce pipe, and reading each
-    // pair twice costs more than it saves.)
-    if (rows <= 32) jacobi_df<4, 8>(tm, X, ldx, rows, ncols, nrm, ds, dv, s_rot, s_amax, sweeps, conv, tol, max_sweeps);
-    else if (rows <= 64) jacobi_df<8, 8>(tm, X, ldx, rows, ncols, nrm, ds, dv, s_rot, s_amax, sweeps, conv, tol, max_sweeps);
-    else if (rows <= 128 && MAXRPL >= 16) jacobi_df<8, 16>(tm, X, ldx, rows, ncols, nrm, ds, dv, s_rot, s_amax, sweeps, conv, tol, max_sweeps);
-    else if (rows <= 128) jacobi_df<16, 8>(tm, X, ldx, rows, ncols, nrm, ds, dv, s_rot, s_amax, sweeps, conv, tol, max_sweeps);
-    else if (rows <= 256 && MAXRPL >= 16) jacobi_df<16, 16>(tm, X, ldx, rows, ncols, nrm, ds, dv, s_rot, s_amax, sweeps, conv, tol, max_sweeps);
-    else if (rows <= 256 || MAXRPL <= 8) jacobi_df<32, 8>(tm, X, ldx, rows, ncols, nrm, ds, dv, s_rot, s_amax, sweeps, conv, tol, max_sweeps);
-    else jacobi_df<32, MAXRPL>(tm, X, ldx, rows, ncols, nrm, ds, dv, s_rot, s_amax, sweeps, conv, tol, max_sweeps);
-}
-
 template <int MAXRPL, class TM>
 __device__ void jacobi_dispatch(const TM &tm, double *X, int ldx, int rows, int ncols, double *nrm, int *s_rot,
                                 double *s_amax, int *sweeps, bool *conv, double tol, int max_sweeps, double *dsc,
@@ -500,131 +334,602 @@ __device__ void jacobi_dispatch(const TM &tm, double *X, int ldx, int rows, int 
 }
 
 // ---------------------------------------------------------------------------------------------
-// FP32 preconditioning of the plain form's Jacobi (the FP64 pipe is the plain core's bound): one-
-// sided Jacobi in single precision on X32 = X * 2^-e (rows x ncols, ld rows) with the rotations
-// accumulated in J (ncols x ncols, ld ncols, float-float), one warp per column pair, until every
-// pair is orthogonal to tol32 or max_sweeps.  The caller then forms X J in FP64 and finishes with
-// FP64 sweeps.  Each rotation is the rotation of a float tangent normalised to float-float accuracy,
-// and J accumulates them in float-float, so J is orthogonal to ~1e-13: X -> X J moves singular values
-// and subspaces only at that level (a truncation at a fixed rank inside a slowly decaying spectrum
-// included), and the FP64 sweeps make the final columns orthogonal to working precision.
+// Preconditioning of the FP64 Jacobi.  One FP64 warp instruction takes ~19 cycles of an SM here, an FP32
+// one a quarter of a cycle, so the sweeps that only have to find the rotations run in single precision:
+//   1. one-sided Jacobi on X32 = X 2^-e with the rotations accumulated in J32 (jacobi32_sweep);
+//   2. J = J32 (I + H), H = -E/2 + 3/8 E^2 - 5/16 E^3, E = J32^T J32 - I: the orthogonal polar factor of
+//      J32 (Newton-Schulz series; E is formed from exact products, so J is orthogonal to ~1e-15);
+//   3. W = X J in FP64: orthogonal columns up to cosines of ~1e-6;
+//   4. corrections W <- W exp(S) (jacobi_correct): S holds every pair's rotation angle, the cosines come
+//      from a float-float Gram matrix and W S is added to W in FP64.  The angles are small, so the rotations
+//      of all pairs commute up to second order and two corrections reach working precision.
+// Only step 3 and one addition per element and correction use the FP64 pipe.  A pair that would turn
+// by more than CORRECT_MAX_TAN (nearly equal singular values), or a correction that does not converge,
+// leaves the rest to the FP64 sweeps.
 // ---------------------------------------------------------------------------------------------
-template <class TM>
-__device__ int jacobi_precond32(const TM &tm, float *X, int rows, int ncols, df *J, float tol32, int max_sweeps,
-                                int *s_rot) {
-    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
-    for (int e = tm.tid; e < ncols * ncols; e += tm.nth) J[e] = df_f((e % ncols) == (e / ncols) ? 1.f : 0.f);
-    const int n2 = ncols + (ncols & 1);
-    const float tol2 = tol32 * tol32;
-    int sweeps = 0;
-    for (; sweeps < max_sweeps; sweeps++) {
-        if (tm.tid == 0) *s_rot = 0;
-        tm.sync();
-        int rot = 0;
-        for (int t = 0; t < n2 - 1; t++) {
-            for (int pp = warp; pp < n2 / 2; pp += nw) {
-                int i, j;
-                jacobi_pair(t, pp, n2, i, j);
-                if (i >= ncols || j >= ncols) continue;
-                float *xi = X + (size_t) i * rows, *xj = X + (size_t) j * rows;
-                float a = 0.f, b = 0.f, c = 0.f;
-                for (int r = lane; r < rows; r += 32) {
-                    const float u = xi[r], w = xj[r];
-                    a = fmaf(u, u, a);
-                    b = fmaf(w, w, b);
-                    c = fmaf(u, w, c);
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    a += __shfl_xor_sync(0xffffffffu, a, o);
-                    b += __shfl_xor_sync(0xffffffffu, b, o);
-                    c += __shfl_xor_sync(0xffffffffu, c, o);
-                }
-                if (c == 0.f || c * c <= tol2 * a * b) continue;
-                const float zeta = (b - a) / (2.f * c);
-                const float tt = copysignf(1.f, zeta) / (fabsf(zeta) + sqrtf(fmaf(zeta, zeta, 1.f)));
-                // The rotation of the float tangent, normalised to float-float accuracy
-                // (cs = 1 / sqrt(1 + t^2), sn = cs t): orthogonal to ~2^-46, so the accumulated J is
-                // orthogonal to working precision of the FP64 phase's purposes.
-                const df tdf = df_f(tt);
-                const df cs = df_rsqrt(df_fma(tdf, tdf, df_f(1.f))), sn = df_mul(cs, tdf);
-                const float cs32 = cs.h, sn32 = sn.h;
-                for (int r = lane; r < rows; r += 32) {
-                    const float u = xi[r], w = xj[r];
-                    xi[r] = cs32 * u - sn32 * w;
-                    xj[r] = fmaf(sn32, u, cs32 * w);
-                }
-                df *ji = J + (size_t) i * ncols, *jj = J + (size_t) j * ncols;
-                for (int r = lane; r < ncols; r += 32) {
-                    const df u = ji[r], w = jj[r];
-                    ji[r] = df_fma(-sn, w, df_mul(cs, u));
-                    jj[r] = df_fma(sn, u, df_mul(cs, w));
-                }
-                rot++;
-            }
-            tm.sync();
-        }
-        if (lane == 0 && rot) atomicAdd(s_rot, rot);
-        tm.sync();
-        const bool done = *s_rot == 0;
-        tm.sync();
-        if (done) break;
-    }
-    return sweeps;
+
+// Tangent of the rotation angle, zeta = (b - a) / (2 c) (Rutishauser; zeta^2 must not overflow).
+__device__ __forceinline__ float rotation_tangent(float zeta) {
+    if (fabsf(zeta) > 1.0e18f) return 0.5f / zeta;
+    return copysignf(1.f, zeta) / (fabsf(zeta) + sqrtf(fmaf(zeta, zeta, 1.f)));
 }
 
-// One step of qrcp_truncated after the reflector of column s is formed (x = column s, v = [1; x[s+1:]],
-// tau): H = I - tau v v^T applied to columns s+1 .. ncols-1 by groups of G lanes (32 / G columns per
-// warp at a time), the squared norms below row s downdated and recomputed exactly when the downdate
-// loses four or more digits (LAPACK dlaqp2's guard).
+// One sweep over columns [0, nc_a) and [off_b, off_b + nc_b) of Y: every pair (cross = false), or the pairs
+// of one column of each range (cross = true).  A column is x4 + j4 quads of floats, ls4 quads apart: its
+// part of X32 and its part of J32 (zero padded); the inner products take the first, rotations both.
 template <int G, class TM>
-__device__ __forceinline__ void qrcp_apply(const TM &tm, double *A, int lda, int mrows, int ncols, int s,
-                                           const double *x, double tau, double *nrm, double *nref) {
+__device__ int jacobi32_sweep(const TM &tm, float4 *Y, int ls4, int x4, int j4, int nc_a, int nc_b, int off_b,
+                              bool cross, float tol) {
+    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
+    constexpr int PPW = 32 / G;
+    const int gl = lane % G, grp = lane / G;
+    const int nc = nc_a + nc_b, n2 = nc + (nc & 1), wide = nc_a > nc_b ? nc_a : nc_b;
+    const int npairs = cross ? wide : n2 / 2, steps = cross ? wide : n2 - 1;
+    const int nchunks = (npairs + PPW - 1) / PPW;
+    int rotations = 0;
+    for (int t = 0; t < steps; t++) {
+        for (int ch = warp; ch < nchunks; ch += nw) {
+            const int pp = ch * PPW + grp;
+            int i = 0, j = 0;
+            bool act = pp < npairs;
+            if (act) {
+                if (cross) {
+                    const int q = pp + t < wide ? pp + t : pp + t - wide;
+                    act = pp < nc_a && q < nc_b;
+                    i = pp;
+                    j = off_b + q;
+                } else {
+                    jacobi_pair(t, pp, n2, i, j);
+                    act = i < nc && j < nc;
+                    i = i < nc_a ? i : off_b + i - nc_a;
+                    j = j < nc_a ? j : off_b + j - nc_a;
+                }
+            }
+            float4 *x = Y + (size_t) (act ? i : 0) * ls4, *y = Y + (size_t) (act ? j : 0) * ls4;
+            float a = 0.f, b = 0.f, c = 0.f;
+            if (act) {
+#pragma unroll 4
+                for (int r = gl; r < x4; r += G) {
+                    const float4 u = x[r], v = y[r];
+                    a = fmaf(u.x, u.x, fmaf(u.y, u.y, fmaf(u.z, u.z, fmaf(u.w, u.w, a))));
+                    b = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, b))));
+                    c = fmaf(u.x, v.x, fmaf(u.y, v.y, fmaf(u.z, v.z, fmaf(u.w, v.w, c))));
+                }
+            }
+#pragma unroll
+            for (int o = G >> 1; o > 0; o >>= 1) {
+                a += __shfl_xor_sync(0xffffffffu, a, o);
+                b += __shfl_xor_sync(0xffffffffu, b, o);
+                c += __shfl_xor_sync(0xffffffffu, c, o);
+            }
+            if (act && a > 0.f && b > 0.f && fabsf(c) * rsqrtf(a) * rsqrtf(b) > tol) {
+                const float zeta = (b - a) / (2.f * c);
+                const float tt = rotation_tangent(zeta);
+                const float cs = 1.f / sqrtf(fmaf(tt, tt, 1.f)), sn = cs * tt;
+#pragma unroll 4
+                for (int r = gl; r < x4 + j4; r += G) {
+                    const float4 u = x[r], v = y[r];
+                    x[r] = make_float4(fmaf(cs, u.x, -sn * v.x), fmaf(cs, u.y, -sn * v.y), fmaf(cs, u.z, -sn * v.z),
+                                       fmaf(cs, u.w, -sn * v.w));
+                    y[r] = make_float4(fmaf(cs, v.x, sn * u.x), fmaf(cs, v.y, sn * u.y), fmaf(cs, v.z, sn * u.z),
+                                       fmaf(cs, v.w, sn * u.w));
+                }
+                if (gl == 0) rotations++;
+            }
+        }
+        tm.sync();
+    }
+    return rotations;
+}
+
+// 16 x 8 output tiles of an M x N result, one warp each: lane (li, lj) accumulates rows i0 + li, i0 + li + 8
+// and columns j0 + lj, j0 + lj + 4 over k = 0 .. K - 1.  mac(acc, i, j0.., k) is given the operands by fa / fb
+// (indices clamped into range); fo stores what lies inside.  keep(i0, j0) skips whole tiles.
+template <class TM, class FA, class FB, class FM, class FI, class FO, class FK>
+__device__ __forceinline__ void warp_tiles(const TM &tm, int M, int N, int K, FA fa, FB fb, FM mac, FI init, FO fo,
+                                           FK keep) {
+    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
+    const int li = lane & 7, lj = lane >> 3;
+    const int nti = (M + 15) >> 4, ntj = (N + 7) >> 3;
+    for (int idx = warp; idx < nti * ntj; idx += nw) {
+        const int i0 = (idx % nti) * 16, j0 = (idx / nti) * 8;
+        if (!keep(i0, j0)) continue;
+        const int ia = i0 + li < M ? i0 + li : M - 1, ib = i0 + li + 8 < M ? i0 + li + 8 : M - 1;
+        const int ja = j0 + lj < N ? j0 + lj : N - 1, jb = j0 + lj + 4 < N ? j0 + lj + 4 : N - 1;
+        df_acc c00 = init(ia, ja), c01 = init(ia, jb), c10 = init(ib, ja), c11 = init(ib, jb);
+#pragma unroll 2
+        for (int k = 0; k < K; k++) {
+            const auto a0 = fa(ia, k), a1 = fa(ib, k);
+            const auto b0 = fb(k, ja), b1 = fb(k, jb);
+            mac(c00, a0, b0);
+            mac(c01, a0, b1);
+            mac(c10, a1, b0);
+            mac(c11, a1, b1);
+        }
+        if (i0 + li < M && j0 + lj < N) fo(i0 + li, j0 + lj, c00);
+        if (i0 + li < M && j0 + lj + 4 < N) fo(i0 + li, j0 + lj + 4, c01);
+        if (i0 + li + 8 < M && j0 + lj < N) fo(i0 + li + 8, j0 + lj, c10);
+        if (i0 + li + 8 < M && j0 + lj + 4 < N) fo(i0 + li + 8, j0 + lj + 4, c11);
+    }
+}
+
+// acc += a b for floats, exactly (Ogita, Rump and Oishi's Dot2).
+__device__ __forceinline__ void acc_exact(df_acc &acc, float a, float b) {
+    const float p = __fmul_rn(a, b), e = __fmaf_rn(a, b, -p);
+    const float t = __fadd_rn(acc.s, p), z = __fsub_rn(t, acc.s);
+    const float es = __fadd_rn(__fsub_rn(acc.s, __fsub_rn(t, z)), __fsub_rn(p, z));
+    acc.s = t;
+    acc.e = __fadd_rn(acc.e, __fadd_rn(e, es));
+}
+
+// E (rk x rk float-float, ld rk) = J^T J - I of the float J (ld ldj).
+template <class TM>
+__device__ void ns_gram(const TM &tm, const float *J, int ldj, int rk, df *E) {
+    warp_tiles(
+        tm, rk, rk, rk, [&](int i, int k) { return J[k + (size_t) i * ldj]; },
+        [&](int k, int j) { return J[k + (size_t) j * ldj]; },
+        [](df_acc &c, float a, float b) { acc_exact(c, a, b); },
+        [](int i, int j) { return df_acc{i == j ? -1.f : 0.f, 0.f}; },
+        [&](int i, int j, df_acc c) { E[i + (size_t) j * rk] = df_acc_value(c); }, [](int, int) { return true; });
+}
+
+// Largest column sum of |E| (bounds its norm).
+template <class TM>
+__device__ float ns_norm(const TM &tm, const df *E, int rk, int *s_bits) {
+    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
+    if (tm.tid == 0) *s_bits = 0;
+    tm.sync();
+    float top = 0.f;
+    for (int j = warp; j < rk; j += nw) {
+        float t = 0.f;
+        for (int i = lane; i < rk; i += 32) t += fabsf(E[i + (size_t) j * rk].h);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (!(t <= top)) top = t;
+    }
+    if (lane == 0) atomicMax(s_bits, __float_as_int(fabsf(top)));  // ordered like its bits, a NaN above all
+    tm.sync();
+    return __int_as_float(*s_bits);
+}
+
+// J64 = J (I + H), written over E (both ld rk), a warp per column.  V (ld ldv): rk x rk floats for
+// 3/8 E^2 - 5/16 E^3.  scr: two vectors of rk floats of shared memory (scr_ld apart) for each of the
+// first scr_warps warps of a CTA; the other warps wait.
+template <class TM>
+__device__ void ns_apply(const TM &tm, const float *J, int ldj, int rk, df *E, float *V, int ldv, float *scr,
+                         int scr_ld, int scr_warps) {
+    const int lane = threadIdx.x & 31;
+    const int wpc = tm.warps_per_cta(), wic = tm.warp() % wpc, cta = tm.warp() / wpc, ctas = tm.nw() / wpc;
+    const int first = wic < scr_warps ? cta * scr_warps + wic : rk, step = ctas * scr_warps;
+    float *s1 = scr + (size_t) (2 * wic) * scr_ld, *s2 = s1 + scr_ld;
+    // out_i = sum_l E_il v(l), four rows a lane at a time
+    auto apply_e = [&](auto v, auto store) {
+        for (int i0 = 0; i0 < rk; i0 += 128) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+            for (int l = 0; l < rk; l++) {
+                const float vl = v(l);
+                const df *El = E + (size_t) l * rk + i0 + lane;
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (i0 + lane + 32 * q < rk) acc[q] = fmaf(El[32 * q].h, vl, acc[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (i0 + lane + 32 * q < rk) store(i0 + lane + 32 * q, acc[q]);
+        }
+    };
+    for (int j = first; j < rk; j += step) {
+        const df *Ej = E + (size_t) j * rk;
+        for (int i = lane; i < rk; i += 32) s2[i] = Ej[i].h;
+        __syncwarp();
+        apply_e([&](int l) { return s2[l]; }, [&](int i, float y) { s1[i] = 0.375f * s2[i] - 0.3125f * y; });
+        __syncwarp();
+        apply_e([&](int l) { return s1[l]; }, [&](int i, float y) { V[i + (size_t) j * ldv] = y; });
+        __syncwarp();
+    }
+    tm.sync();
+    for (int j = first; j < rk; j += step) {
+        df *Ej = E + (size_t) j * rk;
+        for (int i = lane; i < rk; i += 32) {
+            df m = Ej[i];
+            m.h *= -0.5f;
+            m.l *= -0.5f;
+            const df h = df_add(m, df_f(V[i + (size_t) j * ldv]));
+            s1[i] = h.h;
+            s2[i] = h.l;
+        }
+        __syncwarp();
+        double *out = reinterpret_cast<double *>(Ej);
+        for (int i0 = 0; i0 < rk; i0 += 64) {
+            df_acc acc[2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 2
+            for (int l = 0; l < rk; l++) {
+                const float hh = s1[l], hl = s2[l];
+                const float *Jl = J + (size_t) l * ldj + i0 + lane;
+#pragma unroll
+                for (int q = 0; q < 2; q++)
+                    if (i0 + lane + 32 * q < rk) {
+                        const float a = Jl[32 * q];
+                        acc_exact(acc[q], a, hh);
+                        acc[q].e = __fmaf_rn(a, hl, acc[q].e);
+                    }
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int i = i0 + lane + 32 * q;
+                if (i < rk) out[i] = (double) J[i + (size_t) j * ldj] + (double) df_acc_value(acc[q]);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// Largest ||J32^T J32 - I||_1 for which the truncated series is exact to working precision.
+constexpr float PRECOND_MAX_ORTH = 4e-4f;
+constexpr int CORRECT_MAX_PASSES = 4;
+constexpr float CORRECT_MAX_TAN = 0.02f;
+
+// Corrections W <- W exp(S) until every pair of columns is orthogonal to tol, W rows x nc (ld rows).
+// Wh: float-float copy of W 2^-e_j (ld ldh), T: 2 nc^2 floats (S 2^(e_i - e_j), then S^2 / 2 likewise),
+// nrm / ex: a float-float norm and an exponent per column.  Columns below the noise floor of the FP64 sweeps
+// are left alone, as there.  Returns whether the columns are orthogonal to tol.
+template <class TM>
+__device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh, int ldh, float *T, df *nrm, int *ex,
+                               int *s_cos, int *s_tan, float tol, int *passes) {
+    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
+    float *S = T, *Q = T + (size_t) nc * nc;
+    for (int pass = 0; pass < CORRECT_MAX_PASSES; pass++) {
+        // columns as float-float values near 1 and their squared norms
+        for (int j = warp; j < nc; j += nw) {
+            const double *w = W + (size_t) j * rows;
+            int e = 0;
+            for (int r = lane; r < rows; r += 32) {
+                const int f = (int) ((__double_as_longlong(w[r]) >> 52) & 0x7ff);
+                e = e > f ? e : f;
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                const int f = __shfl_xor_sync(0xffffffffu, e, o);
+                e = e > f ? e : f;
+            }
+            e = e ? e - 1023 : -1022;
+            if (e > 1022) e = 1022;  // 2^-e stays a normal number
+            const double down = __hiloint2double((1023 - e) << 20, 0);
+            df sq = df_f(0.f);
+            for (int r = lane; r < rows; r += 32) {
+                const df v = df(w[r] * down);
+                Wh[r + (size_t) j * ldh] = v;
+                sq = df_fma(v, v, sq);
+            }
+            sq = df_group_sum(sq, 32);
+            if (lane == 0) {
+                nrm[j] = sq;
+                ex[j] = e;
+            }
+        }
+        if (tm.tid == 0) {
+            *s_cos = 0;
+            *s_tan = 0;
+        }
+        tm.sync();
+        // the noise floor relative to the largest column (uniform: every thread scans the same norms)
+        int etop = -2000;
+        for (int j = lane; j < nc; j += 32)
+            if (nrm[j].h > 0.f && ex[j] > etop) etop = ex[j];
+        for (int o = 16; o > 0; o >>= 1) {
+            const int f = __shfl_xor_sync(0xffffffffu, etop, o);
+            etop = etop > f ? etop : f;
+        }
+        float top = 0.f;
+        for (int j = lane; j < nc; j += 32)
+            if (ex[j] - etop >= -60) {
+                const float v = ldexpf(nrm[j].h, 2 * (ex[j] - etop));
+                top = top > v ? top : v;
+            }
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        const float noise = 2.220446e-16f * (float) rows;
+        auto live = [&](int j) {
+            const int d = ex[j] - etop;
+            return d >= -60 && ldexpf(nrm[j].h, 2 * d) > top * noise * noise;
+        };
+        float mcos = 0.f, mtan = 0.f;
+        warp_tiles(
+            tm, nc, nc, rows, [&](int i, int k) { return Wh[k + (size_t) i * ldh]; },
+            [&](int k, int j) { return Wh[k + (size_t) j * ldh]; },
+            [](df_acc &c, df a, df b) { df_acc_fma(c, a, b); }, [](int, int) { return df_acc{0.f, 0.f}; },
+            [&](int i, int j, df_acc cc) {
+                if (i > j) return;
+                if (i == j) {
+                    S[i + (size_t) i * nc] = 0.f;
+                    return;
+                }
+                const df c = df_acc_value(cc);
+                const df a = nrm[i], b = nrm[j];
+                const int d = ex[j] - ex[i];
+                float tt = 0.f;
+                const float cosine = fabsf(c.h) * rsqrtf(a.h) * rsqrtf(b.h);
+                if (d >= -60 && d <= 60 && live(i) && live(j) && cosine > 0.1f * tol) {
+                    // in units of the larger column: b' = b 4^d, c' = c 2^d (or a' = a 4^-d, c' = c 2^-d)
+                    const int da = d > 0 ? -d : 0, db = d > 0 ? 0 : d;
+                    df as, bs;
+                    as.h = ldexpf(a.h, 2 * da);
+                    as.l = ldexpf(a.l, 2 * da);
+                    bs.h = ldexpf(b.h, 2 * db);
+                    bs.l = ldexpf(b.l, 2 * db);
+                    const float zeta = df_add(bs, -as).h / (2.f * ldexpf(c.h, d > 0 ? -d : d));
+                    tt = rotation_tangent(zeta);
+                    mcos = fmaxf(mcos, cosine);
+                    mtan = fmaxf(mtan, fabsf(tt));
+                }
+                S[i + (size_t) j * nc] = ldexpf(tt, -d);
+                S[j + (size_t) i * nc] = -ldexpf(tt, d);
+            },
+            [](int i0, int j0) { return i0 <= j0 + 7; });
+        for (int o = 16; o > 0; o >>= 1) {
+            mcos = fmaxf(mcos, __shfl_xor_sync(0xffffffffu, mcos, o));
+            mtan = fmaxf(mtan, __shfl_xor_sync(0xffffffffu, mtan, o));
+        }
+        if (lane == 0) {
+            atomicMax(s_cos, __float_as_int(mcos));
+            atomicMax(s_tan, __float_as_int(mtan));
+        }
+        tm.sync();
+        mcos = __int_as_float(*s_cos);
+        mtan = __int_as_float(*s_tan);
+        *passes = pass + 1;
+        if (mcos <= tol) return true;
+        if (!(mtan < CORRECT_MAX_TAN)) return false;
+        const bool second = (float) nc * mtan * mtan > 1e-17f;  // else S^2 / 2 is below rounding
+        if (second) {
+            warp_tiles(
+                tm, nc, nc, nc, [&](int i, int k) { return S[i + (size_t) k * nc]; },
+                [&](int k, int j) { return S[k + (size_t) j * nc]; },
+                [](df_acc &c, float a, float b) { c.s = fmaf(a, b, c.s); }, [](int, int) { return df_acc{0.f, 0.f}; },
+                [&](int i, int j, df_acc c) { Q[i + (size_t) j * nc] = 0.5f * c.s; }, [](int, int) { return true; });
+            tm.sync();
+        }
+        warp_tiles(
+            tm, rows, nc, nc, [&](int i, int k) { return Wh[i + (size_t) k * ldh]; },
+            [&](int k, int j) {
+                df t;
+                t.h = S[k + (size_t) j * nc];
+                t.l = second ? Q[k + (size_t) j * nc] : 0.f;
+                return t;
+            },
+            [](df_acc &c, df a, df b) { df_acc_fma(c, a, b); }, [](int, int) { return df_acc{0.f, 0.f}; },
+            [&](int i, int j, df_acc c) {
+                const double up = __hiloint2double((1023 + ex[j]) << 20, 0);  // ex >= -1022
+                double *w = W + i + (size_t) j * rows;
+                *w = fma((double) df_acc_value(c), up, *w);
+            },
+            [](int, int) { return true; });
+        tm.sync();
+        // what is left after the correction: second order in the angles
+        if ((float) nc * mtan * mcos < 0.1f * tol) return true;
+    }
+    return false;
+}
+
+
+// Column blocks of the cluster's sweeps: every CTA of the cluster holds one pair of blocks at a time in its
+// shared memory (buf, `quads` float4s) and sweeps the pairs of columns that it gives; the blocks meet in
+// round-robin order, through global memory (Y, columns of x4 + j4 quads).
+template <class TM>
+__device__ int jacobi32_blocks(const TM &tm, float4 *Y, int x4, int j4, int nc, float4 *buf, int quads, float tol) {
+    const int L = x4 + j4;
+    int nblk = 0, w = 0;
+    do {
+        nblk += 2 * TM::ctas;
+        w = (nc + nblk - 1) / nblk;
+    } while (w > 1 && 2 * w * L > quads);
+    const Team<TM::cta_threads> ct{(int) threadIdx.x, 1};
+    int rot = 0;
+    for (int t = 0; t < nblk - 1; t++) {
+        for (int pp = tm.rank; pp < nblk / 2; pp += TM::ctas) {
+            int bi, bj;
+            jacobi_pair(t, pp, nblk, bi, bj);
+            const int ra = nc - bi * w, rb = nc - bj * w;
+            const int na = ra < 0 ? 0 : (ra < w ? ra : w), nb = rb < 0 ? 0 : (rb < w ? rb : w);
+            if (na + nb < 2 || (t > 0 && (na == 0 || nb == 0))) continue;
+            float4 *ya = Y + (size_t) bi * w * L, *yb = Y + (size_t) bj * w * L;
+            for (int e = threadIdx.x; e < na * L; e += TM::cta_threads) buf[e] = __ldcg(ya + e);
+            for (int e = threadIdx.x; e < nb * L; e += TM::cta_threads) buf[w * L + e] = __ldcg(yb + e);
+            ct.sync();
+            if (w <= TM::cta_threads / 32) rot += jacobi32_sweep<32>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
+            else rot += jacobi32_sweep<16>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
+            for (int e = threadIdx.x; e < na * L; e += TM::cta_threads) ya[e] = buf[e];
+            for (int e = threadIdx.x; e < nb * L; e += TM::cta_threads) yb[e] = buf[w * L + e];
+            ct.sync();
+        }
+        tm.sync();
+    }
+    return rot;
+}
+
+// Steps 1-3 and the corrections for X (rows x nc, lower trapezoidal, ld ldx).  Scratch: y (quads float4s, for
+// a cluster in global memory) and for a cluster buf (shared memory); E64 (nc^2 doubles), W (rows x nc
+// doubles; may lie over y in global memory), Wh (rows x nc float-float values, ld ldh; may lie over y in
+// shared memory and over X), V (floats, ldv; unused entries of y or memory of its own).  On return W holds
+// the columns; *converged as for the sweeps.  Returns false with X untouched when J32 is no rotation.
+struct PrecondBuffers {
+    float4 *y;
+    int ls4;           // quads per column of y
+    float4 *buf;       // cluster: shared memory for a pair of blocks and the vectors of ns_apply
+    int buf_quads;
+    double *e64;
+    double *w;
+    df *wh;
+    int ldh;
+    float *v;
+    int ldv;
+};
+
+template <class TM>
+__device__ bool jacobi_precond(const TM &tm, const double *X, int ldx, int rows, int nc, const PrecondBuffers &b,
+                               df *nrm, int *ex, int *s_rot, int *s_emax, int *s_cos, int *s_tan, float tol,
+                               int *sweeps, bool *converged) {
+    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
+    const int lr = lane >> 2, lc = lane & 3;
+    const int x4 = (rows + 3) >> 2, j4 = (nc + 3) >> 2;
+    float *Y = reinterpret_cast<float *>(b.y);
+    const int ldy = 4 * b.ls4;
+    if (tm.tid == 0) *s_emax = 0;
+    tm.sync();
+    int em = 0;
+    for (int j = warp; j < nc; j += nw)
+        for (int r = lane; r < rows; r += 32) {
+            const int f = (int) ((__double_as_longlong(X[r + (size_t) j * ldx]) >> 52) & 0x7ff);
+            em = em > f ? em : f;
+        }
+    atomicMax(s_emax, em);
+    tm.sync();
+    const int esc = *s_emax ? *s_emax - 1023 : 0;
+    const double down = __hiloint2double((1023 - (esc > 1022 ? 1022 : esc)) << 20, 0);
+    for (int j = warp; j < nc; j += nw) {
+        float *y = Y + (size_t) j * ldy;
+        for (int r = lane; r < 4 * x4; r += 32) y[r] = r < rows ? (float) (X[r + (size_t) j * ldx] * down) : 0.f;
+        for (int r = lane; r < 4 * j4; r += 32) y[4 * x4 + r] = r == j ? 1.f : 0.f;
+    }
+    tm.sync();
+    // 1. single-precision sweeps, until one turns few pairs: what it leaves is second order
+    for (int s = 0; s < PRECOND_MAX_SWEEPS; s++) {
+        if (tm.tid == 0) *s_rot = 0;
+        tm.sync();
+        int rot;
+        if constexpr (TM::ctas > 1) rot = jacobi32_blocks(tm, b.y, x4, j4, nc, b.buf, b.buf_quads, PRECOND_TOL32);
+        else rot = jacobi32_sweep<4>(tm, b.y, b.ls4, x4, j4, nc, 0, 0, false, PRECOND_TOL32);
+        if (rot) atomicAdd(s_rot, rot);
+        tm.sync();
+        const int total = *s_rot;
+        tm.sync();
+        ++*sweeps;
+        if (total * 16 <= nc * (nc - 1) / 2) break;
+    }
+    // 2. the orthogonal factor of J32
+    const float *J = Y + 4 * x4;
+    df *E = reinterpret_cast<df *>(b.e64);
+    ns_gram(tm, J, ldy, nc, E);
+    tm.sync();
+    if (!(ns_norm(tm, E, nc, s_rot) < PRECOND_MAX_ORTH)) return false;
+    if constexpr (TM::ctas > 1) {
+        float *scr = reinterpret_cast<float *>(b.buf);
+        const int fit = 4 * b.buf_quads / (2 * nc), wpc = tm.warps_per_cta();
+        ns_apply(tm, J, ldy, nc, E, b.v, b.ldv, scr, nc, fit < wpc ? fit : wpc);
+    } else {
+        ns_apply(tm, J, ldy, nc, E, b.v, b.ldv, Y, ldy, nc / 2 < nw ? nc / 2 : nw);  // over X32, which is done
+    }
+    tm.sync();
+    // 3. W = X J on DMMA; column l of X starts at row l
+    const double *J64 = b.e64;
+    const int ntr = (rows + 7) >> 3, ntc = (nc + 7) >> 3;
+    for (int idx = warp; idx < ntr * ntc; idx += nw) {
+        const int tr = idx % ntr, tc = idx / ntr;
+        const int irow = tr * 8 + lr, icol = tc * 8 + lr;
+        const int kend = nc < tr * 8 + 8 ? nc : tr * 8 + 8;
+        const double *jc = J64 + (size_t) (icol < nc ? icol : 0) * nc;
+        double d0 = 0.0, d1 = 0.0;
+#pragma unroll 4
+        for (int l4 = 0; l4 < kend; l4 += 4) {
+            const int l = l4 + lc;
+            const double av = (irow < rows && l < nc) ? X[irow + (size_t) l * ldx] : 0.0;
+            const double bv = (icol < nc && l < nc) ? jc[l] : 0.0;
+            dmma(d0, d1, av, bv);
+        }
+        const int col = tc * 8 + 2 * lc;
+        if (irow < rows && col < nc) b.w[irow + (size_t) col * rows] = d0;
+        if (irow < rows && col + 1 < nc) b.w[irow + (size_t) (col + 1) * rows] = d1;
+    }
+    tm.sync();
+    int passes = 0;
+    *converged = jacobi_correct(tm, b.w, rows, nc, b.wh, b.ldh, reinterpret_cast<float *>(b.e64), nrm, ex, s_cos, s_tan,
+                                tol, &passes);
+    *sweeps += passes;
+    return true;
+}
+
+// A step's reflector H = I - gamma v v^T for the pivot column x (rows s ..), v = [alpha - beta; x_{s+1}, ..]
+// (dlarfg's beta, v not normalised: only R is kept).  sigma = ||x_{s+1..}||^2.  One reciprocal square root and
+// one reciprocal: every FP64 instruction of this chain holds up the whole team.
+struct Reflector {
+    double beta, vs, gamma;
+};
+__device__ __forceinline__ Reflector make_reflector(double alpha, double sigma) {
+    Reflector h{alpha, 0.0, 0.0};
+    if (sigma != 0.0) {
+        const double q = fma(alpha, alpha, sigma), r = rsqrt(q), nrm = q * r, d = nrm + fabs(alpha);
+        h.beta = -copysign(nrm, alpha);
+        h.vs = copysign(d, alpha);       // alpha - beta
+        h.gamma = r * __drcp_rn(d);      // 2 / ||v||^2 = 1 / (nrm (nrm + |alpha|))
+    }
+    return h;
+}
+
+// One step of the pivoted QR: H applied to column y (rows s .. mrows - 1) by a group of G lanes, its squared norm
+// below row s downdated and recomputed exactly when the downdate loses four or more digits (LAPACK
+// dlaqp2's guard).  act: whether the group has a column (uniform in the group); every lane of the warp calls.
+template <int G>
+__device__ __forceinline__ void reflect_column(bool act, double *y, const double *x, const Reflector &h, int s,
+                                               int mrows, int gl, double *nrm, double *nref) {
+    double w = 0.0;
+    if (act && h.gamma != 0.0) {
+        w = gl == 0 ? h.vs * y[s] : 0.0;
+        for (int i = s + 1 + gl; i < mrows; i += G) w = fma(x[i], y[i], w);
+    }
+    w = group_sum(w, G) * h.gamma;
+    double ys = 0.0;
+    if (act) {
+        ys = fma(-w, h.vs, y[s]);  // every lane of the group reads the old y[s] before lane 0 writes it
+        if (h.gamma != 0.0)
+            for (int i = s + 1 + gl; i < mrows; i += G) y[i] = fma(-w, x[i], y[i]);
+    }
+    __syncwarp();
+    double nn = 0.0;
+    bool exact = false;
+    if (act) {
+        if (gl == 0) y[s] = ys;
+        nn = fma(-ys, ys, *nrm);
+        exact = !(nn > 1e-8 * *nref);
+    }
+    if (__any_sync(0xffffffffu, exact)) {
+        double e = 0.0;
+        if (exact)
+            for (int i = s + 1 + gl; i < mrows; i += G) e = fma(y[i], y[i], e);
+        e = group_sum(e, G);
+        if (exact) nn = e;
+    }
+    __syncwarp();
+    if (act && gl == 0) {
+        *nrm = nn;
+        if (exact) *nref = nn;
+    }
+}
+
+// (value, index) with the largest value over a warp, ties to the lower index; values are the bits of
+// non-negative doubles, ordered like them (a NaN is never chosen).
+constexpr long long NRM_MAX_BITS = 0x7ff0000000000000LL;
+__device__ __forceinline__ void warp_argmax(long long &v, int &i) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long ov = __shfl_xor_sync(0xffffffffu, v, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
+        if (ov > v || (ov == v && oi < i)) {
+            v = ov;
+            i = oi;
+        }
+    }
+}
+
+// Householder QR with column pivoting of A (mrows x ncols, ld lda), stopped early once
+// every remaining column is below sqrt(stop2) in norm (LAPACK dgeqp3 semantics for the part that
+// is computed: A P = Q R).  stop2 < 0 disables the early stop; stop2 == 0 with rel > 0 sets
+// stop2 = (rel * |r_00|)^2 after the first pivot.  Columns stay in place: pvt[s] is the column of step s,
+// R(s, t) stands in A(s, pvt[t]).  Returns the number of rows of R that were computed.
+// Two barriers a step: the first warp picks the pivot and forms the reflector, the team applies it.
+template <int G, class TM>
+__device__ int qrcp_steps(const TM &tm, double *A, int lda, int mrows, int ncols, double stop2, double rel, double *nrm,
+                          double *nref, int *pvt, double *red, int *redi) {
     const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
     constexpr int CPW = 32 / G;
     const int gl = lane % G, grp = lane / G;
-    for (int j0 = s + 1 + warp * CPW; j0 < ncols; j0 += nw * CPW) {
-        const int j = j0 + grp;
-        const bool act = j < ncols;
-        double *y = A + (size_t) (act ? j : s) * lda;  // idle groups read column s and write nothing
-        double w = 0.0;
-        if (tau != 0.0) {
-            w = gl == 0 ? y[s] : 0.0;
-            for (int i = s + 1 + gl; i < mrows; i += G) w = fma(x[i], y[i], w);
-            w = group_sum(w, G) * tau;
-            if (act)
-                for (int i = s + 1 + gl; i < mrows; i += G) y[i] = fma(-w, x[i], y[i]);
-        }
-        const double ys = y[s] - w;  // every lane of the group reads the old y[s] before lane 0 writes it
-        __syncwarp();
-        if (act && gl == 0) y[s] = ys;
-        double nn = act ? nrm[j] - ys * ys : 0.0;
-        const bool exact = act && !(nn > 1e-8 * nref[j]);
-        if (__any_sync(0xffffffffu, exact)) {
-            double e = 0.0;
-            if (exact)
-                for (int i = s + 1 + gl; i < mrows; i += G) e = fma(y[i], y[i], e);
-            e = group_sum(e, G);
-            if (exact) nn = e;
-        }
-        __syncwarp();
-        if (act && gl == 0) {
-            nrm[j] = nn;
-            if (exact) nref[j] = nn;
-        }
-    }
-}
-
-// Householder QR with column pivoting of A (mrows x ncols, ld lda) in place, stopped early once
-// every remaining column is below sqrt(stop2) in norm (LAPACK dgeqp3 semantics for the part that
-// is computed: A P = Q R with R in the upper triangle, pvt[s] = original index of column s).
-// stop2 < 0 disables the early stop; stop2 == 0 with rel > 0 sets stop2 = (rel * |r_00|)^2 after
-// the first pivot.  Column norms are recomputed exactly while each column is updated, so no
-// norm downdating is needed.  Returns the number of rows of R that were computed.
-template <class TM>
-__device__ int qrcp_truncated(const TM &tm, double *A, int lda, int mrows, int ncols, double stop2, double rel, double *nrm,
-                              double *nref, int *pvt, double *red, int *redi) {
-    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
     for (int j = warp; j < ncols; j += nw) {
         const double *col = A + (size_t) j * lda;
         double t = 0.0;
@@ -635,95 +940,197 @@ __device__ int qrcp_truncated(const TM &tm, double *A, int lda, int mrows, int n
     for (int j = tm.tid; j < ncols; j += tm.nth) pvt[j] = j;
     tm.sync();
     const int kk = mrows < ncols ? mrows : ncols;
-    int rkeep = kk;
+    double lim = stop2;
     for (int s = 0; s < kk; s++) {
-        // pivot = argmax of the remaining squared norms (ties to the lower index), by the first warp
-        // alone: the scan is short, and one warp's reduction costs an eighth of the FP64 instructions
-        // of a team-wide one, whose barrier it also saves
-        double bv = -1.0;
-        int bi = s;
         if (warp == 0) {
-            for (int j = s + lane; j < ncols; j += 32)
-                if (nrm[j] > bv) {
-                    bv = nrm[j];
+            long long bv = -1;
+            int bi = s;
+            for (int j = s + lane; j < ncols; j += 32) {
+                long long v = __double_as_longlong(nrm[pvt[j]]);
+                if (v > NRM_MAX_BITS) v = -1;
+                if (v > bv) {
+                    bv = v;
                     bi = j;
                 }
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ov > bv || (ov == bv && oi < bi)) {
-                    bv = ov;
-                    bi = oi;
+            }
+            warp_argmax(bv, bi);
+            const double top = bv < 0 ? 0.0 : __longlong_as_double(bv);
+            if (s == 0 && stop2 == 0.0 && rel > 0.0) lim = rel * rel * top;
+            const bool stop = top <= lim || top <= 0.0;
+            if (!stop) {
+                const int cs = pvt[bi];
+                __syncwarp();
+                if (lane == 0) {
+                    pvt[bi] = pvt[s];
+                    pvt[s] = cs;
+                }
+                double *x = A + (size_t) cs * lda;
+                double t = 0.0;
+                for (int i = s + 1 + lane; i < mrows; i += 32) t = fma(x[i], x[i], t);
+                t = warp_sum(t);
+                const Reflector h = make_reflector(x[s], t);
+                __syncwarp();
+                if (lane == 0) {
+                    red[0] = h.vs;
+                    red[1] = h.gamma;
+                    x[s] = h.beta;
+                    redi[1] = cs;
                 }
             }
-            if (lane == 0) {
-                red[32] = bv;
-                redi[32] = bi;
-                if (s == 0 && stop2 == 0.0 && rel > 0.0) red[33] = rel * rel * bv;
-                else if (s == 0) red[33] = stop2;
-            }
+            if (lane == 0) redi[0] = stop;
         }
         tm.sync();
-        bv = red[32];
-        bi = redi[32];
-        const double lim = red[33];
-        if (bv <= lim || bv <= 0.0) {
-            rkeep = s;
-            break;
+        if (redi[0]) return s;
+        const Reflector h{0.0, red[0], red[1]};
+        const double *x = A + (size_t) redi[1] * lda;
+        for (int j0 = s + 1 + warp * CPW; j0 < ncols; j0 += nw * CPW) {
+            const int j = j0 + grp;
+            const bool act = j < ncols;
+            const int c = pvt[act ? j : s];
+            reflect_column<G>(act, A + (size_t) c * lda, x, h, s, mrows, gl, nrm + c, nref + c);
         }
-        if (bi != s) {
-            double *cs = A + (size_t) s * lda, *cb = A + (size_t) bi * lda;
-            for (int i = tm.tid; i < mrows; i += tm.nth) {
-                const double t = cs[i];
-                cs[i] = cb[i];
-                cb[i] = t;
-            }
-            if (tm.tid == 0) {
-                const double t = nrm[s];
-                nrm[s] = nrm[bi];
-                nrm[bi] = t;
-                const double tr = nref[s];
-                nref[s] = nref[bi];
-                nref[bi] = tr;
-                const int ti = pvt[s];
-                pvt[s] = pvt[bi];
-                pvt[bi] = ti;
-            }
-        }
-        tm.sync();
-        // Householder vector of column s (rows s..mrows-1), dlarfg convention, by the first warp.
-        double *x = A + (size_t) s * lda;
-        double t = 0.0;
-        if (warp == 0) {
-            for (int i = s + 1 + lane; i < mrows; i += 32) t = fma(x[i], x[i], t);
-            t = warp_sum(t);
-        }
-        if (tm.tid == 0) {
-            const double alpha = x[s];
-            double tau = 0.0, scale = 0.0, beta = alpha;
-            if (t != 0.0) {
-                beta = -copysign(sqrt(fma(alpha, alpha, t)), alpha);
-                tau = (beta - alpha) / beta;
-                scale = 1.0 / (alpha - beta);
-            }
-            x[s] = beta;
-            red[40] = tau;
-            red[41] = scale;
-        }
-        tm.sync();
-        const double tau = red[40], scale = red[41];
-        for (int i = s + 1 + tm.tid; i < mrows; i += tm.nth) x[i] *= scale;
-        tm.sync();
-        // Apply H to the remaining columns; downdate their squared norms below row s
-        // (nrm -= y_s^2) and recompute exactly when the downdate cancels (LAPACK dlaqp2's guard).
-        // Columns of up to 64, 256 or more rows are handled by groups of 4, 8 or 16 lanes, several
-        // columns per warp instruction, so the reductions and the per-column scalar work are shared.
-        if (mrows <= 64) qrcp_apply<4>(tm, A, lda, mrows, ncols, s, x, tau, nrm, nref);
-        else if (mrows <= 256) qrcp_apply<8>(tm, A, lda, mrows, ncols, s, x, tau, nrm, nref);
-        else qrcp_apply<16>(tm, A, lda, mrows, ncols, s, x, tau, nrm, nref);
         tm.sync();
     }
-    return rkeep;
+    return kk;
+}
+
+// Columns of up to 64, 256 or more rows are handled by groups of 4, 8 or 16 lanes, several columns per warp
+// instruction, so the reductions and the per-column scalar work are shared.
+template <class TM>
+__device__ int qrcp_truncated(const TM &tm, double *A, int lda, int mrows, int ncols, double stop2, double rel, double *nrm,
+                              double *nref, int *pvt, double *red, int *redi) {
+    if (mrows <= 64) return qrcp_steps<4>(tm, A, lda, mrows, ncols, stop2, rel, nrm, nref, pvt, red, redi);
+    if (mrows <= 256) return qrcp_steps<8>(tm, A, lda, mrows, ncols, stop2, rel, nrm, nref, pvt, red, redi);
+    return qrcp_steps<16>(tm, A, lda, mrows, ncols, stop2, rel, nrm, nref, pvt, red, redi);
+}
+
+// The same for a cluster: column j lives in the shared memory of CTA j % CTAS, and a step costs one
+// cluster barrier: every CTA offers its best column to all, each reads the winner's column from its owner and
+// forms the reflector itself.  (Through global memory a step took 24,000 cycles on a 130-column core, bound
+// by dependent L2 round trips and five cluster barriers.)  R goes to X = R^T directly (rk columns of
+// ncols entries, ld ldx, entry t of column s for pivot order t).  pvt: shared by the cluster.
+constexpr int QRCP_CLUSTER_G = 16;
+__host__ __device__ __forceinline__ int qrcp_cluster_doubles(int mrows, int ncols, int ctas) {
+    const int nl = (ncols + ctas - 1) / ctas;
+    return mrows * nl + 3 * nl + 2 * mrows + (ncols + 1) / 2 + 6 * ctas + 8;
+}
+
+template <class TM>
+__device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, int ncols, double stop2, double rel,
+                            double *X, int ldx, int *pvt, double *pool) {
+    constexpr int C = TM::ctas, G = QRCP_CLUSTER_G, CPW = 32 / G;
+    const Team<TM::cta_threads> ct{(int) threadIdx.x, 1};
+    const int warp = ct.warp(), lane = threadIdx.x & 31, nw = ct.nw(), rank = tm.rank;
+    const int gl = lane % G, grp = lane / G;
+    const int nlmax = (ncols + C - 1) / C, nl = rank < ncols ? (ncols - rank + C - 1) / C : 0;
+    double *A = pool;                               // mrows x nlmax: local column q is column rank + q C
+    double *nrm = A + (size_t) mrows * nlmax;
+    double *nref = nrm + nlmax;
+    double *xb = nref + nlmax;                      // the pivot column
+    double *diag = xb + mrows;                      // beta of every step
+    double *red = diag + mrows;                     // vs, gamma
+    long long *cv = reinterpret_cast<long long *>(red + 4);  // candidates of the CTAs, two steps' worth
+    int *ci = reinterpret_cast<int *>(cv + 2 * C);
+    int *act_list = ci + 2 * C;                     // local columns not chosen yet
+    int *taken = act_list + 2 * nlmax;              // per column: chosen (for the leftovers)
+    for (int q = warp; q < nl; q += nw) {
+        const double *col = M + (size_t) (rank + q * C) * ldm;
+        double t = 0.0;
+        for (int i = lane; i < mrows; i += 32) {
+            const double v = col[i];
+            A[i + (size_t) q * mrows] = v;
+            t = fma(v, v, t);
+        }
+        t = warp_sum(t);
+        if (lane == 0) nrm[q] = nref[q] = t;
+    }
+    for (int q = threadIdx.x; q < nl; q += TM::cta_threads) act_list[q] = q;
+    for (int j = threadIdx.x; j < ncols; j += TM::cta_threads) taken[j] = 0;
+    ct.sync();
+    int nact = nl, rk = mrows < ncols ? mrows : ncols;
+    const int kk = rk;
+    double lim = stop2;
+    for (int s = 0; s < kk; s++) {
+        const int par = (s & 1) * C;
+        if (warp == 0) {
+            long long bv = -1;
+            int bi = ncols;
+            for (int q = lane; q < nact; q += 32) {
+                const int c = act_list[q], j = rank + c * C;
+                long long v = __double_as_longlong(nrm[c]);
+                if (v > NRM_MAX_BITS) v = -1;
+                if (v > bv || (v == bv && j < bi)) {
+                    bv = v;
+                    bi = j;
+                }
+            }
+            warp_argmax(bv, bi);
+            if (lane < C) {
+                cluster_map(cv, lane)[par + rank] = bv;
+                cluster_map(ci, lane)[par + rank] = bi;
+            }
+        }
+        tm.sync();
+        long long bv = lane < C ? cv[par + lane] : -1;
+        int bi = lane < C ? ci[par + lane] : ncols;
+        warp_argmax(bv, bi);
+        const double top = bv < 0 ? 0.0 : __longlong_as_double(bv);
+        if (s == 0 && stop2 == 0.0 && rel > 0.0) lim = rel * rel * top;
+        if (top <= lim || top <= 0.0) {
+            rk = s;
+            break;
+        }
+        const int owner = bi % C, lcol = bi / C;
+        if (warp == 0) {
+            const double *x = cluster_map(A, owner) + (size_t) lcol * mrows;
+            double t = 0.0;
+            for (int i = s + lane; i < mrows; i += 32) {
+                const double v = x[i];
+                xb[i] = v;
+                if (i > s) t = fma(v, v, t);
+            }
+            t = warp_sum(t);
+            __syncwarp();
+            const Reflector h = make_reflector(xb[s], t);
+            if (lane == 0) {
+                red[0] = h.vs;
+                red[1] = h.gamma;
+                diag[s] = h.beta;
+                taken[bi] = 1;
+                if (rank == 0) pvt[s] = bi;
+            }
+        }
+        if (owner == rank) {  // drop it from the list (any order will do)
+            if (warp == 1) {
+                for (int q = lane; q < nact - 1; q += 32)
+                    if (act_list[q] == lcol) act_list[q] = act_list[nact - 1];
+            }
+            nact--;
+        }
+        ct.sync();
+        const Reflector h{0.0, red[0], red[1]};
+        for (int q0 = warp * CPW; q0 < nact; q0 += nw * CPW) {
+            const bool act = q0 + grp < nact;
+            const int c = act_list[act ? q0 + grp : 0];
+            reflect_column<G>(act, A + (size_t) c * mrows, xb, h, s, mrows, gl, nrm + c, nref + c);
+        }
+        ct.sync();
+    }
+    ct.sync();
+    if (rank == 0 && threadIdx.x == 0) {
+        int t = rk;
+        for (int j = 0; j < ncols; j++)
+            if (!taken[j]) pvt[t++] = j;
+    }
+    tm.sync();
+    for (int t = tm.warp(); t < ncols; t += tm.nw()) {
+        const int j = pvt[t];
+        const double *col = cluster_map(A, j % C) + (size_t) (j / C) * mrows;
+        for (int i = lane; i < rk; i += 32) X[t + (size_t) i * ldx] = i < t ? col[i] : (i == t ? diag[i] : 0.0);
+        if (rk == 0 && lane == 0) X[t] = M[(size_t) j * ldm];
+    }
+    tm.sync();
+    return rk;
 }
 
 // qrcp_apply in float-float arithmetic (mixed form): H applied to columns s+1 .. ncols-1 by groups of
@@ -873,9 +1280,15 @@ __device__ int qrcp_truncated_df(const TM &tm, df *A, int lda, int mrows, int nc
     return rkeep;
 }
 
+// Shared variables of a team (of a cluster: in its first CTA).
+struct CoreShared {
+    int rot, rank, emax, cosine, tangent;
+    double amax;
+};
+
 template <int RPL, class TM>
 __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace &ws, const Params &p, int slot,
-                            double *sm, int smem_doubles, int &s_rot, int &s_rank, int &s_emax, double &s_amax);
+                            double *sm, double *pool, int pool_doubles, CoreShared &sh);
 
 // Stage key of an update in ws.order (sorted by decreasing key): its stack width k when C is
 // compressed.  Both fields are written by the plan kernel only, so the key is stable while the
@@ -885,13 +1298,29 @@ __device__ __forceinline__ int order_key(const Workspace &ws, int slot) {
     return m[META_CKIND] ? m[META_K] : 0;
 }
 
-// CTA of SVD_THREADS threads, in one of three team layouts chosen by the update's stack width k:
-// heavy (k > kthr: the core does not fit half of the shared memory) — the whole CTA for one update;
-// light (kthr4 < k <= kthr) — two half-CTA teams of SVD_THREADS / 2 threads, one update each, each
-// with half of the shared memory and its own named barrier; small (k <= kthr4: the core fits a
-// quarter) — four teams of SVD_THREADS / 4 threads.  Small cores are latency-bound (per-step
-// barriers, dependent FP64 chains), so four of them per SM hide each other's latency.  With ws.order
-// (sorted by decreasing k) the classes are contiguous: CTA b < H takes order[b]; the next ceil(L / 2)
+// Updates of `order` (descending keys) with a key above thr.
+__device__ int count_above(const Workspace &ws, int nup, int thr) {
+    int lo = 0, hi = nup;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (order_key(ws, ws.order[mid]) > thr) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Doubles of the auxiliary arrays of an update of stack width k at the start of its team's shared memory.
+__device__ __forceinline__ int core_aux_doubles(const Workspace &ws, int slot) {
+    const int k = ws.meta[(size_t) slot * META_INTS + META_K];
+    return 6 * (k > 0 ? k : 1) + SVD_AUX_FIXED;
+}
+
+// CTA of SVD_THREADS threads, in one of two team layouts chosen by the update's stack width k: light
+// (kthr4 < k <= kthr) — two half-CTA teams of SVD_THREADS / 2 threads, one update each, each with half
+// of the shared memory and its own named barrier; small (k <= kthr4: the core fits a quarter) — four teams
+// of SVD_THREADS / 4 threads.  Small cores are latency-bound (per-step barriers, dependent FP64 chains), so
+// four of them per SM hide each other's latency.  Wider updates are core_wide_kernel's.  With ws.order
+// (sorted by decreasing k) the classes are contiguous: after the H wide updates, the first ceil(L / 2)
 // CTAs take the L light updates in pairs; the rest take the small ones in fours.  Without an order
 // (one update per CTA) the team size follows the same class rule, so an update's arithmetic never
 // depends on the launch it is part of.
@@ -899,72 +1328,84 @@ template <int RPL>
 __global__ void __launch_bounds__(SVD_THREADS, 1) core_svd_kernel(const DevUpdate *ups, int nup, Workspace ws,
                                                                Params p, int team_doubles, int kthr, int kthr4) {
     extern __shared__ double smem_all[];
-    __shared__ int s_rot_a[4], s_rank_a[4], s_emax_a[4], s_nheavy, s_nlight;
-    __shared__ double s_amax_a[4];
+    __shared__ CoreShared s_sh[4];
+    __shared__ int s_wide, s_nlight;
     if (threadIdx.x == 0) {
-        int h = -1, h2 = -1;
-        if (ws.order) {
-            auto count_above = [&](int thr) {  // entries with key > thr (keys descending)
-                int lo = 0, hi = nup;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (order_key(ws, ws.order[mid]) > thr) lo = mid + 1;
-                    else hi = mid;
-                }
-                return lo;
-            };
-            h = count_above(kthr);
-            h2 = count_above(kthr4);
-        }
-        s_nheavy = h;
-        s_nlight = h2 - h;
+        s_wide = ws.order ? count_above(ws, nup, kthr) : -1;
+        s_nlight = ws.order ? count_above(ws, nup, kthr4) - s_wide : 0;
     }
     __syncthreads();
-    const int H = s_nheavy, NL = s_nlight;
+    const int H = s_wide, NL = s_nlight;
     constexpr int HALF = SVD_THREADS / 2, QUART = SVD_THREADS / 4;
     const int quarter_doubles = team_doubles / 2;
-    int idx, part = 0, cls;  // cls 0 heavy, 1 light, 2 small
+    int idx, part = 0;
+    bool light;
     if (H < 0) {
         idx = blockIdx.x;
         if (idx >= nup) return;
         const int key = order_key(ws, idx);
-        cls = key > kthr ? 0 : (key > kthr4 ? 1 : 2);
-        if (cls == 1 && threadIdx.x >= HALF) return;
-        if (cls == 2 && threadIdx.x >= QUART) return;
+        if (key > kthr) return;
+        light = key > kthr4;
+        if (threadIdx.x >= (light ? HALF : QUART)) return;
     } else {
         const int b = blockIdx.x, nlb = (NL + 1) / 2;
-        if (b < H) {
-            idx = b;
-            cls = 0;
-        } else if (b < H + nlb) {
-            cls = 1;
+        light = b < nlb;
+        if (light) {
             part = threadIdx.x / HALF;
-            idx = H + 2 * (b - H) + part;
+            idx = H + 2 * b + part;
             if (idx >= H + NL) return;  // the odd light update's partner slot stays idle
         } else {
-            cls = 2;
             part = threadIdx.x / QUART;
-            idx = H + NL + 4 * (b - H - nlb) + part;
+            idx = H + NL + 4 * (b - nlb) + part;
         }
     }
     if (idx >= nup) return;
-    if (cls == 0)
-        core_update<RPL>(Team<SVD_THREADS>{(int) threadIdx.x, 1}, ups, ws, p, ws.heavy(idx), smem_all,
-                         2 * team_doubles, s_rot_a[0], s_rank_a[0], s_emax_a[0], s_amax_a[0]);
-    else if (cls == 1)
-        core_update<RPL>(Team<HALF>{(int) threadIdx.x % HALF, 1 + part}, ups, ws, p, ws.heavy(idx),
-                         smem_all + (size_t) part * team_doubles, team_doubles, s_rot_a[part], s_rank_a[part],
-                         s_emax_a[part], s_amax_a[part]);
+    const int slot = ws.heavy(idx), doubles = light ? team_doubles : quarter_doubles;
+    double *sm = smem_all + (size_t) part * doubles;
+    const int aux = core_aux_doubles(ws, slot);
+    if (light)
+        core_update<RPL>(Team<HALF>{(int) threadIdx.x % HALF, 1 + part}, ups, ws, p, slot, sm, sm + aux, doubles - aux,
+                         s_sh[part]);
     else
-        core_update<RPL>(Team<QUART>{(int) threadIdx.x % QUART, 1 + part}, ups, ws, p, ws.heavy(idx),
-                         smem_all + (size_t) part * quarter_doubles, quarter_doubles, s_rot_a[part], s_rank_a[part],
-                         s_emax_a[part], s_amax_a[part]);
+        core_update<RPL>(Team<QUART>{(int) threadIdx.x % QUART, 1 + part}, ups, ws, p, slot, sm, sm + aux,
+                         doubles - aux, s_sh[part]);
 }
 
-// The recompression core of one update (slot) by one team, with `smem_doubles` of shared memory at sm.
+// The wide updates (k > kthr: the core does not fit half of an SM's shared memory): a cluster of WIDE_CTAS
+// CTAs each, the matrices in global memory (L2), the auxiliary arrays and shared variables in the first
+// CTA's shared memory.  One SM's FP64 pipe took 35 ms for the Jacobi sweeps of a 200-column core and 180 ms for
+// a 340-column one, and a chain of such updates bounds a multiply, however few they are.
+template <int RPL>
+__global__ void __cluster_dims__(WIDE_CTAS, 1, 1) __launch_bounds__(SVD_THREADS, 1)
+    core_wide_kernel(const DevUpdate *ups, int nup, Workspace ws, Params p, int smem_doubles, int kthr) {
+    extern __shared__ double smem_all[];
+    __shared__ CoreShared s_sh;
+    __shared__ int s_wide;
+    const int rank = cluster_rank();
+    const ClusterTeam<SVD_THREADS, WIDE_CTAS> tm{rank * SVD_THREADS + (int) threadIdx.x, rank};
+    if (threadIdx.x == 0) s_wide = ws.order ? count_above(ws, nup, kthr) : nup;
+    __syncthreads();
+    const int H = s_wide, ncl = gridDim.x / WIDE_CTAS;
+    double *sm = cluster_map(smem_all, 0);
+    CoreShared &sh = *cluster_map(&s_sh, 0);
+    for (int h = blockIdx.x / WIDE_CTAS; h < H; h += ncl) {
+        const int slot = ws.heavy(h);
+        if (order_key(ws, slot) <= kthr) continue;
+        const int aux = (core_aux_doubles(ws, slot) + 1) & ~1;
+        tm.sync();  // the first CTA's shared memory is the previous update's no more (and exists)
+        core_update<RPL>(tm, ups, ws, p, slot, sm, smem_all + aux, smem_doubles - aux, sh);
+    }
+    if ((int) (blockIdx.x / WIDE_CTAS) < H) tm.sync();  // no CTA leaves while another reads its shared memory
+}
+
+// The recompression core of one update (slot) by one team: auxiliary arrays at sm, `pool_doubles` of shared
+// memory at pool (a cluster: of every CTA's own).
 template <int RPL, class TM>
 __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace &ws, const Params &p, int slot,
-                            double *sm, int smem_doubles, int &s_rot, int &s_rank, int &s_emax, double &s_amax) {
+                            double *sm, double *pool, int pool_doubles, CoreShared &sh) {
+    int &s_rot = sh.rot, &s_rank = sh.rank, &s_emax = sh.emax;
+    double &s_amax = sh.amax;
+    constexpr bool CLUSTER = TM::ctas > 1;
     int *meta = ws.meta + (size_t) slot * META_INTS;
     if (meta[META_STATUS] != HCGB_OK || !meta[META_CKIND]) return;
     const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
@@ -988,18 +1429,19 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
     double *dsc = nrm + ka + ka + 1;  // Jacobi column scales d and 1/d (2 ka)
     double *red = dsc + 2 * ka;
     int *redi = reinterpret_cast<int *>(red + SVD_RED_DOUBLES);
-    double *pool = red + SVD_RED_DOUBLES + SVD_REDI_INTS / 2;
-    const int pool_doubles = smem_doubles - (int) (pool - sm);
     // Working copy of M: shared memory when it fits, else the workspace.
     double *Mw;
     int ldw;
-    if ((long) kU * kV <= (long) pool_doubles) {
+    if (!CLUSTER && (long) kU * kV <= (long) pool_doubles) {
         Mw = pool;
         ldw = kU;
     } else {
         Mw = base + ws.off_m;
         ldw = ldm;
     }
+
+    // A cluster holds the columns of M in its CTAs' shared memory during the pivoted QR, where they fit.
+    const bool spread = CLUSTER && qrcp_cluster_doubles(kU, kV, TM::ctas) <= pool_doubles;
 
     const long long t0 = clock64();
     // 1. M = R_U R_V^T on DMMA (R_U = triu of the U stack's top kU rows, likewise R_V).
@@ -1018,11 +1460,11 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
             }
             const int col = tc * 8 + 2 * lc;
             if (i < kU && col < kV) {
-                Mw[i + (size_t) col * ldw] = d0;
+                if (!spread) Mw[i + (size_t) col * ldw] = d0;
                 Mc[i + (size_t) col * ldm] = d0;
             }
             if (i < kU && col + 1 < kV) {
-                Mw[i + (size_t) (col + 1) * ldw] = d1;
+                if (!spread) Mw[i + (size_t) (col + 1) * ldw] = d1;
                 Mc[i + (size_t) (col + 1) * ldm] = d1;
             }
         }
@@ -1046,9 +1488,11 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         }
     }
     const long long t1 = clock64();
-    int rk;
-    int eshift = 0;  // mixed form: Mw holds float-float values of M * 2^-eshift from here to step 4
-    if (p.mode == 1) {
+    int rk = 0;
+    double *XV = base + ws.off_xv;
+    double up = 1.0;  // mixed form: Mw holds float-float values of M / up from here to step 3
+    const bool ff = !CLUSTER && p.mode == 1;  // wide cores are FP64 in every form
+    if (ff) {
         // Exact power-of-two scaling that brings the largest entry of M near 1 (float range), then
         // the pivoted QR and the Jacobi sweeps in float-float arithmetic on the FP32 pipe.
         if (tm.tid == 0) s_emax = 0;
@@ -1060,7 +1504,8 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         }
         atomicMax(&s_emax, em);
         tm.sync();
-        eshift = s_emax ? s_emax - 1023 : 0;
+        const int eshift = s_emax ? s_emax - 1023 : 0;
+        up = __hiloint2double((1023 + eshift) << 20, 0);
         const double down = __hiloint2double((1023 - eshift) << 20, 0);
         df *Md = reinterpret_cast<df *>(Mw);
         for (int e = tm.tid; e < kU * kV; e += tm.nth) {
@@ -1071,91 +1516,80 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         const float stop2f = stop2 > 0.0 ? (float) (stop2 * down * down) : (float) stop2;
         rk = qrcp_truncated_df(tm, Md, ldw, kU, kV, stop2f, (float) (rel * rel), reinterpret_cast<df *>(nrm),
                                reinterpret_cast<df *>(inv), pvt, reinterpret_cast<float *>(red), redi);
+    } else if (spread) {
+        if constexpr (CLUSTER) rk = qrcp_cluster(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool);
     } else {
         rk = qrcp_truncated(tm, Mw, ldw, kU, kV, stop2, rel, nrm, inv, pvt, red, redi);
     }
     const long long t2 = clock64();
     if (rk < 1) rk = 1;
-    double *XV = base + ws.off_xv;
-    // 3. X = R(0:rk, :)^T (kV x rk), staged through XV, then into the working buffer (ld kV).
-    for (int i = warp; i < rk; i += nw)
-        for (int l = lane; l < kV; l += 32) XV[l + (size_t) i * ld] = l >= i ? Mw[i + (size_t) l * ldw] : 0.0;
+    // 3. X = R(0:rk, :)^T (kV x rk) in XV.
+    for (int i = spread ? rk : warp; i < rk; i += nw)
+        for (int l = lane; l < kV; l += 32) {
+            double x = 0.0;
+            if (l >= i) {
+                const double *e = Mw + i + (size_t) (ff ? l : pvt[l]) * ldw;  // the float-float QR swaps columns
+                x = ff ? (double) *reinterpret_cast<const df *>(e) * up : *e;
+            }
+            XV[l + (size_t) i * ld] = x;
+        }
     tm.sync();
     double *X = Mw;
     const int ldx = kV;
-    for (int i = warp; i < rk; i += nw)
-        for (int l = lane; l < kV; l += 32) X[l + (size_t) i * ldx] = XV[l + (size_t) i * ld];
-    tm.sync();
-
-    // 4. One-sided Jacobi on the rk columns of X (lane group sized to the column length kV).
-    //    X J = W with orthogonal columns: sigma_i = ||w_i||, right singular vectors P W Sigma^-1.
+    // 4. One-sided Jacobi on the rk columns of X: X J = W with orthogonal columns: sigma_i = ||w_i||, right
+    //    singular vectors P W Sigma^-1.  Preconditioned in single precision from precond_min columns on
+    //    (where its buffers fit); what that leaves, and smaller cores, go to the FP64 sweeps.
     int sweeps = 0;
     bool converged = true;
     const double tol64 = 8.0 * DBL_EPSILON * (double) (kV > 1 ? kV : 1);
-    if (p.mode == 1) {
-        // Mixed form: X = R_rk^T is already float-float (scaled by 2^-eshift); the sweeps run in
-        // float-float arithmetic, every per-pair quantity included (see jacobi_sweep_df).
-        df *Xd = reinterpret_cast<df *>(X);
-        const double up = __hiloint2double((1023 + eshift) << 20, 0);
-        const float tol_df = 16.f * 3.5527137e-15f * (float) (kV > 1 ? kV : 1);
-        // norms and scales as float-float values in the (double-sized) nrm and dsc arrays
-        jacobi_df_dispatch<RPL>(tm, Xd, ldx, kV, rk, reinterpret_cast<df *>(nrm), reinterpret_cast<df *>(dsc),
-                                reinterpret_cast<df *>(dsc + ka), &s_rot, reinterpret_cast<float *>(&s_amax),
-                                &sweeps, &converged, tol_df, MAX_JACOBI_SWEEPS);
-        for (int e = tm.tid; e < kV * rk; e += tm.nth) {
-            const size_t o = (e % kV) + (size_t) (e / kV) * ldx;
-            X[o] = (double) Xd[o] * up;
+    const double *Xs = XV;
+    int lds = ld;
+    if (rk >= p.precond_min && rk >= 4) {
+        PrecondBuffers b;
+        const int x4 = (kV + 3) >> 2, j4 = (rk + 3) >> 2;
+        bool fits;
+        if constexpr (CLUSTER) {
+            b.ls4 = x4 + j4;
+            b.y = reinterpret_cast<float4 *>(base + ws.off_mixed);
+            b.buf = reinterpret_cast<float4 *>(pool);
+            b.buf_quads = pool_doubles / 2;
+            b.wh = reinterpret_cast<df *>(XV);
+            b.ldh = ld;
+            b.v = reinterpret_cast<float *>(b.y);
+            b.ldv = 4 * b.ls4;
+            fits = 4 * (size_t) b.ls4 * rk <= (size_t) ws.kmax * (ws.kmax + ws.ld) && 2 * b.ls4 <= b.buf_quads;
+        } else {
+            b.ls4 = ((x4 + j4 + 3) & ~7) + 4;  // 4 mod 8 quads: two 4-lane groups a quarter-warp, no bank conflicts
+            const int skip = (int) ((reinterpret_cast<uintptr_t>(pool) >> 3) & 1);
+            b.y = reinterpret_cast<float4 *>(pool + skip);
+            b.buf = nullptr;
+            b.buf_quads = 0;
+            b.wh = reinterpret_cast<df *>(pool);
+            b.ldh = (long) (kV | 1) * rk <= (long) pool_doubles ? (kV | 1) : kV;
+            b.v = reinterpret_cast<float *>(base + ws.off_mixed);
+            b.ldv = rk;
+            fits = Mw == pool && 2L * b.ls4 * rk + skip <= (long) pool_doubles;
         }
-        tm.sync();
+        b.e64 = base + ws.off_m;
+        b.w = base + ws.off_mixed;
+        if (fits && jacobi_precond(tm, XV, ld, kV, rk, b, reinterpret_cast<df *>(nrm), perm, &s_rot, &s_emax,
+                                   &sh.cosine, &sh.tangent, (float) tol64, &sweeps, &converged)) {
+            Xs = b.w;
+            lds = kV;
+            if (converged) sweeps = -sweeps;
+        }
+    }
+    tm.sync();
+    for (int i = warp; i < rk; i += nw)
+        for (int l = lane; l < kV; l += 32) X[l + (size_t) i * ldx] = Xs[l + (size_t) i * lds];
+    tm.sync();
+    if (sweeps < 0) {
+        sweeps = -sweeps;  // the corrections left orthogonal columns
     } else {
-        // X32 (kV x rk floats) and J (rk x rk float-float): in shared memory behind X when they fit
-        // the team's pool, else in the float region of the slot.
-        const size_t x32_floats = ((size_t) kV * rk + 1) & ~size_t(1);
-        const size_t pre_doubles = x32_floats / 2 + (size_t) rk * rk;
-        const bool in_smem = Mw == pool && (size_t) kV * rk + pre_doubles <= (size_t) pool_doubles;
-        const bool fits = in_smem || x32_floats + 2 * (size_t) rk * rk <= (size_t) ws.kmax * (ws.kmax + ws.ld);
-        if (rk >= p.precond_min && fits) {
-            // FP32 sweeps with accumulated rotations (FP32 pipe), then X <- X J in FP64: the FP64
-            // sweeps below start from a nearly orthogonal X and need about half as many.
-            float *X32 = reinterpret_cast<float *>(in_smem ? pool + (size_t) kV * rk : base + ws.off_mixed);
-            df *J32 = reinterpret_cast<df *>(X32 + x32_floats);
-            if (tm.tid == 0) s_emax = 0;
-            tm.sync();
-            int em = 0;
-            for (int e = tm.tid; e < kV * rk; e += tm.nth) {
-                const int ef = (int) ((__double_as_longlong(X[(e % kV) + (size_t) (e / kV) * ldx]) >> 52) & 0x7ff);
-                em = em > ef ? em : ef;
-            }
-            atomicMax(&s_emax, em);
-            tm.sync();
-            const int esc = s_emax ? s_emax - 1023 : 0;
-            const double down = __hiloint2double((1023 - esc) << 20, 0);
-            for (int e = tm.tid; e < kV * rk; e += tm.nth)
-                X32[e] = (float) (X[(e % kV) + (size_t) (e / kV) * ldx] * down);
-            tm.sync();
-            jacobi_precond32(tm, X32, kV, rk, J32, PRECOND_TOL32, PRECOND_MAX_SWEEPS, &s_rot);
-            // XV (ld ws.ld) <- X J32 in FP64, then back into X
-            for (int e = tm.tid; e < kV * rk; e += tm.nth) {
-                const int r = e % kV, c = e / kV;
-                const df *jc = J32 + (size_t) c * rk;
-                double s0 = 0.0, s1 = 0.0;
-                int l = 0;
-                for (; l + 1 < rk; l += 2) {
-                    s0 = fma(X[r + (size_t) l * ldx], (double) jc[l], s0);
-                    s1 = fma(X[r + (size_t) (l + 1) * ldx], (double) jc[l + 1], s1);
-                }
-                if (l < rk) s0 = fma(X[r + (size_t) l * ldx], (double) jc[l], s0);
-                XV[r + (size_t) c * ld] = s0 + s1;
-            }
-            tm.sync();
-            for (int e = tm.tid; e < kV * rk; e += tm.nth) {
-                const int r = e % kV, c = e / kV;
-                X[r + (size_t) c * ldx] = XV[r + (size_t) c * ld];
-            }
-            tm.sync();
-        }
-        jacobi_dispatch<RPL>(tm, X, ldx, kV, rk, nrm, &s_rot, &s_amax, &sweeps, &converged, tol64, MAX_JACOBI_SWEEPS,
-                             dsc, ka, Mw == pool);
+        int more = 0;
+        jacobi_dispatch<RPL>(tm, X, ldx, kV, rk, nrm, &s_rot, &s_amax, &more, &converged, tol64, MAX_JACOBI_SWEEPS, dsc,
+                             ka, Mw == pool);
+        sweeps += more;
     }
 
     const long long t3 = clock64();
@@ -1264,7 +1698,7 @@ int svd_team_doubles(int kmax) {
         return v > 0 ? v : 48 * 1024;
     }();
     const long aux = 6L * kmax + SVD_AUX_FIXED;
-    const long want = aux + (long) kmax * kmax;
+    const long want = aux + (long) kmax * kmax + 14L * kmax;  // the square, or the preconditioner's padded columns
     const long cap = (optin - 256) / 2 / (long) sizeof(double);
     long t = want < cap ? want : cap;
     if (t < aux) t = aux;  // checked against the device limit by the caller
@@ -1275,27 +1709,28 @@ int svd_team_doubles(int kmax) {
 
 size_t svd_smem_bytes(int kmax) { return 2 * sizeof(double) * (size_t) svd_team_doubles(kmax); }
 
-template <int RPL>
-static void launch_core_svd_t(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {
+// Register tiles of the FP64 sweeps: up to 16 rows a lane (longer columns take the looped sweep).
+constexpr int CORE_RPL = 16;
+
+void launch_core_svd(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {
     const int team = svd_team_doubles(ws.kmax);
     const size_t smem = 2 * sizeof(double) * (size_t) team;
-    // Heavy: a core of k columns (its aux arrays, 6 k + SVD_AUX_FIXED doubles, and a k x k working
+    // Wide: a core of k columns (its aux arrays, 6 k + SVD_AUX_FIXED doubles, and a k x k working
     // copy) does not fit the half-CTA team's shared memory; small: it fits a quarter-CTA team's.
     auto fits = [](long k, long doubles) { return k * k + 6 * k + SVD_AUX_FIXED <= doubles; };
     int kthr = 0, kthr4 = 0;
     while (fits(kthr + 1, team)) kthr++;
     while (fits(kthr4 + 1, team / 2)) kthr4++;
-    cudaFuncSetAttribute(core_svd_kernel<RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    { core_svd_kernel<RPL><<<n, SVD_THREADS, smem, st>>>(ups, n, ws, p, team, kthr, kthr4); note_launch(); }
-}
-
-// Rows of M are at most min(ld, kmax); the register tile of a rotation covers 32 * RPL rows.
-void launch_core_svd(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {
-    const int rows = ws.ld < ws.kmax ? ws.ld : ws.kmax;
-    if (rows <= 128) launch_core_svd_t<4>(ups, n, ws, p, st);
-    else if (rows <= 256) launch_core_svd_t<8>(ups, n, ws, p, st);
-    else if (rows <= 512) launch_core_svd_t<16>(ups, n, ws, p, st);
-    else launch_core_svd_t<32>(ups, n, ws, p, st);
+    if (ws.kmax > kthr) {
+        const int aux = 6 * ws.kmax + SVD_AUX_FIXED + 1;
+        const int doubles = std::min(aux + WIDE_POOL_DOUBLES, 2 * team);
+        const size_t bytes = sizeof(double) * (size_t) doubles;
+        cudaFuncSetAttribute(core_wide_kernel<CORE_RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
+        const int ctas = std::min(n, WIDE_CLUSTERS) * WIDE_CTAS;
+        { core_wide_kernel<CORE_RPL><<<ctas, SVD_THREADS, bytes, st>>>(ups, n, ws, p, doubles, kthr); note_launch(); }
+    }
+    cudaFuncSetAttribute(core_svd_kernel<CORE_RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    { core_svd_kernel<CORE_RPL><<<n, SVD_THREADS, smem, st>>>(ups, n, ws, p, team, kthr, kthr4); note_launch(); }
 }
 
 }  // namespace hcgb

@@ -182,10 +182,10 @@ int hcgb_set_graph(hcgb_context *ctx, int enable);
  * least wy_min_reflectors reflectors (default 48). */
 int hcgb_set_tuning(hcgb_context *ctx, int oz_min_outputs, int wy_min_reflectors);
 
-/* Plain form: a core SVD with at least min_cols Jacobi columns first runs one-sided Jacobi sweeps in
- * FP32 with the rotations accumulated in float-float (J orthogonal to ~1e-13), then X <- X J in FP64
- * and FP64 sweeps to working precision; smaller cores run FP64 sweeps only.  min_cols = 0 restores
- * the default (off: a value above every core width); same results up to rounding. */
+/* A core SVD with at least min_cols Jacobi columns finds its rotations in FP32 sweeps (accumulated, made
+ * orthogonal to ~1e-15), forms X <- X J in FP64 and corrects the columns to working precision; smaller
+ * cores, and what the corrections leave, run FP64 sweeps.  min_cols = 0 restores the default (16); a
+ * value above every core width turns it off; same results up to rounding. */
 int hcgb_set_precond(hcgb_context *ctx, int min_cols);
 
 /* Learned form: an update is sketched only when its sketch (predicted rank + 8 oversampling + 4

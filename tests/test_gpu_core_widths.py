@@ -1,0 +1,70 @@
+"""The recompression core at the edges of its classes: stack widths around the preconditioner's smallest core
+(16 columns), the quarter- and half-CTA teams' shared memory (82 and 117 columns), the wide cores of a
+thread-block cluster, odd sizes, slow and fast decay, nearly equal singular values."""
+import numpy as np
+import pytest
+
+from oracle import hcore_oracle as O
+from tests.helpers import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+
+
+@pytest.fixture(scope="module")
+def T():
+    import torch
+    assert torch.cuda.is_available()
+    from hcorepp_gb300 import tiles
+    return tiles
+
+
+def _factor(rng, m, n, s):
+    """A compressed tile with singular values s: U orthonormal, rows of V orthogonal."""
+    r = len(s)
+    u = np.linalg.qr(rng.standard_normal((m, r)))[0]
+    v = np.linalg.qr(rng.standard_normal((n, r)))[0]
+    return u, s[:, None] * v.T
+
+
+def _spectrum(kind, r, top):
+    if kind == "decay":      # the kernels' own: down to the accuracy
+        return top * np.logspace(0, -8, r)
+    if kind == "slow":       # nothing to truncate
+        return top * np.linspace(1.0, 0.5, r)
+    s = np.repeat(np.logspace(0, -7, (r + 2) // 3), 3)[:r]  # "triples": clusters of equal singular values
+    return top * s
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("kind", ["decay", "slow", "triples"])
+@pytest.mark.parametrize("n,rc,ra", [(40, 7, 8), (40, 8, 9), (75, 33, 31), (300, 41, 41), (301, 42, 41), (300, 60, 57),
+                                     (301, 61, 57), (299, 80, 75), (320, 120, 105), (512, 170, 170)])
+def test_recompression_at_class_edges(T, n, rc, ra, kind, mode):
+    rng = np.random.default_rng([n, rc, ra, len(kind)])
+    acc, k, cap = 1e-8, rc + ra, min(n, rc + ra)
+    cu, cv = _factor(rng, n, n, _spectrum(kind, rc, 1.0))
+    au, av = _factor(rng, n, n, _spectrum(kind, ra, 0.7))
+    bu, bv = _factor(rng, n, n, np.ones(min(n, ra + 3)))
+    oc = O.CompressedTile(cu, cv, cap)
+    oa = O.CompressedTile(au, av, cap)
+    ob = O.CompressedTile(bu, bv, max(cap, bu.shape[1]))
+    gc, ga = (T.CompressedTile(n, n, t.u, t.v, max_rank=cap) for t in (oc, oa))
+    gb = T.CompressedTile(n, n, bu, bv, max_rank=max(cap, bu.shape[1]))
+    exact = oa.to_dense() @ ob.to_dense() + oc.to_dense()
+    O.hcore_gemm(1.0, oa, ob, 1.0, oc, O.CompressionParameters(acc, truncated_svd=True))
+    T.HCore.Gemm(1.0, ga, 0, gb, 0, 1.0, gc, T.CompressionParameters(acc, truncated_svd=True, mode=mode))
+    assert abs(gc.rank - oc.rank) <= 1
+    assert rel_fro(gc.to_dense(), exact) <= 2 * max(rel_fro(oc.to_dense(), exact), acc)
+    # V's rows are singular vectors: orthogonal to the sweeps' tolerance (8 eps k) plus the rounding of the Q application, a few units of roundoff
+    # (2^-48 in the float-float form) a reflector
+    v = np.asarray(gc.v(), dtype=np.float64)
+    norms = np.linalg.norm(v, axis=1)
+    assert np.all(norms > 0)
+    g = np.abs((v / norms[:, None]) @ (v / norms[:, None]).T - np.eye(len(norms)))
+    unit = EPS / 2 if mode == 0 else 2.0 ** -48
+    assert g.max() <= 64 * k * unit
+    # U = M XV Sigma^-2: orthonormal up to rounding relative to the smallest kept singular value
+    u = np.asarray(gc.u(), dtype=np.float64)
+    assert np.abs(u.T @ u - np.eye(u.shape[1])).max() <= 64 * k * unit * norms.max() / norms.min()
