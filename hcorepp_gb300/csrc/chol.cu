@@ -3,8 +3,7 @@
 // Replace HCoreKernels<T>::potrf / trsm / syrk on the GPU (src/kernels/cuda/kernels.cpp:290-306,
 // src/kernels/cuda/CudaKernels.cu:1019-1049: cuSOLVER Xpotrf, cuBLAS trsm/syrk) with the
 // semantics of LAPACK dpotrf and BLAS dtrsm / dsyrk (column-major), which the CPU backend calls
-// (src/kernels/omp/kernels.cpp:234-282).  One CTA per call: these operate on one tile (nb <= 1024)
-// and sit off the GEMM hot path.
+// (src/kernels/omp/kernels.cpp:234-282).
 #include "internal.cuh"
 
 namespace hcgb {
@@ -13,52 +12,135 @@ namespace {
 
 constexpr int CT = 1024;
 
-__device__ double block_reduce_sum(double v, double *red) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    v = warp_sum(v);
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        double t = lane < nw ? red[lane] : 0.0;
-        t = warp_sum(t);
-        if (lane == 0) red[32] = t;
+// Blocked right-looking Cholesky.  One launch per 32-column block solves the rows below it, one updates the
+// trailing 32 x 32 tiles over the whole GPU; the CTA of the next diagonal tile factors it on the spot, so a
+// block costs two launches.  (One CTA walking the columns, each a left-looking product from L2, took 55 ms
+// for n = 512: one SM's FP64 pipe and dependent loads.)  L(i, k) stands at A[i rs + k cs]: lower triangle
+// rs = 1, cs = lda, upper the other way round.  Every L(i, j) takes its products in ascending k.
+constexpr int PB = 32;
+
+// Factors the leading nb x nb block held in shared memory (lower part); returns the failing column + 1 or 0.
+__device__ int potrf_block(double (*T)[PB + 1], int nb) {
+    for (int j = 0; j < nb; j++) {
+        const double d = T[j][j];
+        if (!(d > 0.0)) return j + 1;
+        const double ljj = sqrt(d);
+        __syncthreads();
+        if (threadIdx.x == 0) T[j][j] = ljj;
+        for (int i = j + 1 + (int) threadIdx.x; i < nb; i += blockDim.x) T[i][j] /= ljj;
+        __syncthreads();
+        for (int e = threadIdx.x; e < (nb - 1 - j) * PB; e += blockDim.x) {
+            const int i = j + 1 + e / PB, k = e % PB;
+            if (k > j && k <= i) T[i][k] = fma(-T[i][j], T[k][j], T[i][k]);
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    return red[32];
+    return 0;
 }
 
-// Left-looking Cholesky of the lower (uplo 0) or upper (uplo 1) triangle of A (n x n, ld lda).
-// info: 0, or j + 1 when the leading minor of order j + 1 is not positive (dpotrf's convention;
-// the factorisation stops there).  The other triangle is not referenced.
-__global__ void __launch_bounds__(CT) potrf_kernel(double *A, int n, int lda, int uplo, int *info) {
-    __shared__ double red[40];
-    __shared__ int s_info;
-    if (threadIdx.x == 0) s_info = 0;
-    __syncthreads();
-    // L(i, k) for the lower case; the upper case stores U(k, i) = L(i, k).
-    auto L = [&](int i, int k) -> double & { return uplo == 0 ? A[i + (size_t) k * lda] : A[k + (size_t) i * lda]; };
-    for (int j = 0; j < n; j++) {
-        double part = 0.0;
-        for (int k = threadIdx.x; k < j; k += blockDim.x) part = fma(L(j, k), L(j, k), part);
-        const double s = block_reduce_sum(part, red);
-        const double d = L(j, j) - s;
-        if (!(d > 0.0)) {
-            if (threadIdx.x == 0) s_info = j + 1;
-            __syncthreads();
-            break;
-        }
-        const double ljj = sqrt(d);
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-            double t = L(i, j);
-            for (int k = 0; k < j; k++) t = fma(-L(i, k), L(j, k), t);
-            L(i, j) = t / ljj;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) L(j, j) = ljj;
-        __syncthreads();
+__global__ void __launch_bounds__(256) potrf_first_kernel(double *A, int n, int rs, int cs, int *info) {
+    __shared__ double T[PB][PB + 1];
+    const int nb = n < PB ? n : PB;
+    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
+        const int i = e % nb, k = e / nb;
+        if (i >= k) T[i][k] = A[(size_t) i * rs + (size_t) k * cs];
     }
-    if (threadIdx.x == 0 && info) *info = s_info;
+    __syncthreads();
+    const int bad = potrf_block(T, nb);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
+        const int i = e % nb, k = e / nb;
+        if (i >= k) A[(size_t) i * rs + (size_t) k * cs] = T[i][k];
+    }
+    if (threadIdx.x == 0) *info = bad;
+}
+
+// Rows below block column j0 (width PB): 32 rows a CTA, four threads a row, each with every fourth column.
+__global__ void __launch_bounds__(128) potrf_panel_kernel(double *A, int n, int j0, int rs, int cs, const int *info) {
+    __shared__ double D[PB][PB + 1];
+    if (*info) return;
+    for (int e = threadIdx.x; e < PB * PB; e += blockDim.x) {
+        const int i = e % PB, k = e / PB;
+        D[i][k] = i >= k ? A[(size_t) (j0 + i) * rs + (size_t) (j0 + k) * cs] : 0.0;
+    }
+    __syncthreads();
+    const int row = j0 + PB + blockIdx.x * 32 + (threadIdx.x >> 2), q = threadIdx.x & 3;
+    const bool in = row < n;
+    double *r = A + (size_t) (in ? row : 0) * rs + (size_t) j0 * cs;
+    double t[PB / 4];
+#pragma unroll
+    for (int u = 0; u < PB / 4; u++) t[u] = in ? r[(size_t) (4 * u + q) * cs] : 0.0;
+#pragma unroll
+    for (int j = 0; j < PB; j++) {
+        double x = t[j / 4] / D[j][j];
+        x = __shfl_sync(0xffffffffu, x, j & 3, 4);
+        if (q == (j & 3)) t[j / 4] = x;
+#pragma unroll
+        for (int u = 0; u < PB / 4; u++) {
+            const int k = 4 * u + q;
+            if (4 * u + 3 > j && k > j) t[u] = fma(-x, D[k][j], t[u]);
+        }
+    }
+    if (in)
+#pragma unroll
+        for (int u = 0; u < PB / 4; u++) r[(size_t) (4 * u + q) * cs] = t[u];
+}
+
+// Trailing tiles (ti, tj), ti >= tj, behind block column j0: A -= L_i L_j^T; tile (0, 0) is factored too.
+__global__ void __launch_bounds__(256) potrf_update_kernel(double *A, int n, int j0, int rs, int cs, int *info) {
+    __shared__ double Li[PB][PB + 1], Lj[PB][PB + 1];
+    if (*info) return;  // written by tile (0, 0) alone, after every earlier launch
+    int ti = 0, base = 0;
+    while (base + ti + 1 <= (int) blockIdx.x) {
+        base += ti + 1;
+        ti++;
+    }
+    const int tj = (int) blockIdx.x - base, i0 = j0 + PB * (1 + ti), k0 = j0 + PB * (1 + tj);
+    const int ni = n - i0 < PB ? n - i0 : PB, nk = n - k0 < PB ? n - k0 : PB;
+    for (int e = threadIdx.x; e < PB * PB; e += blockDim.x) {
+        const int i = e % PB, l = e / PB;
+        Li[i][l] = i < ni ? A[(size_t) (i0 + i) * rs + (size_t) (j0 + l) * cs] : 0.0;
+        Lj[i][l] = i < nk ? A[(size_t) (k0 + i) * rs + (size_t) (j0 + l) * cs] : 0.0;
+    }
+    __syncthreads();
+    const int x = threadIdx.x & 15, y = threadIdx.x >> 4;
+    double t[2][2];
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+            const int i = x + 16 * u, k = y + 16 * v;
+            t[u][v] = (i < ni && k < nk && i0 + i >= k0 + k) ? A[(size_t) (i0 + i) * rs + (size_t) (k0 + k) * cs] : 0.0;
+        }
+#pragma unroll 4
+    for (int l = 0; l < PB; l++) {
+        const double a0 = Li[x][l], a1 = Li[x + 16][l], b0 = Lj[y][l], b1 = Lj[y + 16][l];
+        t[0][0] = fma(-a0, b0, t[0][0]);
+        t[0][1] = fma(-a0, b1, t[0][1]);
+        t[1][0] = fma(-a1, b0, t[1][0]);
+        t[1][1] = fma(-a1, b1, t[1][1]);
+    }
+    const bool next = ti == 0;
+    if (next) __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int v = 0; v < 2; v++) {
+            const int i = x + 16 * u, k = y + 16 * v;
+            if (i < ni && k < nk && i0 + i >= k0 + k) {
+                if (next) Li[i][k] = t[u][v];
+                else A[(size_t) (i0 + i) * rs + (size_t) (k0 + k) * cs] = t[u][v];
+            }
+        }
+    if (!next) return;
+    __syncthreads();
+    const int bad = potrf_block(Li, ni);
+    __syncthreads();
+    for (int e = threadIdx.x; e < ni * ni; e += blockDim.x) {
+        const int i = e % ni, k = e / ni;
+        if (i >= k) A[(size_t) (i0 + i) * rs + (size_t) (i0 + k) * cs] = Li[i][k];
+    }
+    if (threadIdx.x == 0 && bad) *info = i0 + bad;
 }
 
 // op(A) X = alpha B (side 0) or X op(A) = alpha B (side 1); X overwrites B (m x n, ld ldb).
@@ -122,32 +204,72 @@ __global__ void fill_triangle_kernel(int uplo, int n, double *A, int lda, double
 
 // Panel solve of a tile Cholesky step: for every compressed_vt tile of the panel, W <- L^-1 W
 // (Left, Lower, NoTrans, NonUnit, alpha 1 on the W region, rows x rank, ld rows): HCore<T>::Trsm
-// as the tile Cholesky applies it (src/api/HCore.cpp:623-647), one CTA per tile, the rank read on
-// the device.  Same operations in the same order as trsm_kernel, so the results are identical.
-__global__ void __launch_bounds__(256) trsm_panel_kernel(const double *L, int nb, int ldl, const DevTile *tiles) {
-    const DevTile t = tiles[blockIdx.x];
-    const int r = *t.rank;
-    if (r <= 0 || r > t.max_rank || t.rows != nb) return;
-    double *W = t.v;
-    const int ld = t.rows;
-    for (int i = 0; i < nb; i++) {
-        const double lii = L[i + (size_t) i * ldl];
-        for (int c = threadIdx.x; c < r; c += blockDim.x) W[i + (size_t) c * ld] /= lii;
+// as the tile Cholesky applies it (src/api/HCore.cpp:623-647), the rank read on the device.  One CTA per
+// tile and TRSM_COLS columns, which stay in shared memory: blocks of 32 rows are solved, then taken out of
+// the rows below.  Every element takes the same operations in the same order as in trsm_kernel, so the
+// results are identical.  (One CTA per tile, one row a step through L2: 15 ms for 512 rows and 100 columns.)
+constexpr int TRSM_COLS = 4, TRSM_THREADS = 256;
+__global__ void __launch_bounds__(TRSM_THREADS) trsm_panel_kernel(const double *L, int nb, int ldl, const DevTile *tiles,
+                                                                  int in_smem) {
+    extern __shared__ double smem_w[];  // nb x TRSM_COLS, where that fits
+    __shared__ double D[PB][PB + 1];
+    const DevTile t = tiles[blockIdx.y];
+    const int r = *t.rank, c0 = blockIdx.x * TRSM_COLS;
+    if (r <= 0 || r > t.max_rank || t.rows != nb || c0 >= r) return;
+    const int nc = r - c0 < TRSM_COLS ? r - c0 : TRSM_COLS;
+    double *W = t.v + (size_t) c0 * nb;
+    double *Ws = in_smem ? smem_w : W;
+    if (in_smem)
+        for (int e = threadIdx.x; e < nb * nc; e += TRSM_THREADS) Ws[e] = W[e];
+    for (int i0 = 0; i0 < nb; i0 += PB) {
+        const int ni = nb - i0 < PB ? nb - i0 : PB;
         __syncthreads();
-        const int rest = nb - 1 - i;
-        for (int e = threadIdx.x; e < rest * r; e += blockDim.x) {
-            const int q = e % rest, c = e / rest;
-            const int k = i + 1 + q;
-            W[k + (size_t) c * ld] = fma(-L[k + (size_t) i * ldl], W[i + (size_t) c * ld], W[k + (size_t) c * ld]);
+        for (int e = threadIdx.x; e < ni * ni; e += TRSM_THREADS) {
+            const int i = e % ni, k = e / ni;
+            if (i >= k) D[i][k] = L[(i0 + i) + (size_t) (i0 + k) * ldl];
         }
         __syncthreads();
+        if ((int) threadIdx.x < 32 * nc) {  // a warp per column, a lane per row
+            const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            double w = lane < ni ? Ws[i0 + lane + c * nb] : 0.0;
+            for (int i = 0; i < ni; i++) {
+                if (lane == i) w /= D[i][i];
+                const double wi = __shfl_sync(0xffffffffu, w, i);
+                if (lane > i && lane < ni) w = fma(-D[lane][i], wi, w);
+            }
+            if (lane < ni) Ws[i0 + lane + c * nb] = w;
+        }
+        __syncthreads();
+        for (int k = i0 + ni + threadIdx.x; k < nb; k += TRSM_THREADS) {
+            double w[TRSM_COLS];
+#pragma unroll
+            for (int c = 0; c < TRSM_COLS; c++) w[c] = c < nc ? Ws[k + c * nb] : 0.0;
+#pragma unroll 8
+            for (int i = 0; i < ni; i++) {
+                const double l = -L[k + (size_t) (i0 + i) * ldl];
+#pragma unroll
+                for (int c = 0; c < TRSM_COLS; c++)
+                    if (c < nc) w[c] = fma(l, Ws[i0 + i + c * nb], w[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < TRSM_COLS; c++)
+                if (c < nc) Ws[k + c * nb] = w[c];
+        }
     }
+    __syncthreads();
+    if (in_smem)
+        for (int e = threadIdx.x; e < nb * nc; e += TRSM_THREADS) W[e] = Ws[e];
 }
 
 }  // namespace
 
-void launch_trsm_panel(const double *L, int nb, int ldl, const DevTile *tiles, int count, cudaStream_t st) {
-    if (count > 0) { trsm_panel_kernel<<<count, 256, 0, st>>>(L, nb, ldl, tiles); note_launch(); }
+void launch_trsm_panel(const double *L, int nb, int ldl, const DevTile *tiles, int count, int max_rank, cudaStream_t st) {
+    if (count <= 0 || max_rank <= 0) return;
+    size_t smem = sizeof(double) * (size_t) nb * TRSM_COLS;
+    if (smem > 200 * 1024) smem = 0;
+    cudaFuncSetAttribute(trsm_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    const dim3 grid((max_rank + TRSM_COLS - 1) / TRSM_COLS, count);
+    { trsm_panel_kernel<<<grid, TRSM_THREADS, smem, st>>>(L, nb, ldl, tiles, smem > 0); note_launch(); }
 }
 
 void launch_fill_triangle(int uplo, int n, double *A, int lda, double value, cudaStream_t st) {
@@ -156,7 +278,13 @@ void launch_fill_triangle(int uplo, int n, double *A, int lda, double value, cud
 }
 
 void launch_potrf(double *A, int n, int lda, int uplo, int *info_dev, cudaStream_t st) {
-    { potrf_kernel<<<1, CT, 0, st>>>(A, n, lda, uplo, info_dev); note_launch(); }
+    const int rs = uplo == 0 ? 1 : lda, cs = uplo == 0 ? lda : 1;
+    { potrf_first_kernel<<<1, 256, 0, st>>>(A, n, rs, cs, info_dev); note_launch(); }
+    for (int j0 = 0; j0 + PB < n; j0 += PB) {
+        const int rest = (n - j0 - 1) / PB;  // row blocks below
+        { potrf_panel_kernel<<<rest, 128, 0, st>>>(A, n, j0, rs, cs, info_dev); note_launch(); }
+        { potrf_update_kernel<<<rest * (rest + 1) / 2, 256, 0, st>>>(A, n, j0, rs, cs, info_dev); note_launch(); }
+    }
 }
 
 void launch_trsm(int side, int uplo, int trans, int diag, int m, int n, double alpha, const double *A, int lda,

@@ -1224,10 +1224,14 @@ extern "C" int hcgb_tile_cholesky(hcgb_context *ctx, int nt, const hcgb_tile *gr
         if (k == nt - 1) break;
         // Panel: W_ik <- L_kk^-1 W_ik for every i > k.
         std::vector<DevTile> panel;
-        for (int i = k + 1; i < nt; i++) panel.push_back(to_dev(tile(i, k)));
+        int widest = 0;
+        for (int i = k + 1; i < nt; i++) {
+            panel.push_back(to_dev(tile(i, k)));
+            widest = std::max(widest, tile(i, k).max_rank);
+        }
         HCGB_CUDA(ctx, cudaMemcpyAsync(dpanel, panel.data(), sizeof(DevTile) * panel.size(), cudaMemcpyHostToDevice,
                                        ctx->stream));
-        launch_trsm_panel(tile(k, k).data, nb, nb, dpanel, (int) panel.size(), ctx->stream);
+        launch_trsm_panel(tile(k, k).data, nb, nb, dpanel, (int) panel.size(), widest, ctx->stream);
         HCGB_CUDA(ctx, cudaGetLastError());
         // Trailing updates A_ij -= A_ik A_jk^T (j <= i): Syrk on the diagonal, Gemm(aCholesky) below.
         // B = A_jk^T is the stored compressed_vt tile with its factors swapped (U' = W, W' = U).

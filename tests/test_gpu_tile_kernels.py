@@ -1,0 +1,86 @@
+"""The blocked tile kernels at the edges of their blocks: Cholesky factorisation (32-column blocks), the panel
+solve of the tile Cholesky (32 rows, 4 columns)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import hcore_oracle as O
+from tests.helpers import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+EPS = np.finfo(np.float64).eps
+
+
+@pytest.fixture(scope="module")
+def T():
+    import torch
+    assert torch.cuda.is_available()
+    from hcorepp_gb300 import tiles
+    return tiles
+
+
+def _potrf(T, a, uplo, lda=None):
+    import torch
+    n = a.shape[0]
+    lda = lda or n
+    buf = np.full((lda, n), 7.0, order="F")
+    buf[:n] = a
+    d = torch.from_numpy(buf.ravel(order="F").copy()).cuda()
+    info = T.Blas.potrf(uplo, n, d, lda)
+    out = d.cpu().numpy().reshape((lda, n), order="F")
+    assert np.all(out[n:] == 7.0)
+    return info, out[:n]
+
+
+@pytest.mark.parametrize("uplo", [0, 1])
+@pytest.mark.parametrize("n,lda", [(1, 1), (31, 31), (32, 40), (33, 33), (64, 64), (97, 101), (300, 300)])
+def test_potrf_blocks(T, n, lda, uplo):
+    rng = np.random.default_rng(n)
+    g = rng.standard_normal((n, n + 3))
+    a = g @ g.T + n * np.eye(n)
+    stored = np.tril(a) + np.triu(np.full((n, n), -3.0), 1) if uplo == 0 else np.triu(a) + np.tril(np.full((n, n), -3.0), -1)
+    info, out = _potrf(T, stored, uplo, lda)
+    assert info == 0
+    f = np.tril(out) if uplo == 0 else np.triu(out).T
+    # the other triangle is not touched; |A - L L^T| <= gamma_{n+1} |L| |L|^T (Higham, Theorem 10.3)
+    other = np.triu(out, 1) if uplo == 0 else np.tril(out, -1)
+    assert np.array_equal(other, np.triu(stored, 1) if uplo == 0 else np.tril(stored, -1))
+    assert np.all(np.abs(f @ f.T - a) <= 2 * (n + 2) * EPS * (np.abs(f) @ np.abs(f).T))
+
+
+@pytest.mark.parametrize("n,bad", [(5, 0), (40, 31), (40, 32), (70, 69), (70, 40)])
+def test_potrf_reports_the_first_failing_minor(T, n, bad):
+    a = np.eye(n)
+    a[bad, bad] = -1.0
+    assert _potrf(T, a, 0)[0] == bad + 1
+
+
+@pytest.mark.parametrize("nb,nt", [(33, 3), (100, 4), (64, 3)])
+def test_cholesky_panel_solve_matches_the_tile_loop(T, nb, nt):
+    """The batched driver and the per-tile calls give the same bits."""
+    import torch
+    from hcorepp_gb300 import _lib as L
+    from hcorepp_gb300.problems import KernelMatrix
+    km = KernelMatrix(nb * nt, nb, 3, 0.2, 2, diag_shift=1e-2)
+    kinds = [[L.DENSE if i == j else L.COMPRESSED if i > j else None for j in range(nt)] for i in range(nt)]
+    params = T.CompressionParameters(1e-8, truncated_svd=True)
+    out = []
+    for batched in (True, False):
+        tm = T.TileMatrix(nt, nt, nb, kinds, nb, vt=True)
+        for j in range(nt):
+            for i in range(j, nt):
+                d = km.tile(i, j)
+                if i == j:
+                    tm.set_tile(i, j, dense=d)
+                else:
+                    t = O.CompressedTile.from_dense(d, O.CompressionParameters(1e-8, truncated_svd=True), max_rank=nb)
+                    tm.set_tile(i, j, u=t.u, v=t.v)
+        assert T.tile_cholesky(tm, params, batched=batched) == 0
+        torch.cuda.synchronize()
+        out.append((tm.rank_grid(), np.tril(tm.to_dense())))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    a = np.block([[km.tile(i, j) for j in range(nt)] for i in range(nt)])
+    assert rel_fro(out[0][1] @ out[0][1].T, a) < 1e-7
