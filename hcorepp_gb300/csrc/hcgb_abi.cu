@@ -146,6 +146,7 @@ struct BatchShape {
     int ld = 8, kmax = 8, rmax = 8;
     int p_m[3] = {0, 0, 0}, p_n[3] = {0, 0, 0};
     bool any_compressed_c = false;
+    bool direct = false;  // truncated SVDs of dense tiles (DevUpdate::direct)
 };
 
 BatchShape shape_of(const hcgb_update *ups, int n) {
@@ -240,6 +241,18 @@ void launch_pipeline(hcgb_context *ctx, cudaStream_t st, const DevUpdate *dups, 
     mark(HCGB_STAGE_PLAN);
     launch_plan(dups, n, alpha, beta, ws, p, djobs, st);
     cnt[HCGB_STAGE_PLAN]++;
+    if (sh.direct) {  // truncated SVDs of dense tiles: no stacks to form, factor or apply
+        mark(HCGB_STAGE_CORE_SVD);
+        if (ws.order) launch_order(n, ws, st);
+        launch_core_svd(dups, n, ws, p, st);
+        cnt[HCGB_STAGE_CORE_SVD]++;
+        mark(HCGB_STAGE_FINALIZE);
+        launch_finalize(dups, n, ws, info, st);
+        cnt[HCGB_STAGE_FINALIZE]++;
+        mark(-1);
+        if (ctx->prof) ctx->ev_pending.push_back(ev);
+        return;
+    }
     mark(HCGB_STAGE_STACK);
     if (sh.any_compressed_c) {
         launch_stack(dups, n, alpha, beta, ws, st);
@@ -323,11 +336,16 @@ void launch_pipeline(hcgb_context *ctx, cudaStream_t st, const DevUpdate *dups, 
     if (ctx->prof) ctx->ev_pending.push_back(ev);
 }
 
-int prepare_workspace(hcgb_context *ctx, const BatchShape &sh, int n, bool ddc, Workspace *out, int mode = 0) {
-    // The QR panels and the core's bookkeeping live in shared memory: refuse shapes beyond it.
+// The QR panels and the core's bookkeeping live in shared memory: refuse shapes beyond it.
+int check_shared_memory(hcgb_context *ctx, const BatchShape &sh) {
     const size_t smem_limit = 227 * 1024;
     if (sh.any_compressed_c && (qr_smem_bytes(sh.ld, sh.kmax) > smem_limit || svd_smem_bytes(sh.kmax) > smem_limit))
         return fail(ctx, HCGB_POOL_TOO_SMALL, "tile too large: the QR panel or core bookkeeping exceeds shared memory");
+    return HCGB_OK;
+}
+
+int prepare_workspace(hcgb_context *ctx, const BatchShape &sh, int n, bool ddc, Workspace *out, int mode = 0) {
+    if (int refused = check_shared_memory(ctx, sh)) return refused;
     const bool learned = ctx->learned, features = learned || ctx->feature_sink;
     Workspace w = make_workspace_layout(sh.ld, sh.kmax, sh.rmax, ddc, ctx->oz != 0 || lowp_prec(mode) != 0, learned);
     size_t need = workspace_bytes_for(w, n, features);
@@ -975,12 +993,49 @@ __global__ void identity_kernel(double *a, int n, int ld) {
 
 }  // namespace
 
+namespace {
+
+// Whether a compression runs the core on the dense tiles themselves.  The low-precision forms and the learned
+// form (and a feature sink) take the identity-operand update instead: their product precision, sketch
+// and records belong to it.
+bool compress_direct(const hcgb_context *ctx, const hcgb_params *params) {
+    return !ctx->learned && !ctx->feature_sink && !lowp_prec(params ? params->mode : 0);
+}
+
+// Truncated SVDs of n dense tiles (rows x cols) into out, chunk by chunk; statuses and ranks in dinfo.
+// With k = cols columns the stacks of an update D * I would be as large as the tile: their QR, the products and the
+// Q application only cost time.
+int direct_batch(hcgb_context *ctx, int n, const double *const *dense, int rows, int cols, hcgb_tile *out,
+                 const hcgb_params *params, const BatchShape &sh, hcgb_update_info *dinfo) {
+    const Params p = to_params(params, ctx);
+    Workspace ws;
+    int rc = prepare_workspace(ctx, sh, n, false, &ws, p.mode);
+    if (rc) return rc;
+    std::vector<DevUpdate> dv((size_t) n);
+    for (int i = 0; i < n; i++) {
+        dv[i].a = to_dev(hcgb_tile{const_cast<double *>(dense[i]), nullptr, rows, cols, 0, HCGB_DENSE});
+        dv[i].c = to_dev(out[i]);
+        dv[i].uid = i;
+        dv[i].direct = 1;
+    }
+    DevUpdate *dups;
+    GemmJob *djobs;
+    int *dsched;
+    if ((rc = upload_updates(ctx, dv, &dups, &djobs, &dsched))) return rc;
+    launch_pipeline(ctx, ctx->stream, dups, djobs, dsched, n, 1.0, 0.0, ws, sh, p, dinfo);
+    HCGB_CUDA(ctx, cudaGetLastError());
+    return HCGB_OK;
+}
+
+}  // namespace
+
 extern "C" int hcgb_compress_tile(hcgb_context *ctx, const double *dense, int rows, int cols, hcgb_tile *out,
                                   const hcgb_params *params, int *rank) {
     if (!ctx) return HCGB_BAD_ARG;
     if (!dense || !out || rows <= 0 || cols <= 0 || !compressed(out->kind) || out->rows != rows ||
         out->cols != cols || !out->rank || out->max_rank <= 0)
         return fail(ctx, HCGB_BAD_ARG, "hcgb_compress_tile: bad arguments");
+    if (compress_direct(ctx, params)) return hcgb_compress_tiles(ctx, 1, &dense, rows, cols, out, params, rank);
     HCGB_CUDA(ctx, cudaSetDevice(ctx->device));
     // D = D * I: an update with A = the dense tile, B = I (compressed, U = V = I_cols), C = 0 (rank 0)
     // recompresses exactly the columns of D, i.e. computes its truncated SVD.
@@ -1029,15 +1084,20 @@ extern "C" int hcgb_compress_tiles(hcgb_context *ctx, int count, const double *c
         if (dinfo) cudaFree(dinfo);
         return rc;
     };
-    if (cudaMalloc(&ibuf, sizeof(double) * 2 * n * n) != cudaSuccess || cudaMalloc(&irank, sizeof(int)) != cudaSuccess)
-        return done(fail(ctx, HCGB_CUDA_ERROR, "hcgb_compress_tiles: cudaMalloc failed"));
-    { identity_kernel<<<64, 256, 0, ctx->stream>>>(ibuf, cols, cols); note_launch(); }
-    { identity_kernel<<<64, 256, 0, ctx->stream>>>(ibuf + n * n, cols, cols); note_launch(); }
+    const bool direct = compress_direct(ctx, params);
+    if (!direct) {
+        if (cudaMalloc(&ibuf, sizeof(double) * 2 * n * n) != cudaSuccess ||
+            cudaMalloc(&irank, sizeof(int)) != cudaSuccess)
+            return done(fail(ctx, HCGB_CUDA_ERROR, "hcgb_compress_tiles: cudaMalloc failed"));
+        { identity_kernel<<<64, 256, 0, ctx->stream>>>(ibuf, cols, cols); note_launch(); }
+        { identity_kernel<<<64, 256, 0, ctx->stream>>>(ibuf + n * n, cols, cols); note_launch(); }
+    }
     const int ncols = cols;
     auto failed = [&](cudaError_t e) {  // a CUDA call failed: release what this call allocated
         return done(fail(ctx, HCGB_CUDA_ERROR, std::string("hcgb_compress_tiles: ") + cudaGetErrorString(e)));
     };
-    cudaError_t ce = cudaMemcpyAsync(irank, &ncols, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
+    cudaError_t ce = cudaSuccess;
+    if (!direct) ce = cudaMemcpyAsync(irank, &ncols, sizeof(int), cudaMemcpyHostToDevice, ctx->stream);
     if (ce != cudaSuccess) return failed(ce);
     const hcgb_tile ident{ibuf, irank, cols, cols, cols, HCGB_COMPRESSED};
     std::vector<hcgb_update> ups(count);
@@ -1047,14 +1107,24 @@ extern "C" int hcgb_compress_tiles(hcgb_context *ctx, int count, const double *c
                              out[i]};
     }
     const int mode = params ? params->mode : 0;
-    const int chunk = updates_per_launch(ctx, shape_of(ups.data(), 1), mode, count);
+    BatchShape sh = shape_of(ups.data(), 1);
+    if (direct) {
+        int rc = check_shared_memory(ctx, sh);  // the same tiles are accepted on either route
+        if (rc) return done(rc);
+        sh.kmax = std::max(rows, cols);
+        sh.ld = (sh.kmax + 7) / 8 * 8;
+        sh.rmax = 8;
+        sh.direct = true;
+    }
+    const int chunk = updates_per_launch(ctx, sh, mode, count);
     if (cudaMalloc(&dinfo, sizeof(hcgb_update_info) * (size_t) chunk) != cudaSuccess)
         return done(fail(ctx, HCGB_CUDA_ERROR, "hcgb_compress_tiles: cudaMalloc failed"));
     std::vector<hcgb_update_info> hinfo(chunk);
     bool not_converged = false;
     for (int off = 0; off < count; off += chunk) {
         const int nb = std::min(chunk, count - off);
-        int rc = hcgb_gemm_batch(ctx, 1.0, 0.0, nb, ups.data() + off, params, dinfo);
+        int rc = direct ? direct_batch(ctx, nb, dense + off, rows, cols, out + off, params, sh, dinfo)
+                        : hcgb_gemm_batch(ctx, 1.0, 0.0, nb, ups.data() + off, params, dinfo);
         if (rc) return done(rc);
         if ((ce = cudaMemcpyAsync(hinfo.data(), dinfo, sizeof(hcgb_update_info) * (size_t) nb,
                                   cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess ||

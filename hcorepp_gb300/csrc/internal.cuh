@@ -140,6 +140,7 @@ struct DevUpdate {
     DevTile a, b, c;
     int uid;   // index of this update's record in the caller's hcgb_update_info array
     int dist;  // |i - j| of the C tile in a tile-matrix multiply (a feature of the rank predictor)
+    int direct;  // 1: C = truncated SVD of the dense tile a (b unused, C at rank 0): the core alone
 };
 
 // Per-update bookkeeping written by the plan kernel and read by the later stages.

@@ -69,11 +69,11 @@ __device__ void plan_update(const DevUpdate *ups, int n, double alpha, double be
     const int rC = ck ? *u.c.rank : 0;
     const int m = u.c.rows, nn = u.c.cols, kd = u.a.cols;
     int status = HCGB_OK;
-    if (u.a.rows != m || u.b.cols != nn || u.b.rows != kd) status = HCGB_BAD_ARG;
+    if (u.a.rows != m || (u.direct ? kd != nn : u.b.cols != nn || u.b.rows != kd)) status = HCGB_BAD_ARG;
     if ((ak && (rA < 0 || rA > u.a.max_rank)) || (bk && (rB < 0 || rB > u.b.max_rank)) ||
         (ck && (rC < 0 || rC > u.c.max_rank)))
         status = HCGB_RANK_OVERFLOW;
-    if (!ak && !bk && ck) status = HCGB_UNSUPPORTED;  // DDC: hcgb_tile_gemm only
+    if (!ak && !bk && ck && !u.direct) status = HCGB_UNSUPPORTED;  // DDC: hcgb_tile_gemm only
     if (m > ws.ld || nn > ws.ld || rA > ws.rmax || rB > ws.rmax) status = HCGB_POOL_TOO_SMALL;
     meta[META_CKIND] = ck;
     meta[META_RA] = rA;
@@ -83,6 +83,12 @@ __device__ void plan_update(const DevUpdate *ups, int n, double alpha, double be
     meta[META_N] = nn;
     if (status != HCGB_OK) {
         meta[META_STATUS] = status;
+        return;
+    }
+    if (u.direct) {  // no stacks, no products: the core takes the tile as it is
+        const int k = m > nn ? m : nn;
+        meta[META_K] = k;
+        if (k > ws.kmax) meta[META_STATUS] = HCGB_POOL_TOO_SMALL;
         return;
     }
     double *slot = ws.slot(s);

@@ -1444,8 +1444,16 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
     const bool spread = CLUSTER && qrcp_cluster_doubles(kU, kV, TM::ctas) <= pool_doubles;
 
     const long long t0 = clock64();
-    // 1. M = R_U R_V^T on DMMA (R_U = triu of the U stack's top kU rows, likewise R_V).
-    {
+    // 1. M = R_U R_V^T on DMMA (R_U = triu of the U stack's top kU rows, likewise R_V), or the tile itself.
+    if (ups[slot].direct) {
+        const double *D = ups[slot].a.data;
+        for (int j = warp; j < kV; j += nw)
+            for (int i = lane; i < kU; i += 32) {
+                const double v = D[i + (size_t) j * m];
+                if (!spread) Mw[i + (size_t) j * ldw] = v;
+                Mc[i + (size_t) j * ldm] = v;
+            }
+    } else {
         const int ntr = (kU + 7) >> 3, ntc = (kV + 7) >> 3;
         for (int idx = warp; idx < ntr * ntc; idx += nw) {
             const int tr = idx % ntr, tc = idx / ntr;

@@ -1,5 +1,6 @@
 """The blocked tile kernels at the edges of their blocks: Cholesky factorisation (32-column blocks), the panel
-solve of the tile Cholesky (32 rows, 4 columns)."""
+solve of the tile Cholesky (32 rows, 4 columns), and compression of dense
+tiles by the core alone."""
 import ctypes as C
 
 import numpy as np
@@ -84,3 +85,16 @@ def test_cholesky_panel_solve_matches_the_tile_loop(T, nb, nt):
     np.testing.assert_array_equal(out[0][1], out[1][1])
     a = np.block([[km.tile(i, j) for j in range(nt)] for i in range(nt)])
     assert rel_fro(out[0][1] @ out[0][1].T, a) < 1e-7
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("m,n", [(1, 1), (5, 40), (40, 5), (100, 100), (131, 90), (90, 131), (300, 257)])
+def test_compression_of_rectangular_tiles(T, m, n, mode):
+    rng = np.random.default_rng([m, n])
+    r = min(m, n)
+    d = (np.linalg.qr(rng.standard_normal((m, r)))[0] * np.logspace(0, -12, r)) @ np.linalg.qr(
+        rng.standard_normal((n, r)))[0].T
+    g = T.CompressedTile.from_dense(d, T.CompressionParameters(1e-8, truncated_svd=True, mode=mode), max_rank=r)
+    o = O.CompressedTile.from_dense(d, O.CompressionParameters(1e-8, truncated_svd=True), max_rank=r)
+    assert abs(g.rank - o.rank) <= 1
+    assert rel_fro(g.to_dense(), d) <= 2 * max(rel_fro(o.to_dense(), d), 1e-14)
