@@ -683,6 +683,7 @@ int hcgb_tlr_gemm(hcgb_context *ctx, int mt, int nt, int kt, double alpha, const
         if (!single) HCGB_CUDA(ctx, cudaStreamWaitEvent(st, ctx->group_events[0], 0));
         Workspace &wg = wgs[g];
         wg = ws;
+        wg.conc = G;
         wg.base = ws.base + ws.slot_doubles * (size_t) first[g];
         wg.meta = ws.meta + (size_t) META_INTS * first[g];
         wg.order = ws.order + first[g];

@@ -71,6 +71,8 @@ struct ClusterTeam {
     }
 };
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ int cluster_rank() {
     int r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -179,6 +181,7 @@ struct Workspace {
     int ld;               // leading dimension of every stack / temporary (>= rows, cols)
     int kmax;             // max columns of a stack
     int rmax;             // max rank of an A/B factor
+    int conc = 1;         // launches like this one in flight at a time (the C-tile groups of a multiply)
     size_t off_ustack, off_vstack, off_tmp1, off_tmp2, off_tauu, off_tauv, off_tu, off_tv;
     size_t off_m, off_mcopy, off_xv, off_sigma, off_mixed;
     size_t off_w;  // WY application: W_U, W_V (kmax x kmax each), present when built with wy

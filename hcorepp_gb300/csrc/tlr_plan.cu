@@ -2,6 +2,8 @@
 // the plain form's full-WY Q application, ordering and write-back of a batch of TLR tile
 // updates.  Follows HCore<T>::Gemm's dispatch (src/api/HCore.cpp:23-344) and the
 // stacking of CompressedTile<T>::Gemm (src/operators/concrete/Compressed.cpp:331-379).
+#include <algorithm>
+
 #include "internal.cuh"
 
 namespace hcgb {
@@ -486,7 +488,7 @@ __global__ void plan_wy_kernel(const DevUpdate *ups, int n, Workspace ws, Params
     }
 }
 
-// Two CTAs per update (U side, V side): solve T^-1 W = Y in place, T^-1 = striu(G) + diag(1/tau),
+// blockIdx.x / 2, % 2: update and side (U, V); the columns of X are split over gridDim.y CTAs.  Solve T^-1 W = Y in place, T^-1 = striu(G) + diag(1/tau),
 // by blocked back substitution over row blocks of 32 (bottom up): the block's rows first take the
 // product of the already solved rows (every thread a few (row, column) dot products; G is
 // symmetric, so row i of its upper part is read as column i, contiguous), then the 32 x 32
@@ -505,13 +507,16 @@ __global__ void __launch_bounds__(256) wy_solve_kernel(Workspace ws) {
     double *base = ws.slot(slot);
     const double *G = base + (side ? ws.off_mcopy : ws.off_m);
     const double *tau = base + (side ? ws.off_tauv : ws.off_tauu);
-    double *W = base + ws.off_w + (size_t) side * ws.kmax * ws.kmax;
     const int lk = ws.kmax;
+    const int share = (r + gridDim.y - 1) / gridDim.y, c0 = blockIdx.y * share;
+    const int nc = r - c0 < share ? r - c0 : share;
+    if (nc <= 0) return;
+    double *W = base + ws.off_w + (size_t) side * lk * lk + (size_t) c0 * lk;
     for (int bs = ((kk - 1) / BS) * BS; bs >= 0; bs -= BS) {
         const int be = bs + BS < kk ? bs + BS : kk, nbk = be - bs;
         // 1. rows bs..be-1 of W -= G[bs:be, be:kk] W[be:kk, :]
         if (be < kk) {
-            for (int e = threadIdx.x; e < nbk * r; e += blockDim.x) {
+            for (int e = threadIdx.x; e < nbk * nc; e += blockDim.x) {
                 const int i = bs + e % nbk, c = e / nbk;
                 const double *gi = G + (size_t) i * lk;
                 const double *wc = W + (size_t) c * lk;
@@ -532,7 +537,7 @@ __global__ void __launch_bounds__(256) wy_solve_kernel(Workspace ws) {
         }
         if (threadIdx.x < nbk) tb[threadIdx.x] = tau[bs + threadIdx.x];
         __syncthreads();
-        for (int c = threadIdx.x; c < r; c += blockDim.x) {
+        for (int c = threadIdx.x; c < nc; c += blockDim.x) {
             double *wc = W + (size_t) c * lk + bs;
             double x[BS];
 #pragma unroll
@@ -557,12 +562,25 @@ __global__ void __launch_bounds__(256) wy_solve_kernel(Workspace ws) {
 
 }  // namespace
 
+static int device_sms() {
+    static int sms[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return 152;
+    if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
+    return sms[dev] > 0 ? sms[dev] : 152;
+}
+
 void launch_plan_wy(const DevUpdate *ups, int n, Workspace ws, Params p, GemmJob *jobs, cudaStream_t st) {
     { plan_wy_kernel<<<(n + 127) / 128, 128, 0, st>>>(ups, n, ws, p, jobs); note_launch(); }
 }
 
 void launch_wy_solve(int n, Workspace ws, cudaStream_t st) {
-    { wy_solve_kernel<<<2 * n, 256, 0, st>>>(ws); note_launch(); }
+    // As many CTAs a side as leave no SM idle (up to one per eight columns): a side's solve on one SM took 3 ms at
+    // 340 reflectors and 170 columns.
+    const int sms = device_sms(), cols = (ws.kmax + 7) / 8;
+    const int split = std::max(1, std::min(cols, 2 * sms / (2 * n * ws.conc)));
+    { wy_solve_kernel<<<dim3(2 * n, split), 256, 0, st>>>(ws); note_launch(); }
 }
 
 void launch_transpose(const double *src, int lds, int rows, int cols, double *dst, int ldd, cudaStream_t st) {
@@ -589,15 +607,6 @@ void launch_order(int n, Workspace ws, cudaStream_t st) {
 
 void launch_stack(const DevUpdate *ups, int n, double alpha, double beta, Workspace ws, cudaStream_t st) {
     { stack_kernel<<<n, 256, 0, st>>>(ups, alpha, beta, ws); note_launch(); }
-}
-
-static int device_sms() {
-    static int sms[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return 152;
-    if (!sms[dev]) cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    return sms[dev] > 0 ? sms[dev] : 152;
 }
 
 void launch_gemm_jobs(const GemmJob *jobs, int njobs, int *sched, cudaStream_t st, bool has_lowp) {

@@ -21,6 +21,7 @@ namespace {
 constexpr int NB = QR_NB;
 constexpr int QR_THREADS = 256;
 constexpr int QRD_THREADS = 512;  // mixed-form kernels: one heavy side, or both sides of a light update
+constexpr int QR_SMS = 152;       // CTAs that the clusters of the launches in flight may take
 constexpr int QR_HEAVY_K = 95;    // sides of updates with a wider stack get a whole CTA
 
 __host__ __device__ __forceinline__ int round_up(int x, int m) { return (x + m - 1) / m * m; }
@@ -34,45 +35,74 @@ __host__ __device__ __forceinline__ int qr_w_cols(int kmax) {
 // Householder QR of the panel in shared memory: column c at Ps + c*ldp, rows 0..mr-1.
 // LAPACK dlarfg convention: beta = -sign(alpha) * ||x||, tau = (beta - alpha) / beta,
 // v = x / (alpha - beta) with v_0 = 1 implicit; tau = 0 when the tail is zero.
-__device__ void factor_panel(double *Ps, int ldp, int mr, int nbp, double *tau_s, double *red) {
+// One barrier a column: the warp that updates the next column also takes its norm and forms its reflector.
+// The columns are scaled by 1 / (alpha - beta) at the end, the products carry the factor until then.
+// Returns whether any reflector differs from the identity.  red: >= NB doubles.
+__device__ bool factor_panel(double *Ps, int ldp, int mr, int nbp, double *tau_s, double *red) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int j = 0; j < nbp; j++) {
-        double *x = Ps + (size_t) j * ldp;
-        // the reflector's norm on the first warp alone: a block-wide sum would issue eight warps'
-        // reductions on the FP64 pipe and cost two more barriers
+    // reflector of column c from its entry alpha on the diagonal and its tail's squared norm (one warp);
+    // tau = 1 + |alpha| / ||x||: one reciprocal square root and one reciprocal, no division
+    auto form = [&](int c, double alpha, double ss) {
+        double tau = 0.0, scale = 0.0, beta = alpha;
+        if (ss != 0.0) {
+            const double q = fma(alpha, alpha, ss), r = rsqrt(q), nrm = q * r;
+            beta = -copysign(nrm, alpha);
+            tau = fma(fabs(alpha), r, 1.0);
+            scale = copysign(__drcp_rn(nrm + fabs(alpha)), alpha);
+        }
+        if (lane == 0) {
+            tau_s[c] = tau;
+            red[c] = scale;
+            Ps[c + (size_t) c * ldp] = beta;
+        }
+    };
+    if (warp == 0 && nbp > 0) {
         double ss = 0.0;
-        if (warp == 0) {
-            for (int r = j + 1 + lane; r < mr; r += 32) ss = fma(x[r], x[r], ss);
-            ss = warp_sum(ss);
-        }
-        if (threadIdx.x == 0) {
-            const double alpha = x[j];
-            double tau = 0.0, scale = 0.0, beta = alpha;
-            if (ss != 0.0) {
-                beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
-                tau = (beta - alpha) / beta;
-                scale = 1.0 / (alpha - beta);
-            }
-            tau_s[j] = tau;
-            red[40] = scale;
-            x[j] = beta;
-        }
-        __syncthreads();
-        const double scale = red[40], tau = tau_s[j];
-        for (int r = j + 1 + threadIdx.x; r < mr; r += blockDim.x) x[r] *= scale;
-        __syncthreads();
-        if (tau != 0.0) {
-            for (int c = j + 1 + warp; c < nbp; c += nw) {
-                double *y = Ps + (size_t) c * ldp;
-                double w = lane == 0 ? y[j] : 0.0;
+        for (int r = 1 + lane; r < mr; r += 32) ss = fma(Ps[r], Ps[r], ss);
+        ss = warp_sum(ss);
+        const double alpha = Ps[0];
+        __syncwarp();
+        form(0, alpha, ss);
+    }
+    __syncthreads();
+    for (int j = 0; j + 1 < nbp; j++) {
+        const double *x = Ps + (size_t) j * ldp;
+        const double scale = red[j], tau = tau_s[j];
+        for (int c = j + 1 + warp; c < nbp; c += nw) {
+            double *y = Ps + (size_t) c * ldp;
+            double ss = 0.0, alpha = y[c];
+            if (tau != 0.0) {
+                double w = 0.0;
                 for (int r = j + 1 + lane; r < mr; r += 32) w = fma(x[r], y[r], w);
-                w = warp_sum(w) * tau;
+                w = fma(warp_sum(w), scale, y[j]) * tau;
+                const double ws = w * scale;
+                alpha = fma(-ws, x[c], alpha);
+                __syncwarp();
                 if (lane == 0) y[j] -= w;
-                for (int r = j + 1 + lane; r < mr; r += 32) y[r] = fma(-w, x[r], y[r]);
+                for (int r = j + 1 + lane; r < mr; r += 32) {
+                    const double v = fma(-ws, x[r], y[r]);
+                    y[r] = v;
+                    if (c == j + 1 && r > c) ss = fma(v, v, ss);
+                }
+            } else if (c == j + 1) {
+                for (int r = c + 1 + lane; r < mr; r += 32) ss = fma(y[r], y[r], ss);
+            }
+            if (c == j + 1) {
+                ss = warp_sum(ss);
+                __syncwarp();
+                form(c, alpha, ss);
             }
         }
         __syncthreads();
     }
+    bool any = false;
+    for (int c = 0; c < nbp; c++) {
+        any |= tau_s[c] != 0.0;
+        const double scale = red[c];
+        for (int r = c + 1 + threadIdx.x; r < mr; r += blockDim.x) Ps[r + (size_t) c * ldp] *= scale;
+    }
+    __syncthreads();
+    return any;
 }
 
 // Float-float version of factor_panel (mixed form), in place on the panel held as float-float
@@ -278,10 +308,14 @@ __device__ QrShared carve(double *sm, int ld, int kmax) {
     return s;
 }
 
-// grid = 2 * n: block 2s factors the U stack of update s, block 2s+1 its V stack.
+// Side blockIdx.x / C of the launch (2s: the U stack of update s, 2s + 1: its V stack), by a cluster of C CTAs:
+// each factors every panel for itself (no broadcast of V and T) and updates its share of the trailing columns;
+// the first CTA writes the panel back.  A column's arithmetic does not depend on C.
+template <int C>
 __global__ void __launch_bounds__(QR_THREADS) qr_kernel(Workspace ws) {
     extern __shared__ double sm[];
-    const int slot = ws.heavy(blockIdx.x >> 1), side = blockIdx.x & 1;
+    const int part = C > 1 ? cluster_rank() : 0;
+    const int id = blockIdx.x / C, slot = ws.heavy(id >> 1), side = id & 1;
     const int *meta = ws.meta + (size_t) slot * META_INTS;
     if (meta[META_STATUS] != HCGB_OK || !meta[META_CKIND]) return;
     const int k = meta[META_K];
@@ -301,19 +335,37 @@ __global__ void __launch_bounds__(QR_THREADS) qr_kernel(Workspace ws) {
             s.Ps[e] = (c < nbp && r < mr) ? A[(j0 + r) + (size_t) (j0 + c) * lda] : 0.0;
         }
         __syncthreads();
-        factor_panel(s.Ps, s.ldp, mr, nbp, s.tau, s.red);
-        for (int e = threadIdx.x; e < nbp * mr; e += blockDim.x) {
-            const int c = e / mr, r = e % mr;
-            A[(j0 + r) + (size_t) (j0 + c) * lda] = s.Ps[(size_t) c * s.ldp + r];
+        if (C > 1) cluster_arrive();  // this CTA has read the panel
+        const bool any = factor_panel(s.Ps, s.ldp, mr, nbp, s.tau, s.red);
+        if (C > 1) cluster_wait();    // so has every other: it may be written
+        if (part == 0) {
+            for (int e = threadIdx.x; e < nbp * mr; e += blockDim.x) {
+                const int c = e / mr, r = e % mr;
+                A[(j0 + r) + (size_t) (j0 + c) * lda] = s.Ps[(size_t) c * s.ldp + r];
+            }
+            if (threadIdx.x < nbp) tau[j0 + threadIdx.x] = s.tau[threadIdx.x];
         }
-        if (threadIdx.x < nbp) tau[j0 + threadIdx.x] = s.tau[threadIdx.x];
         __syncthreads();
-        make_explicit_v(s.Ps, s.ldp, nbp);
+        if (any) {
+            make_explicit_v(s.Ps, s.ldp, nbp);
+            __syncthreads();
+            build_t(s.Ps, s.ldp, mr, nbp, s.tau, s.Ts, s.Gs);
+        }
+        if (part == 0)
+            for (int e = threadIdx.x; e < NB * NB; e += blockDim.x)
+                Tg[(size_t) (j0 / NB) * NB * NB + e] = any ? s.Ts[e] : 0.0;
+        if (any) {  // else the panel's reflectors are the identity
+            const int nt = k - j0 - nbp, share = round_up((nt + C - 1) / C, 8), first = part * share;
+            const int cols = nt - first < share ? nt - first : share;
+            const int c0 = j0 + nbp + first;
+            if (cols > 0)
+                apply_block_reflector(s.Ps, s.ldp, s.Ts, true, A + j0 + (size_t) c0 * lda, lda, mr, cols, s.Ws, s.ldw);
+        }
+        if (C > 1) {
+            cluster_arrive();
+            cluster_wait();
+        }
         __syncthreads();
-        build_t(s.Ps, s.ldp, mr, nbp, s.tau, s.Ts, s.Gs);
-        for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) Tg[(size_t) (j0 / NB) * NB * NB + e] = s.Ts[e];
-        const int c0 = j0 + nbp;
-        apply_block_reflector(s.Ps, s.ldp, s.Ts, true, A + j0 + (size_t) c0 * lda, lda, mr, k - c0, s.Ws, s.ldw);
     }
 }
 
@@ -703,6 +755,24 @@ static bool qr_pair_fits(size_t team_bytes) {
     return 2 * team_bytes + 256 <= (size_t) optin;
 }
 
+template <int C>
+static void launch_qr_clusters(Workspace ws, int n, size_t smem, cudaStream_t st) {
+    cudaFuncSetAttribute(qr_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * n * C);
+    cfg.blockDim = dim3(QR_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, qr_kernel<C>, ws);
+    note_launch();
+}
+
 void launch_qr(Workspace ws, int n, bool mixed, cudaStream_t st) {
     const size_t smem = qr_smem_bytes(ws.ld, ws.kmax);
     if (mixed) {
@@ -711,8 +781,13 @@ void launch_qr(Workspace ws, int n, bool mixed, cudaStream_t st) {
         cudaFuncSetAttribute(qr_kernel_df, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) cta);
         { qr_kernel_df<<<2 * n, QRD_THREADS, cta, st>>>(ws, n, (int) (smem / sizeof(double)), pair); note_launch(); }
     } else {
-        cudaFuncSetAttribute(qr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-        { qr_kernel<<<2 * n, QR_THREADS, smem, st>>>(ws); note_launch(); }
+        // A cluster per side while the launches in flight leave SMs idle: at k = 340, m = 512 one CTA took
+        // 15.7 ms (its SM's FP64 pipe).
+        const long sides = 2L * n * ws.conc;
+        if (sides * 8 <= QR_SMS) launch_qr_clusters<8>(ws, n, smem, st);
+        else if (sides * 4 <= QR_SMS) launch_qr_clusters<4>(ws, n, smem, st);
+        else if (sides * 2 <= QR_SMS) launch_qr_clusters<2>(ws, n, smem, st);
+        else launch_qr_clusters<1>(ws, n, smem, st);
     }
 }
 

@@ -1,6 +1,6 @@
 """The blocked tile kernels at the edges of their blocks: Cholesky factorisation (32-column blocks), the panel
-solve of the tile Cholesky (32 rows, 4 columns), and compression of dense
-tiles by the core alone."""
+solve of the tile Cholesky (32 rows, 4 columns), the stack QR's clusters (their size follows the load), and
+compression of dense tiles by the core alone."""
 import ctypes as C
 
 import numpy as np
@@ -85,6 +85,33 @@ def test_cholesky_panel_solve_matches_the_tile_loop(T, nb, nt):
     np.testing.assert_array_equal(out[0][1], out[1][1])
     a = np.block([[km.tile(i, j) for j in range(nt)] for i in range(nt)])
     assert rel_fro(out[0][1] @ out[0][1].T, a) < 1e-7
+
+
+@pytest.mark.parametrize("rc,ra", [(9, 8), (60, 45), (100, 90)])
+def test_results_do_not_depend_on_the_number_of_updates(T, rc, ra):
+    """One update, and the same one among 3, 12, 30 and 50: the QR's clusters have 8, 8, 4, 2 and 1 CTAs."""
+    import torch
+    from hcorepp_gb300 import _lib as L
+    rng = np.random.default_rng([rc, ra])
+    n, cap = 203, rc + ra
+    q = lambda r: np.linalg.qr(rng.standard_normal((n, r)))[0]
+    cu, cv = q(rc), np.logspace(0, -8, rc)[:, None] * q(rc).T
+    au, av, bu, bv = q(ra), np.logspace(0, -8, ra)[:, None] * q(ra).T, q(ra), q(ra).T
+    params = T.CompressionParameters(1e-8, truncated_svd=True)
+    p, first = params.c(), None
+    for count in (1, 3, 12, 30, 50):
+        a, b = T.CompressedTile(n, n, au, av, max_rank=cap), T.CompressedTile(n, n, bu, bv, max_rank=cap)
+        cs = [T.CompressedTile(n, n, cu, cv, max_rank=cap) for _ in range(count)]
+        ups = (L.Update * count)(*[L.Update(a.c_tile(), b.c_tile(), c.c_tile()) for c in cs])
+        ctx = T.run_context()
+        ctx.check(L.lib().hcgb_gemm_batch(ctx.handle, 1.0, 1.0, count, ups, C.byref(p), None))
+        torch.cuda.synchronize()
+        got = [(c.rank, c.u(), c.v()) for c in cs]
+        first = first or got[0]
+        for r, u, v in got:
+            assert r == first[0]
+            np.testing.assert_array_equal(u, first[1])
+            np.testing.assert_array_equal(v, first[2])
 
 
 @pytest.mark.parametrize("mode", [0, 1])
