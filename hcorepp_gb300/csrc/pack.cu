@@ -22,6 +22,8 @@ __device__ __forceinline__ long long packed_doubles(const DevTile &t) {
     return r * (t.rows + t.cols);
 }
 
+constexpr int PACK_CTAS = 3648;
+
 // offsets[0..n] = exclusive prefix sum of the packed sizes; one CTA: every thread sums a
 // contiguous run of tiles, a Hillis-Steele scan combines the runs.
 __global__ void __launch_bounds__(1024) pack_offsets_kernel(const DevTile *tiles, int n, long long *offsets) {
@@ -47,31 +49,44 @@ __global__ void __launch_bounds__(1024) pack_offsets_kernel(const DevTile *tiles
     if (threadIdx.x == blockDim.x - 1) offsets[n] = part[blockDim.x - 1];
 }
 
-__device__ __forceinline__ void copy_run(const double *src, double *dst, long long len) {
-    for (long long e = threadIdx.x; e < len; e += blockDim.x) dst[e] = src[e];
+// The part-th of `parts` shares of a copy, eight values a thread in flight.
+__device__ __forceinline__ void copy_run(const double *__restrict__ src, double *__restrict__ dst, long long len,
+                                         int part, int parts) {
+    constexpr int U = 8;
+    const long long step = (long long) blockDim.x * U, share = (len + parts - 1) / parts;
+    const long long end = share * (part + 1) < len ? share * (part + 1) : len;
+    for (long long e0 = share * part; e0 < end; e0 += step) {
+        double v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long e = e0 + threadIdx.x + (long long) u * blockDim.x;
+            if (e < end) v[u] = src[e];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long e = e0 + threadIdx.x + (long long) u * blockDim.x;
+            if (e < end) dst[e] = v[u];
+        }
+    }
 }
 
-// One CTA per tile: unpack = 0 copies the tile's used part into the packed buffer, 1 back.
+// gridDim.y CTAs per tile, a share of its values each: unpack = 0 copies the tile's used part into the packed
+// buffer, 1 back.  Bound by memory; with one CTA a tile the 2 MB of a dense 512 x 512 tile set the time
+// (a 16 x 16-tile matrix out and back in: 950 us).
 __global__ void __launch_bounds__(256) pack_kernel(const DevTile *tiles, int n, const long long *offsets,
                                                    double *packed, int unpack) {
     const int t = blockIdx.x;
     if (t >= n) return;
     const DevTile d = tiles[t];
     double *p = packed + offsets[t];
-    if (!d.kind) {
-        const long long len = (long long) d.rows * d.cols;
-        if (unpack) copy_run(p, d.data, len);
-        else copy_run(d.data, p, len);
-        return;
-    }
-    const long long r = *d.rank;
-    const long long lu = r * d.rows, lv = r * d.cols;
+    const long long r = d.kind ? *d.rank : 0;
+    const long long lu = d.kind ? r * d.rows : (long long) d.rows * d.cols, lv = r * d.cols;
     if (unpack) {
-        copy_run(p, d.data, lu);
-        copy_run(p + lu, d.v, lv);
+        copy_run(p, d.data, lu, blockIdx.y, gridDim.y);
+        if (lv > 0) copy_run(p + lu, d.v, lv, blockIdx.y, gridDim.y);
     } else {
-        copy_run(d.data, p, lu);
-        copy_run(d.v, p + lu, lv);
+        copy_run(d.data, p, lu, blockIdx.y, gridDim.y);
+        if (lv > 0) copy_run(d.v, p + lu, lv, blockIdx.y, gridDim.y);
     }
 }
 
@@ -79,7 +94,9 @@ __global__ void __launch_bounds__(256) pack_kernel(const DevTile *tiles, int n, 
 
 void launch_pack(const DevTile *tiles, int n, long long *offsets, double *packed, bool unpack, cudaStream_t st) {
     { pack_offsets_kernel<<<1, 1024, 0, st>>>(tiles, n, offsets); note_launch(); }
-    { pack_kernel<<<n, 256, 0, st>>>(tiles, n, offsets, packed, unpack ? 1 : 0); note_launch(); }
+    // enough CTAs for the whole GPU whatever the number of tiles (PACK_CTAS: 152 SMs x 8 CTAs, three times over)
+    const int split = PACK_CTAS / n < 1 ? 1 : (PACK_CTAS / n < 128 ? PACK_CTAS / n : 128);
+    { pack_kernel<<<dim3(n, split), 256, 0, st>>>(tiles, n, offsets, packed, unpack ? 1 : 0); note_launch(); }
 }
 
 }  // namespace hcgb
