@@ -20,10 +20,20 @@
 //     C_ij = 2^(e_i + f_j) (hi 2^-35 + lo 2^-63).
 // Tensor memory holds the eight level accumulators of a 128 x 64 output tile (512 columns); one
 // thread issues the 72 MMAs (36 pairs x 2 k-steps of 16) of a 32-wide K chunk while the others cut
-// the next chunk into digit planes in the second shared-memory stage.  The splitting and combining
-// is integer work; an output element costs 4 FP64 instructions (two conversions, two scalings)
-// plus the epilogue.
+// the next chunk into digit planes in the second shared-memory stage.
+//
+// What bounds it is the splitting, not the tensor cores: every operand element becomes eight FP16 digits.  A
+// bias of 64 in every digit makes the balanced digits independent bit fields (no carry from digit to digit),
+// two of them at a time become halves by one exact subtraction (1024 + d as a bit pattern), a thread takes
+// eight consecutive K of a row, so a plane costs one 16-byte store without bank conflicts, and rows beyond
+// the job are left alone (they only reach accumulators nobody reads).  Sixteen warps, four to a
+// sub-partition, hide the latencies; sums and outputs are put together by integer operations, one FP64
+// instruction an output for beta C.  Sixteen warps instead of eight and this
+// splitting took the products of a 32 x 32-tile multiply (nb = 512) from 108 to 86 ms and its Q application
+// from 214 to 184.
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "internal.cuh"
 #include "tcgen05.cuh"
@@ -40,7 +50,7 @@ constexpr int OZ_TM = 128, OZ_TN = 64;  // output tile per CTA (UMMA M = 128, N 
 constexpr int OZ_KC = 32;               // K elements per shared-memory stage (64 bytes per row and plane)
 constexpr int OZ_KB = OZ_KC * 2 / 16;   // core matrices along K per stage (4)
 constexpr int OZ_FLUSH = 4;             // stages per exact read-out of the level accumulators (128 k)
-constexpr int OZ_THREADS = 256;         // 8 warps
+constexpr int OZ_THREADS = 512;         // 16 warps
 constexpr int OZ_A_PLANE = OZ_TM * OZ_KC * 2;   // 8 KB
 constexpr int OZ_B_PLANE = OZ_TN * OZ_KC * 2;   // 4 KB
 constexpr int OZ_STAGE = OZ_S * (OZ_A_PLANE + OZ_B_PLANE);  // 96 KB
@@ -55,9 +65,13 @@ __device__ __forceinline__ int exp_field(double x) {
     return (int) ((__double_as_longlong(x) >> 52) & 0x7ff);
 }
 
-// Balanced digits of x relative to the group exponent e (|x| < 2^e): digit s has weight
-// 2^(e - 7 (s + 1)), d[1..7] in [-64, 63], d[0] in [-128, 128].  Subnormals count as zero.
-__device__ __forceinline__ void oz_digits(double x, int e, int (&d)[OZ_S]) {
+// The 56-bit fixed-point integer of x relative to the group exponent e (|x| < 2^e), v = round(x 2^(56 - e)), plus
+// 64 in each digit but the leading one and 128 in that: digit s is the 7-bit field at 7 (7 - s) minus 64, the
+// leading digit what lies above bit 49 minus 128: d[1..7] in [-64, 63], d[0] in [-128, 128].  Subnormals
+// count as zero.
+constexpr unsigned long long OZ_BIAS = (128ull << 49) | (64ull << 42) | (64ull << 35) | (64ull << 28) | (64ull << 21) |
+                                       (64ull << 14) | (64ull << 7) | 64ull;
+__device__ __forceinline__ unsigned long long oz_biased(double x, int e) {
     const long long bits = __double_as_longlong(x);
     const int E = (int) ((bits >> 52) & 0x7ff);
     long long u = 0;
@@ -67,15 +81,19 @@ __device__ __forceinline__ void oz_digits(double x, int e, int (&d)[OZ_S]) {
         if (sh >= 0) u = M << sh;
         else if (sh > -64) u = (M + (1LL << (-sh - 1))) >> (-sh);
     }
-    long long v = bits < 0 ? -u : u;
-#pragma unroll
-    for (int s = OZ_S - 1; s > 0; s--) {
-        long long r = v & 127;
-        if (r >= 64) r -= 128;
-        d[s] = (int) r;
-        v = (v - r) >> OZ_B;
-    }
-    d[0] = (int) v;
+    return (unsigned long long) (bits < 0 ? -u : u) + OZ_BIAS;
+}
+
+// Digits `s` of two biased integers as a pair of halves.
+template <int S>
+__device__ __forceinline__ uint32_t oz_digit_pair(unsigned long long u0, unsigned long long u1) {
+    constexpr int SHIFT = OZ_B * (OZ_S - 1 - S);
+    constexpr uint32_t MASK = S ? 127u : 511u;
+    const uint32_t x0 = (uint32_t) (u0 >> SHIFT) & MASK, x1 = (uint32_t) (u1 >> SHIFT) & MASK;
+    const uint32_t m = x0 | (x1 << 16) | 0x64006400u;  // 1024 + x as FP16
+    const uint32_t off = S ? 0x64406440u : 0x64806480u;  // 1024 + 64, 1024 + 128
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&m), *reinterpret_cast<const __half2 *>(&off));
+    return *reinterpret_cast<const uint32_t *>(&d);
 }
 
 // Byte offset of (row r, K element kk of the stage) inside one plane (core-matrix layout, 2-byte
@@ -84,55 +102,90 @@ __device__ __forceinline__ int oz_off(int r, int kk) {
     return ((r >> 3) * OZ_KB + (kk >> 3)) * 128 + (r & 7) * 16 + (kk & 7) * 2;
 }
 
-__device__ __forceinline__ uint32_t pack_h2(int lo, int hi) {
-    const __half a = __int2half_rn(lo), b = __int2half_rn(hi);
-    return (uint32_t) __half_as_ushort(a) | ((uint32_t) __half_as_ushort(b) << 16);
-}
-
-// 2^ex as a double (0 below the normal range).
-__device__ __forceinline__ double pow2(int ex) {
-    if (ex < -1022) return 0.0;
-    if (ex > 1023) ex = 1023;
-    return __hiloint2double((ex + 1023) << 20, 0);
-}
-
-// Cuts rows [0, R) x K elements [k0, k0 + 32) of op(X) (a = true: op(A) with the row exponents;
-// false: op(B)^T with the column exponents) into the stage's digit planes, two K elements per
-// 32-bit store.
-template <bool IS_A>
-__device__ void split_chunk(const GemmJob &jb, int base, int R, int k0, const int *ex, unsigned char *planes,
-                            int plane_bytes) {
-    constexpr int PAIRS = OZ_KC / 2;
-    const bool kfast = IS_A ? jb.opA != 0 : jb.opB == 0;  // consecutive K contiguous in memory
-    const int lim = IS_A ? jb.M : jb.N;
-    for (int e = threadIdx.x; e < R * PAIRS; e += OZ_THREADS) {
-        int r, kp;
-        if (kfast) {
-            kp = e % PAIRS;
-            r = e / PAIRS;
-        } else {
-            r = e % R;
-            kp = e / R;
+// (hi 2^28 + lo) 2^(e - 63) as a double, rounded once (to nearest even), by integer operations.
+__device__ __forceinline__ double oz_value(long long hi, long long lo, int e) {
+    long long t = hi + (lo >> 28);
+    uint32_t r = (uint32_t) lo & 0xfffffffu;  // the number is t 2^28 + r
+    const bool neg = t < 0;
+    if (neg) {
+        t = -t;
+        if (r) {
+            t -= 1;
+            r = 0x10000000u - r;
         }
-        const int g = base + r, k = k0 + 2 * kp;
-        double v0 = 0.0, v1 = 0.0;
-        if (g < lim) {
-            if (IS_A) {
-                if (k < jb.K) v0 = job_a(jb, g, k);
-                if (k + 1 < jb.K) v1 = job_a(jb, g, k + 1);
-            } else {
-                if (k < jb.K) v0 = job_b(jb, k, g);
-                if (k + 1 < jb.K) v1 = job_b(jb, k + 1, g);
-            }
-        }
-        int d0[OZ_S], d1[OZ_S];
-        oz_digits(v0, ex[r], d0);
-        oz_digits(v1, ex[r], d1);
-        const int off = oz_off(r, 2 * kp);
-#pragma unroll
-        for (int s = 0; s < OZ_S; s++)
-            *reinterpret_cast<uint32_t *>(planes + s * plane_bytes + off) = pack_h2(d0[s], d1[s]);
     }
+    const unsigned long long u = (unsigned long long) t;
+    unsigned long long x;
+    int ex;
+    bool sticky = false;
+    if (u) {
+        const int n = __clzll(u);
+        x = u << n;
+        if (n >= 28) {
+            x |= (unsigned long long) r << (n - 28);
+        } else {
+            x |= r >> (28 - n);
+            sticky = (r & ((1u << (28 - n)) - 1u)) != 0;
+        }
+        ex = 28 - n;
+    } else if (r) {
+        const int n = __clzll((unsigned long long) r);
+        x = (unsigned long long) r << n;
+        ex = -n;
+    } else {
+        return 0.0;
+    }
+    ex += e - 63;  // x 2^ex, the leading bit of x set
+    const uint32_t rest = (uint32_t) x & 0x7ffu;
+    unsigned long long m = x >> 11;
+    if (rest > 0x400u || (rest == 0x400u && (sticky || (m & 1)))) m++;
+    const int field = ex + 63 + 1023;
+    double v;
+    if (field > 0 && field < 2046) v = __longlong_as_double((long long) (((unsigned long long) (field - 1) << 52) + m));
+    else v = ldexp((double) m, ex + 11);
+    return neg ? -v : v;
+}
+
+// Elements k0 .. k0 + NK - 1 of row g of op(A) (IS_A) or of column g of op(B), zero beyond K.
+template <bool IS_A, int NK>
+__device__ __forceinline__ void load_run(const GemmJob &jb, int g, int k0, double (&v)[NK]) {
+    const int op = IS_A ? jb.opA : jb.opB, ld = IS_A ? jb.lda : jb.ldb, tri = IS_A ? jb.triA : jb.triB;
+    const bool kcol = IS_A ? op == 0 : op != 0;  // k is the stored column index
+    const double *p = (IS_A ? jb.A : jb.B) + (kcol ? (size_t) g + (size_t) k0 * ld : (size_t) k0 + (size_t) g * ld);
+    const size_t step = kcol ? (size_t) ld : 1;
+#pragma unroll
+    for (int q = 0; q < NK; q++) {
+        v[q] = k0 + q < jb.K ? p[step * q] : 0.0;
+        if (tri) {
+            const int r = kcol ? g : k0 + q, c = kcol ? k0 + q : g;
+            if (r <= c && k0 + q < jb.K) v[q] = r == c ? 1.0 : 0.0;
+        }
+    }
+}
+
+// NK (4 or 8) consecutive K elements of row r of the tile (row g of the operand) into the eight digit planes.
+template <int NK>
+__device__ __forceinline__ void split_run(const double (&v)[NK], int e, unsigned char *at, int plane_bytes) {
+    unsigned long long u[NK];
+#pragma unroll
+    for (int q = 0; q < NK; q++) u[q] = oz_biased(v[q], e);
+    auto plane = [&](auto tag) {
+        constexpr int S = decltype(tag)::value;
+        uint32_t w[NK / 2];
+#pragma unroll
+        for (int q = 0; q < NK / 2; q++) w[q] = oz_digit_pair<S>(u[2 * q], u[2 * q + 1]);
+        unsigned char *d = at + S * plane_bytes;
+        if constexpr (NK == 8) *reinterpret_cast<uint4 *>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+        else *reinterpret_cast<uint2 *>(d) = make_uint2(w[0], w[1]);
+    };
+    plane(std::integral_constant<int, 0>{});
+    plane(std::integral_constant<int, 1>{});
+    plane(std::integral_constant<int, 2>{});
+    plane(std::integral_constant<int, 3>{});
+    plane(std::integral_constant<int, 4>{});
+    plane(std::integral_constant<int, 5>{});
+    plane(std::integral_constant<int, 6>{});
+    plane(std::integral_constant<int, 7>{});
 }
 
 // One 128 x 64 output tile of one job.
@@ -141,33 +194,43 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     const int ntm = (jb.M + OZ_TM - 1) / OZ_TM;
     const int m0 = (tile % ntm) * OZ_TM, n0 = (tile / ntm) * OZ_TN;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr uint32_t IDESC = tc::instr_desc(tc::FMT_F16, OZ_TM, OZ_TN);
+    const int rows = jb.M - m0 < OZ_TM ? jb.M - m0 : OZ_TM, cols = jb.N - n0 < OZ_TN ? jb.N - n0 : OZ_TN;
+    const uint32_t idesc = tc::instr_desc(tc::FMT_F16, OZ_TM, (cols + 15) & ~15);
 
-    // 1. Group exponents over all of K: PA threads per row of op(A), PB per column of op(B).
-    {
-        constexpr int PA = OZ_THREADS / OZ_TM, PB = OZ_THREADS / OZ_TN;
-        const int gi = m0 + tid / PA, pa = tid % PA;
-        int ma = 0;
-        if (gi < jb.M)
-            for (int k = pa; k < jb.K; k += PA) ma = max(ma, exp_field(job_a(jb, gi, k)));
+    // 1. Group exponents over all of K, largest exponent field per row of op(A) and column of op(B); the
+    //    threads of a group are laid out so that consecutive lanes read consecutive addresses.
+    if (tid < OZ_TM) ea[tid] = 0;
+    else if (tid < OZ_TM + OZ_TN) eb[tid - OZ_TM] = 0;
+    __syncthreads();
+    auto exponents = [&](auto is_a, int count, int groups, int *out) {
+        constexpr bool IS_A = decltype(is_a)::value;
+        const bool kfast = IS_A ? jb.opA != 0 : jb.opB == 0;
+        const int per = OZ_THREADS / groups;
+        const int g = kfast ? tid / per : tid % groups, part = kfast ? tid % per : tid / groups;
+        if (g >= count) return;
+        int top = 0;
+        for (int k = 4 * part; k < jb.K; k += 4 * per) {
+            double v[4];
+            load_run<IS_A, 4>(jb, (IS_A ? m0 : n0) + g, k, v);
 #pragma unroll
-        for (int o = 1; o < PA; o <<= 1) ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-        if (pa == 0) ea[tid / PA] = ma ? ma - 1022 : OZ_NOGROUP;
-        const int gj = n0 + tid / PB, pb = tid % PB;
-        int mb = 0;
-        if (gj < jb.N)
-            for (int k = pb; k < jb.K; k += PB) mb = max(mb, exp_field(job_b(jb, k, gj)));
-#pragma unroll
-        for (int o = 1; o < PB; o <<= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-        if (pb == 0) eb[tid / PB] = mb ? mb - 1022 : OZ_NOGROUP;
-    }
+            for (int q = 0; q < 4; q++) top = max(top, exp_field(v[q]));
+        }
+        if (top) atomicMax(out + g, top);
+    };
+    exponents(std::true_type{}, rows, OZ_TM, ea);
+    exponents(std::false_type{}, cols, OZ_TN, eb);
+    __syncthreads();
+    if (tid < OZ_TM) ea[tid] = ea[tid] ? ea[tid] - 1022 : OZ_NOGROUP;
+    else if (tid < OZ_TM + OZ_TN) eb[tid - OZ_TM] = eb[tid - OZ_TM] ? eb[tid - OZ_TM] - 1022 : OZ_NOGROUP;
     __syncthreads();
 
-    // This thread's share of the read-out: TMEM lanes 32 (warp % 4) .. (rows), columns 32 (warp / 4) ..
+    // This thread's share of the read-out: TMEM lanes 32 (warp % 4) .. (rows), columns 16 (warp / 4) ..
     const int q = warp & 3, h = warp >> 2;
-    long long hi[32], lo[32];  // levels 0-3 at scale 2^-35, levels 4-7 at scale 2^-63
+    const bool reads = q * 32 < rows && h * 16 < cols;
+    unsigned long long hi[16], lo[16];  // levels 0-3 at scale 2^-35, levels 4-7 at scale 2^-63
 #pragma unroll
-    for (int j = 0; j < 32; j++) hi[j] = lo[j] = 0;
+    for (int j = 0; j < 16; j++) hi[j] = lo[j] = 0;
+    int windows = 0;
     bool ok = true;
     auto drain = [&]() {  // every committed MMA complete (each commit waited for exactly once)
         for (int b = 0; b < 2; b++)
@@ -178,38 +241,55 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
             }
         tc::fence_after();
     };
+    // A level sum iv appears as the bit pattern 0x4B400000 + iv of iv + 1.5 2^23; the pattern is added with the
+    // level's weight, what the constant contributes is taken off at the end.
     auto readout = [&]() {
+        if (reads) {
 #pragma unroll 1
-        for (int l = 0; l < OZ_S; l++) {
-            float v[32];
-            tc::tmem_ld32(tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (l * OZ_TN + h * 32), v);
+            for (int l = 0; l < OZ_S; l++) {
+                float v[16];
+                tc::tmem_ld16(tmem + ((uint32_t) (q * 32) << 16) + (uint32_t) (l * OZ_TN + h * 16), v);
+                const uint32_t weight = 1u << (OZ_B * ((l < 4 ? 3 : 7) - l));
+                if (l < 4) {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const long long iv = (long long) (__float_as_int(v[j] + 12582912.0f) - 0x4B400000);
-                if (l < 4) hi[j] += iv << (OZ_B * (3 - l));
-                else lo[j] += iv << (OZ_B * (7 - l));
+                    for (int j = 0; j < 16; j++)
+                        hi[j] += (unsigned long long) __float_as_uint(v[j] + 12582912.0f) * weight;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; j++)
+                        lo[j] += (unsigned long long) __float_as_uint(v[j] + 12582912.0f) * weight;
+                }
             }
         }
+        windows++;
         tc::fence_before();
         __syncthreads();  // the next MMAs overwrite the accumulators only after every read-out
     };
 
+    // this thread's runs: eight K of a row of A, four of a column of B (see oz_off for the layout)
+    const bool ka = jb.opA != 0;
+    const int ra = ka ? tid >> 2 : tid & 127, ca = ka ? tid & 3 : tid >> 7;
+    const int rb = (tid & 7) + 8 * (tid >> 6), cb = ((tid >> 4) & 3) * 8 + ((tid >> 3) & 1) * 4;
     const int nchunks = (jb.K + OZ_KC - 1) / OZ_KC;
     for (int c = 0; c < nchunks; c++) {
-        const int buf = c & 1;
+        const int buf = c & 1, k0 = c * OZ_KC;
         unsigned char *sa = stage0 + buf * OZ_STAGE, *sb = sa + OZ_S * OZ_A_PLANE;
+        double va[8], vb[4];
+        if (ra < rows) load_run<true, 8>(jb, m0 + ra, k0 + 8 * ca, va);
+        if (rb < cols) load_run<false, 4>(jb, n0 + rb, k0 + cb, vb);
         if (pending[buf]) {  // the MMAs of chunk c - 2 have read this stage
             ok &= tc::mbar_wait(mbar0 + 8 * buf, phase[buf]);
             phase[buf] ^= 1;
             pending[buf] = false;
         }
-        split_chunk<true>(jb, m0, OZ_TM, c * OZ_KC, ea, sa, OZ_A_PLANE);
-        split_chunk<false>(jb, n0, OZ_TN, c * OZ_KC, eb, sb, OZ_B_PLANE);
+        if (ra < rows) split_run<8>(va, ea[ra], sa + oz_off(ra, 8 * ca), OZ_A_PLANE);
+        if (rb < cols) split_run<4>(vb, eb[rb], sb + oz_off(rb, cb), OZ_B_PLANE);
         tc::fence_smem_to_async();
         __syncthreads();
-        if (tid == 0) {
+        if (tid == OZ_THREADS - 32) {
             tc::fence_after();
-            const uint32_t a0 = tc::smem_u32(sa), b0 = tc::smem_u32(sb);
+            const uint64_t ad = tc::smem_desc(tc::smem_u32(sa), 128, OZ_KB * 128);
+            const uint64_t bd = tc::smem_desc(tc::smem_u32(sb), 128, OZ_KB * 128);
             const bool first = (c % OZ_FLUSH) == 0;  // accumulators restart after every read-out
 #pragma unroll
             for (int ks = 0; ks < OZ_KC / 16; ks++)
@@ -217,12 +297,11 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
                 for (int s = 0; s < OZ_S; s++)
 #pragma unroll
                     for (int t = 0; t < OZ_S - s; t++) {
-                        const uint64_t ad = tc::smem_desc(a0 + s * OZ_A_PLANE + ks * 256, 128, OZ_KB * 128);
-                        const uint64_t bd = tc::smem_desc(b0 + t * OZ_B_PLANE + ks * 256, 128, OZ_KB * 128);
                         // The first MMA into level L of a read-out window overwrites it: in this order
                         // that is the pair (0, L) of the window's first k-step.
                         const bool overwrite = first && ks == 0 && s == 0;
-                        tc::mma_f16(tmem + (uint32_t) ((s + t) * OZ_TN), ad, bd, IDESC, overwrite ? 0u : 1u);
+                        tc::mma_f16(tmem + (uint32_t) ((s + t) * OZ_TN), ad + ((s * OZ_A_PLANE + ks * 256) >> 4),
+                                    bd + ((t * OZ_B_PLANE + ks * 256) >> 4), idesc, overwrite ? 0u : 1u);
                     }
             tc::commit(mbar0 + 8 * buf);
         }
@@ -234,19 +313,21 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     }
     if (!ok && tid == 0) atomicAdd(&g_oz_wait_timeouts, 1u);
 
-    // Epilogue: C = alpha * product + beta * C, one row per thread, 32 columns.
-    const int row_l = q * 32 + lane, row = m0 + row_l;
-    if (row < jb.M) {
-        const bool scale = jb.alpha != 1.0, accum = jb.beta != 0.0;
+    // Epilogue: C = alpha * product + beta * C, one row per thread, 16 columns.
+    const int row_l = q * 32 + lane;
+    if (reads && row_l < rows) {
+        const unsigned long long constant =
+            (unsigned long long) windows * 0x4B400000ull * ((1ull << 21) + (1ull << 14) + (1ull << 7) + 1ull);
+        const bool scale = jb.alpha != 1.0 && jb.alpha != -1.0, negate = jb.alpha == -1.0, accum = jb.beta != 0.0;
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-            const int cl = h * 32 + j, col = n0 + cl;
-            if (col < jb.N) {
-                double *cp = jb.C + row + (size_t) col * jb.ldc;
-                const int eab = ea[row_l] + eb[cl];
-                double prod = 0.0;
-                if (jb.K > 0) prod = fma((double) hi[j], pow2(eab - 35), (double) lo[j] * pow2(eab - 63));
-                double v = scale ? jb.alpha * prod : prod;
+        for (int j = 0; j < 16; j++) {
+            const int cl = h * 16 + j;
+            if (cl < cols) {
+                double *cp = jb.C + m0 + row_l + (size_t) (n0 + cl) * jb.ldc;
+                double v = 0.0;
+                if (jb.K > 0) v = oz_value((long long) (hi[j] - constant), (long long) (lo[j] - constant), ea[row_l] + eb[cl]);
+                if (negate) v = -v;
+                if (scale) v *= jb.alpha;
                 if (accum) v = fma(jb.beta, *cp, v);
                 *cp = v;
             }
