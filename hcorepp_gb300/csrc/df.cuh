@@ -127,6 +127,29 @@ __device__ __forceinline__ df df_acc_value(df_acc acc) {  // two-sum: |e| may ex
     return r;
 }
 
+// v 2^-e as a float-float value (|v| < 2^(e + 1); what falls below the float range is dropped), and f 2^e as a
+// double, by integer operations: a conversion or scaling on the FP64 pipe holds an SM for ~19 cycles a warp.
+__device__ __forceinline__ df df_scaled_down(double v, int e) {
+    const unsigned hi = (unsigned) __double2hiint(v), lo = (unsigned) __double2loint(v);
+    const int x = (int) ((hi >> 20) & 0x7ffu), f = x - 1023 - e + 127;
+    df r = df_f(0.f);
+    if (x == 0 || f <= 0) return r;
+    const unsigned sign = hi & 0x80000000u;
+    r.h = __uint_as_float(sign | ((unsigned) f << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+    const float rest = __uint2float_rn(lo & 0x1fffffffu);  // in units of 2^(f - 127 - 52)
+    const float unit = f > 52 ? __uint_as_float((unsigned) (f - 52) << 23) : 0.f;
+    r.l = sign ? -rest * unit : rest * unit;
+    return r;
+}
+__device__ __forceinline__ double double_scaled_up(float f, int e) {
+    const unsigned b = __float_as_uint(f);
+    const int x = (int) ((b >> 23) & 0xffu);
+    const int d = x - 127 + 1023 + e;
+    if (x == 0 || d <= 0) return 0.0;
+    const unsigned m = b & 0x7fffffu;
+    return __hiloint2double((int) ((b & 0x80000000u) | ((unsigned) (d < 0x7ff ? d : 0x7ff) << 20) | (m >> 3)), (int) (m << 29));
+}
+
 // Sum over groups of G consecutive lanes (G a power of two <= 32), every lane gets its group's sum.
 __device__ __forceinline__ df df_group_sum(df v, int G) {
     for (int o = G >> 1; o > 0; o >>= 1) {

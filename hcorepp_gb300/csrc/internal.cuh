@@ -86,6 +86,42 @@ __device__ __forceinline__ T *cluster_map(T *p, int rank) {
     return q;
 }
 
+// Every kernel launch of the library is counted (hcgb_kernel_launches reads the total).
+void note_launch();
+
+// Two launches on different updates run side by side in one stream: the first (the wide updates' clusters) lets the
+// second start as soon as it runs itself; the second's first CTA ends only when the first is done, so what
+// follows in the stream comes after both.  (A second stream would do, but the groups of a multiply already
+// take every hardware queue: with one more stream a group the multiplies of few tiles took 30 % longer.)
+__device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous_launch() {
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Launches the second of two such kernels (beside = whether there is a first one); cluster: its CTAs per cluster.
+template <class... P, class... A>
+void launch_beside(bool beside, int cluster, int grid, int block, size_t smem, cudaStream_t st, void (*kernel)(P...), A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    cfg.attrs = at;
+    cfg.numAttrs = 0;
+    if (beside) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = cluster;
+        at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+        cfg.numAttrs++;
+    }
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+    note_launch();
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -172,6 +208,9 @@ enum MetaField {
     META_INTS = 22
 };
 
+constexpr int WIDE_CTAS = 8;       // CTAs of a wide core's cluster
+constexpr int WIDE_CLUSTERS = 19;  // clusters of a launch (152 SMs / 8)
+
 // Device workspace: n slots of `slot_doubles` doubles plus an int meta block.
 struct Workspace {
     double *base;
@@ -182,6 +221,7 @@ struct Workspace {
     int kmax;             // max columns of a stack
     int rmax;             // max rank of an A/B factor
     int conc = 1;         // launches like this one in flight at a time (the C-tile groups of a multiply)
+    int k_wide, k_heavy;  // stack widths above which a core does not fit an SM's / half an SM's shared memory
     size_t off_ustack, off_vstack, off_tmp1, off_tmp2, off_tauu, off_tauv, off_tu, off_tv;
     size_t off_m, off_mcopy, off_xv, off_sigma, off_mixed;
     size_t off_w;  // WY application: W_U, W_V (kmax x kmax each), present when built with wy
@@ -193,6 +233,28 @@ struct Workspace {
     // Update processed by CTA `b` of the QR / core / Q-application launches: largest first, so the
     // long updates of a launch start at once instead of after the short ones.
     __device__ int heavy(int b) const { return order ? order[b] : b; }
+    // Key of an update in `order` (descending): its stack width when C is compressed.  Both fields are written by
+    // the plan kernel only, so the key is stable while the heavy stages run.
+    __device__ int key(int slot) const {
+        const int *m = meta + (size_t) slot * META_INTS;
+        return m[META_CKIND] ? m[META_K] : 0;
+    }
+    // Updates of `order` (of n) with a key above thr.
+    __device__ int count_above(int n, int thr) const {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key(order[mid]) > thr) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    }
+    // The first wide_updates(n) updates of `order` go to clusters of CTAs, stack QR and core: those whose core does not
+    // fit an SM, and the heavy ones too while the launches in flight leave SMs for them.
+    __device__ int wide_updates(int n) const {
+        const int h = count_above(n, k_heavy);
+        return (long) h * conc <= WIDE_CLUSTERS ? h : count_above(n, k_wide);
+    }
 };
 
 // Layout of one workspace slot for stacks of up to `ld` rows and `kmax` columns; factor ranks
@@ -251,6 +313,8 @@ void launch_plan_wy(const DevUpdate *ups, int n, Workspace ws, Params p, GemmJob
 void launch_wy_solve(int n, Workspace ws, cudaStream_t st);
 void launch_qr(Workspace ws, int n, bool mixed, cudaStream_t st);
 void launch_core_svd(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st);
+// Stack widths up to which a core fits a whole, half and a quarter of an SM's shared memory in launches of kmax.
+void core_classes(int kmax, int *whole, int *half, int *quarter);
 void launch_apply_q(const DevUpdate *ups, int n, Workspace ws, bool mixed, cudaStream_t st);
 void launch_finalize(const DevUpdate *ups, int n, Workspace ws, hcgb_update_info *info, cudaStream_t st);
 // FP64 throughput probes (TFLOP/s): tensor-core DMMA and SIMT DFMA.
@@ -271,9 +335,6 @@ void launch_syrk(int uplo, int trans, int n, int k, double alpha, const double *
 
 // Rank-trimmed packing of a tile list (pack.cu): offsets (n + 1) and the packed copy, or back.
 void launch_pack(const DevTile *tiles, int n, long long *offsets, double *packed, bool unpack, cudaStream_t st);
-
-// Every kernel launch of the library is counted (hcgb_kernel_launches reads the total).
-void note_launch();
 
 // ---- learned form (learned.cu): features, sketch recompression and its fallback ----
 // Per-update features (ws.feat, and sink[uid * MLP_IN ..] when sink != null); needs ws.feat.

@@ -308,14 +308,10 @@ __device__ QrShared carve(double *sm, int ld, int kmax) {
     return s;
 }
 
-// Side blockIdx.x / C of the launch (2s: the U stack of update s, 2s + 1: its V stack), by a cluster of C CTAs:
-// each factors every panel for itself (no broadcast of V and T) and updates its share of the trailing columns;
+// One side (0: the U stack, 1: the V stack) of an update by a cluster of C CTAs: each factors every panel for itself (no broadcast of V and T) and updates its share of the trailing columns;
 // the first CTA writes the panel back.  A column's arithmetic does not depend on C.
 template <int C>
-__global__ void __launch_bounds__(QR_THREADS) qr_kernel(Workspace ws) {
-    extern __shared__ double sm[];
-    const int part = C > 1 ? cluster_rank() : 0;
-    const int id = blockIdx.x / C, slot = ws.heavy(id >> 1), side = id & 1;
+__device__ void qr_side(const Workspace &ws, int slot, int side, int part, double *sm) {
     const int *meta = ws.meta + (size_t) slot * META_INTS;
     if (meta[META_STATUS] != HCGB_OK || !meta[META_CKIND]) return;
     const int k = meta[META_K];
@@ -366,6 +362,32 @@ __global__ void __launch_bounds__(QR_THREADS) qr_kernel(Workspace ws) {
             cluster_wait();
         }
         __syncthreads();
+    }
+}
+
+// Sides blockIdx.x / C (2s, 2s + 1: of the s-th update in order) but the wide updates'.
+template <int C>
+__global__ void __launch_bounds__(QR_THREADS) qr_kernel(Workspace ws, int nup) {
+    extern __shared__ double sm[];
+    __shared__ int s_wide;
+    const int id = blockIdx.x / C, slot = ws.heavy(id >> 1);
+    if (threadIdx.x == 0) s_wide = ws.order ? ws.wide_updates(nup) : (ws.key(slot) > ws.k_heavy ? nup : 0);
+    __syncthreads();
+    if ((id >> 1) >= s_wide) qr_side<C>(ws, slot, id & 1, C > 1 ? cluster_rank() : 0, sm);
+    wait_for_previous_launch();
+}
+
+// The wide updates' sides, clusters striding over them.
+template <int C>
+__global__ void __launch_bounds__(QR_THREADS) qr_wide_kernel(Workspace ws, int nup) {
+    extern __shared__ double sm[];
+    __shared__ int s_wide;
+    let_next_launch_start();
+    if (threadIdx.x == 0) s_wide = ws.order ? ws.wide_updates(nup) : nup;
+    __syncthreads();
+    for (int id = blockIdx.x / C; id < 2 * s_wide; id += gridDim.x / C) {
+        const int slot = ws.heavy(id >> 1);
+        if (ws.key(slot) > ws.k_heavy) qr_side<C>(ws, slot, id & 1, cluster_rank(), sm);
     }
 }
 
@@ -666,20 +688,7 @@ __device__ void apply_q_side_df(const TM &tm, const DevUpdate *ups, const Worksp
 // the launch.  Returns false for threads without work.
 __device__ bool qr_assign(const Workspace &ws, int nup, int pair, int &slot, int &side, int &half, bool &heavy) {
     __shared__ int s_nheavy;
-    if (threadIdx.x == 0) {
-        int h = -1;
-        if (ws.order) {
-            int lo = 0, hi = nup;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                const int *m = ws.meta + (size_t) ws.order[mid] * META_INTS;
-                if ((m[META_CKIND] ? m[META_K] : 0) > QR_HEAVY_K) lo = mid + 1;
-                else hi = mid;
-            }
-            h = lo;
-        }
-        s_nheavy = h;
-    }
+    if (threadIdx.x == 0) s_nheavy = ws.order ? ws.count_above(nup, QR_HEAVY_K) : -1;
     __syncthreads();
     const int H = s_nheavy;
     constexpr int HALF = QRD_THREADS / 2;
@@ -756,21 +765,24 @@ static bool qr_pair_fits(size_t team_bytes) {
 }
 
 template <int C>
-static void launch_qr_clusters(Workspace ws, int n, size_t smem, cudaStream_t st) {
+static void launch_qr_clusters(bool wide, Workspace ws, int n, size_t smem, cudaStream_t st) {
     cudaFuncSetAttribute(qr_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * n * C);
-    cfg.blockDim = dim3(QR_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = C;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = C > 1 ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, qr_kernel<C>, ws);
-    note_launch();
+    launch_beside(wide, C, 2 * n * C, QR_THREADS, smem, st, qr_kernel<C>, ws, n);
+}
+
+template <int C>
+static void launch_qr_wide_clusters(Workspace ws, int n, size_t smem, cudaStream_t st) {
+    cudaFuncSetAttribute(qr_wide_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    const int clusters = 2 * n < QR_SMS / C ? 2 * n : QR_SMS / C;
+    launch_beside(false, C, clusters * C, QR_THREADS, smem, st, qr_wide_kernel<C>, ws, n);
+}
+
+// Clusters of four cost a 200-column side 1.4 times the SM time of one CTA and a third of its duration; of eight
+// while few updates are in flight.
+static void launch_qr_wide(Workspace ws, int n, cudaStream_t st) {
+    const size_t smem = qr_smem_bytes(ws.ld, ws.kmax);
+    if (2L * n * ws.conc * 8 <= 2 * QR_SMS) launch_qr_wide_clusters<8>(ws, n, smem, st);
+    else launch_qr_wide_clusters<4>(ws, n, smem, st);
 }
 
 void launch_qr(Workspace ws, int n, bool mixed, cudaStream_t st) {
@@ -783,11 +795,13 @@ void launch_qr(Workspace ws, int n, bool mixed, cudaStream_t st) {
     } else {
         // A cluster per side while the launches in flight leave SMs idle: at k = 340, m = 512 one CTA took
         // 15.7 ms (its SM's FP64 pipe).
+        const bool wide = ws.kmax > ws.k_heavy;
+        if (wide) launch_qr_wide(ws, n, st);
         const long sides = 2L * n * ws.conc;
-        if (sides * 8 <= QR_SMS) launch_qr_clusters<8>(ws, n, smem, st);
-        else if (sides * 4 <= QR_SMS) launch_qr_clusters<4>(ws, n, smem, st);
-        else if (sides * 2 <= QR_SMS) launch_qr_clusters<2>(ws, n, smem, st);
-        else launch_qr_clusters<1>(ws, n, smem, st);
+        if (sides * 8 <= QR_SMS) launch_qr_clusters<8>(wide, ws, n, smem, st);
+        else if (sides * 4 <= QR_SMS) launch_qr_clusters<4>(wide, ws, n, smem, st);
+        else if (sides * 2 <= QR_SMS) launch_qr_clusters<2>(wide, ws, n, smem, st);
+        else launch_qr_clusters<1>(wide, ws, n, smem, st);
     }
 }
 

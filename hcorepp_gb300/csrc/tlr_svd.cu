@@ -28,8 +28,6 @@ namespace hcgb {
 namespace {
 
 constexpr int SVD_THREADS = 512;
-constexpr int WIDE_CTAS = 8;              // CTAs of a wide update's cluster
-constexpr int WIDE_CLUSTERS = 19;         // clusters of a launch (152 SMs / 8)
 constexpr int WIDE_POOL_DOUBLES = 16640;  // shared memory of a CTA for a pair of column blocks (130 KB)
 constexpr float PRECOND_TOL32 = 1e-6f;  // above the rounding of a single-precision cosine
 constexpr int PRECOND_MAX_SWEEPS = 12;
@@ -354,68 +352,115 @@ __device__ __forceinline__ float rotation_tangent(float zeta) {
     return copysignf(1.f, zeta) / (fabsf(zeta) + sqrtf(fmaf(zeta, zeta, 1.f)));
 }
 
-// One sweep over columns [0, nc_a) and [off_b, off_b + nc_b) of Y: every pair (cross = false), or the pairs
-// of one column of each range (cross = true).  A column is x4 + j4 quads of floats, ls4 quads apart: its
-// part of X32 and its part of J32 (zero padded); the inner products take the first, rotations both.
+// Pair `pp` of step t over columns [0, nc_a) and [off_b, off_b + nc_b): round robin over all of them (cross =
+// false) or one column of each range.  Returns whether the step has such a pair.
+__device__ __forceinline__ bool sweep_pair(int t, int pp, int nc_a, int nc_b, int off_b, bool cross, int &i, int &j) {
+    if (cross) {
+        const int wide = nc_a > nc_b ? nc_a : nc_b;
+        const int q = pp + t < wide ? pp + t : pp + t - wide;
+        i = pp;
+        j = off_b + q;
+        return t < wide && pp < nc_a && q < nc_b;
+    }
+    const int nc = nc_a + nc_b, n2 = nc + (nc & 1);
+    if (t >= n2 - 1 || pp >= n2 / 2) return false;
+    jacobi_pair(t, pp, n2, i, j);
+    if (i >= nc || j >= nc) return false;
+    i = i < nc_a ? i : off_b + i - nc_a;
+    j = j < nc_a ? j : off_b + j - nc_a;
+    return true;
+}
+
+// Rotates columns x and y (x4 quads of X32, then j4 of J32, zero padded) by G lanes when their cosine exceeds tol;
+// the inner products take the first part, the rotation both.  Every lane of the warp calls.
+template <int G>
+__device__ __forceinline__ int jacobi32_rotate(bool act, float4 *x, float4 *y, int x4, int j4, int gl, float tol) {
+    float a = 0.f, b = 0.f, c = 0.f;
+    if (act) {
+#pragma unroll 4
+        for (int r = gl; r < x4; r += G) {
+            const float4 u = x[r], v = y[r];
+            a = fmaf(u.x, u.x, fmaf(u.y, u.y, fmaf(u.z, u.z, fmaf(u.w, u.w, a))));
+            b = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, b))));
+            c = fmaf(u.x, v.x, fmaf(u.y, v.y, fmaf(u.z, v.z, fmaf(u.w, v.w, c))));
+        }
+    }
+#pragma unroll
+    for (int o = G >> 1; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (!(act && a > 0.f && b > 0.f && fabsf(c) * rsqrtf(a) * rsqrtf(b) > tol)) return 0;
+    const float zeta = (b - a) / (2.f * c);
+    const float tt = rotation_tangent(zeta);
+    const float cs = 1.f / sqrtf(fmaf(tt, tt, 1.f)), sn = cs * tt;
+#pragma unroll 4
+    for (int r = gl; r < x4 + j4; r += G) {
+        const float4 u = x[r], v = y[r];
+        x[r] = make_float4(fmaf(cs, u.x, -sn * v.x), fmaf(cs, u.y, -sn * v.y), fmaf(cs, u.z, -sn * v.z),
+                           fmaf(cs, u.w, -sn * v.w));
+        y[r] = make_float4(fmaf(cs, v.x, sn * u.x), fmaf(cs, v.y, sn * u.y), fmaf(cs, v.z, sn * u.z),
+                           fmaf(cs, v.w, sn * u.w));
+    }
+    return gl == 0;
+}
+
+// One sweep over the columns of Y (ls4 quads apart), in shared memory: round robin (blocks = 0), or the cluster's
+// order of column blocks (blocks = their number: jacobi32_blocks), block pairs side by side, so that a core gives the
+// same result on one SM and on a cluster.
 template <int G, class TM>
-__device__ int jacobi32_sweep(const TM &tm, float4 *Y, int ls4, int x4, int j4, int nc_a, int nc_b, int off_b,
-                              bool cross, float tol) {
+__device__ int jacobi32_sweep(const TM &tm, float4 *Y, int ls4, int x4, int j4, int nc, int blocks, float tol) {
+    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
+    constexpr int PPW = 32 / G;
+    const int gl = lane % G, grp = lane / G;
+    const int w = blocks ? (nc + blocks - 1) / blocks : nc, per = blocks ? w : (nc + 1) / 2;
+    const int npairs = blocks ? blocks / 2 * per : per, nchunks = (npairs + PPW - 1) / PPW;
+    const int rounds = blocks ? blocks - 1 : 1, n2 = nc + (nc & 1);
+    int rotations = 0;
+    for (int round = 0; round < rounds; round++) {
+        const int steps = blocks ? (round ? w : 2 * w - 1) : n2 - 1;
+        for (int t = 0; t < steps; t++) {
+            for (int ch = warp; ch < nchunks; ch += nw) {
+                const int id = ch * PPW + grp;
+                int i = 0, j = 0;
+                bool act = id < npairs;
+                if (act && blocks) {
+                    int bi, bj;
+                    jacobi_pair(round, id / per, blocks, bi, bj);
+                    const int ra = nc - bi * w, rb = nc - bj * w;
+                    const int na = ra < 0 ? 0 : (ra < w ? ra : w), nb = rb < 0 ? 0 : (rb < w ? rb : w);
+                    act = sweep_pair(t, id % per, na, nb, (bj - bi) * w, round > 0, i, j);
+                    i += bi * w;
+                    j += bi * w;
+                } else if (act) {
+                    act = sweep_pair(t, id, nc, 0, 0, false, i, j);
+                }
+                rotations += jacobi32_rotate<G>(act, Y + (size_t) (act ? i : 0) * ls4, Y + (size_t) (act ? j : 0) * ls4, x4,
+                                                j4, gl, tol);
+            }
+            tm.sync();
+        }
+    }
+    return rotations;
+}
+
+// The steps of one block pair (columns [0, nc_a) and [off_b, off_b + nc_b) of Y, ls4 quads apart) by one CTA.
+template <int G, class TM>
+__device__ int jacobi32_block_pair(const TM &tm, float4 *Y, int ls4, int x4, int j4, int nc_a, int nc_b, int off_b,
+                                   bool cross, float tol) {
     const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
     constexpr int PPW = 32 / G;
     const int gl = lane % G, grp = lane / G;
     const int nc = nc_a + nc_b, n2 = nc + (nc & 1), wide = nc_a > nc_b ? nc_a : nc_b;
     const int npairs = cross ? wide : n2 / 2, steps = cross ? wide : n2 - 1;
-    const int nchunks = (npairs + PPW - 1) / PPW;
     int rotations = 0;
     for (int t = 0; t < steps; t++) {
-        for (int ch = warp; ch < nchunks; ch += nw) {
-            const int pp = ch * PPW + grp;
+        for (int p0 = warp * PPW; p0 < npairs; p0 += nw * PPW) {
             int i = 0, j = 0;
-            bool act = pp < npairs;
-            if (act) {
-                if (cross) {
-                    const int q = pp + t < wide ? pp + t : pp + t - wide;
-                    act = pp < nc_a && q < nc_b;
-                    i = pp;
-                    j = off_b + q;
-                } else {
-                    jacobi_pair(t, pp, n2, i, j);
-                    act = i < nc && j < nc;
-                    i = i < nc_a ? i : off_b + i - nc_a;
-                    j = j < nc_a ? j : off_b + j - nc_a;
-                }
-            }
-            float4 *x = Y + (size_t) (act ? i : 0) * ls4, *y = Y + (size_t) (act ? j : 0) * ls4;
-            float a = 0.f, b = 0.f, c = 0.f;
-            if (act) {
-#pragma unroll 4
-                for (int r = gl; r < x4; r += G) {
-                    const float4 u = x[r], v = y[r];
-                    a = fmaf(u.x, u.x, fmaf(u.y, u.y, fmaf(u.z, u.z, fmaf(u.w, u.w, a))));
-                    b = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, b))));
-                    c = fmaf(u.x, v.x, fmaf(u.y, v.y, fmaf(u.z, v.z, fmaf(u.w, v.w, c))));
-                }
-            }
-#pragma unroll
-            for (int o = G >> 1; o > 0; o >>= 1) {
-                a += __shfl_xor_sync(0xffffffffu, a, o);
-                b += __shfl_xor_sync(0xffffffffu, b, o);
-                c += __shfl_xor_sync(0xffffffffu, c, o);
-            }
-            if (act && a > 0.f && b > 0.f && fabsf(c) * rsqrtf(a) * rsqrtf(b) > tol) {
-                const float zeta = (b - a) / (2.f * c);
-                const float tt = rotation_tangent(zeta);
-                const float cs = 1.f / sqrtf(fmaf(tt, tt, 1.f)), sn = cs * tt;
-#pragma unroll 4
-                for (int r = gl; r < x4 + j4; r += G) {
-                    const float4 u = x[r], v = y[r];
-                    x[r] = make_float4(fmaf(cs, u.x, -sn * v.x), fmaf(cs, u.y, -sn * v.y), fmaf(cs, u.z, -sn * v.z),
-                                       fmaf(cs, u.w, -sn * v.w));
-                    y[r] = make_float4(fmaf(cs, v.x, sn * u.x), fmaf(cs, v.y, sn * u.y), fmaf(cs, v.z, sn * u.z),
-                                       fmaf(cs, v.w, sn * u.w));
-                }
-                if (gl == 0) rotations++;
-            }
+            const bool act = sweep_pair(t, p0 + grp, nc_a, nc_b, off_b, cross, i, j);
+            rotations += jacobi32_rotate<G>(act, Y + (size_t) (act ? i : 0) * ls4, Y + (size_t) (act ? j : 0) * ls4, x4, j4,
+                                            gl, tol);
         }
         tm.sync();
     }
@@ -557,7 +602,11 @@ __device__ void ns_apply(const TM &tm, const float *J, int ldj, int rk, df *E, f
 #pragma unroll
             for (int q = 0; q < 2; q++) {
                 const int i = i0 + lane + 32 * q;
-                if (i < rk) out[i] = (double) J[i + (size_t) j * ldj] + (double) df_acc_value(acc[q]);
+                if (i < rk) {
+                    const df d = df_acc_value(acc[q]);
+                    out[i] = double_scaled_up(J[i + (size_t) j * ldj], 0) +
+                             (double_scaled_up(d.h, 0) + double_scaled_up(d.l, 0));
+                }
             }
         }
         __syncwarp();
@@ -592,11 +641,9 @@ __device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh
                 e = e > f ? e : f;
             }
             e = e ? e - 1023 : -1022;
-            if (e > 1022) e = 1022;  // 2^-e stays a normal number
-            const double down = __hiloint2double((1023 - e) << 20, 0);
             df sq = df_f(0.f);
             for (int r = lane; r < rows; r += 32) {
-                const df v = df(w[r] * down);
+                const df v = df_scaled_down(w[r], e);
                 Wh[r + (size_t) j * ldh] = v;
                 sq = df_fma(v, v, sq);
             }
@@ -697,9 +744,9 @@ __device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh
             },
             [](df_acc &c, df a, df b) { df_acc_fma(c, a, b); }, [](int, int) { return df_acc{0.f, 0.f}; },
             [&](int i, int j, df_acc c) {
-                const double up = __hiloint2double((1023 + ex[j]) << 20, 0);  // ex >= -1022
+                const df d = df_acc_value(c);
                 double *w = W + i + (size_t) j * rows;
-                *w = fma((double) df_acc_value(c), up, *w);
+                *w += double_scaled_up(d.h, ex[j]) + double_scaled_up(d.l, ex[j]);  // the inner sum is exact
             },
             [](int, int) { return true; });
         tm.sync();
@@ -709,6 +756,12 @@ __device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh
     return false;
 }
 
+
+// Stack widths up to which a core fits a quarter and half of an SM's shared memory: the sweep's order and lanes per pair
+// go by the width, not by the team that a launch gives the update.
+constexpr int SMALL_K = 82, LIGHT_K = 117;
+constexpr int SWEEP_BLOCKS = 2 * WIDE_CTAS;  // column blocks of a core that a cluster can hold two at a time a CTA
+constexpr int BLOCK_G16_QUADS = 42;          // up to 168 rows
 
 // Column blocks of the cluster's sweeps: every CTA of the cluster holds one pair of blocks at a time in its
 // shared memory (buf, `quads` float4s) and sweeps the pairs of columns that it gives; the blocks meet in
@@ -722,6 +775,7 @@ __device__ int jacobi32_blocks(const TM &tm, float4 *Y, int x4, int j4, int nc, 
         w = (nc + nblk - 1) / nblk;
     } while (w > 1 && 2 * w * L > quads);
     const Team<TM::cta_threads> ct{(int) threadIdx.x, 1};
+    const bool rows_g16 = x4 <= BLOCK_G16_QUADS;  // cores that one SM can hold: the lanes per pair it takes
     int rot = 0;
     for (int t = 0; t < nblk - 1; t++) {
         for (int pp = tm.rank; pp < nblk / 2; pp += TM::ctas) {
@@ -734,8 +788,8 @@ __device__ int jacobi32_blocks(const TM &tm, float4 *Y, int x4, int j4, int nc, 
             for (int e = threadIdx.x; e < na * L; e += TM::cta_threads) buf[e] = __ldcg(ya + e);
             for (int e = threadIdx.x; e < nb * L; e += TM::cta_threads) buf[w * L + e] = __ldcg(yb + e);
             ct.sync();
-            if (w <= TM::cta_threads / 32) rot += jacobi32_sweep<32>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
-            else rot += jacobi32_sweep<16>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
+            if (rows_g16) rot += jacobi32_block_pair<16>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
+            else rot += jacobi32_block_pair<32>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
             for (int e = threadIdx.x; e < na * L; e += TM::cta_threads) ya[e] = buf[e];
             for (int e = threadIdx.x; e < nb * L; e += TM::cta_threads) yb[e] = buf[w * L + e];
             ct.sync();
@@ -753,6 +807,8 @@ __device__ int jacobi32_blocks(const TM &tm, float4 *Y, int x4, int j4, int nc, 
 struct PrecondBuffers {
     float4 *y;
     int ls4;           // quads per column of y
+    int blocks;        // column blocks of the sweep order (0: round robin)
+    bool g8;           // round robin: eight lanes a pair, not four
     float4 *buf;       // cluster: shared memory for a pair of blocks and the vectors of ns_apply
     int buf_quads;
     double *e64;
@@ -783,10 +839,9 @@ __device__ bool jacobi_precond(const TM &tm, const double *X, int ldx, int rows,
     atomicMax(s_emax, em);
     tm.sync();
     const int esc = *s_emax ? *s_emax - 1023 : 0;
-    const double down = __hiloint2double((1023 - (esc > 1022 ? 1022 : esc)) << 20, 0);
     for (int j = warp; j < nc; j += nw) {
         float *y = Y + (size_t) j * ldy;
-        for (int r = lane; r < 4 * x4; r += 32) y[r] = r < rows ? (float) (X[r + (size_t) j * ldx] * down) : 0.f;
+        for (int r = lane; r < 4 * x4; r += 32) y[r] = r < rows ? df_scaled_down(X[r + (size_t) j * ldx], esc).h : 0.f;
         for (int r = lane; r < 4 * j4; r += 32) y[4 * x4 + r] = r == j ? 1.f : 0.f;
     }
     tm.sync();
@@ -796,7 +851,9 @@ __device__ bool jacobi_precond(const TM &tm, const double *X, int ldx, int rows,
         tm.sync();
         int rot;
         if constexpr (TM::ctas > 1) rot = jacobi32_blocks(tm, b.y, x4, j4, nc, b.buf, b.buf_quads, PRECOND_TOL32);
-        else rot = jacobi32_sweep<4>(tm, b.y, b.ls4, x4, j4, nc, 0, 0, false, PRECOND_TOL32);
+        else if (b.blocks) rot = jacobi32_sweep<16>(tm, b.y, b.ls4, x4, j4, nc, b.blocks, PRECOND_TOL32);
+        else if (b.g8) rot = jacobi32_sweep<8>(tm, b.y, b.ls4, x4, j4, nc, 0, PRECOND_TOL32);
+        else rot = jacobi32_sweep<4>(tm, b.y, b.ls4, x4, j4, nc, 0, PRECOND_TOL32);
         if (rot) atomicAdd(s_rot, rot);
         tm.sync();
         const int total = *s_rot;
@@ -941,27 +998,34 @@ __device__ int qrcp_steps(const TM &tm, double *A, int lda, int mrows, int ncols
     tm.sync();
     const int kk = mrows < ncols ? mrows : ncols;
     double lim = stop2;
+    int rk = kk;
     for (int s = 0; s < kk; s++) {
         if (warp == 0) {
             long long bv = -1;
-            int bi = s;
+            int bi = ncols, at = s;  // the largest norm's column (ties to the lower one) and its place in pvt
             for (int j = s + lane; j < ncols; j += 32) {
-                long long v = __double_as_longlong(nrm[pvt[j]]);
+                const int c = pvt[j];
+                long long v = __double_as_longlong(nrm[c]);
                 if (v > NRM_MAX_BITS) v = -1;
-                if (v > bv) {
+                if (v > bv || (v == bv && c < bi)) {
                     bv = v;
-                    bi = j;
+                    bi = c;
+                    at = j;
                 }
             }
-            warp_argmax(bv, bi);
+            {
+                const int mine = bi;
+                warp_argmax(bv, bi);
+                at = __shfl_sync(0xffffffffu, at, __ffs(__ballot_sync(0xffffffffu, mine == bi)) - 1);
+            }
             const double top = bv < 0 ? 0.0 : __longlong_as_double(bv);
             if (s == 0 && stop2 == 0.0 && rel > 0.0) lim = rel * rel * top;
             const bool stop = top <= lim || top <= 0.0;
             if (!stop) {
-                const int cs = pvt[bi];
+                const int cs = bi;
                 __syncwarp();
                 if (lane == 0) {
-                    pvt[bi] = pvt[s];
+                    pvt[at] = pvt[s];
                     pvt[s] = cs;
                 }
                 double *x = A + (size_t) cs * lda;
@@ -980,7 +1044,10 @@ __device__ int qrcp_steps(const TM &tm, double *A, int lda, int mrows, int ncols
             if (lane == 0) redi[0] = stop;
         }
         tm.sync();
-        if (redi[0]) return s;
+        if (redi[0]) {
+            rk = s;
+            break;
+        }
         const Reflector h{0.0, red[0], red[1]};
         const double *x = A + (size_t) redi[1] * lda;
         for (int j0 = s + 1 + warp * CPW; j0 < ncols; j0 += nw * CPW) {
@@ -991,7 +1058,17 @@ __device__ int qrcp_steps(const TM &tm, double *A, int lda, int mrows, int ncols
         }
         tm.sync();
     }
-    return kk;
+    // the columns never chosen, in ascending order (at most one a thread: a team has more threads than columns)
+    const int j = rk + tm.tid;
+    int c = 0, pos = rk;
+    if (j < ncols) {
+        c = pvt[j];
+        for (int t = rk; t < ncols; t++) pos += pvt[t] < c;
+    }
+    tm.sync();
+    if (j < ncols) pvt[pos] = c;
+    tm.sync();
+    return rk;
 }
 
 // Columns of up to 64, 256 or more rows are handled by groups of 4, 8 or 16 lanes, several columns per warp
@@ -1009,16 +1086,15 @@ __device__ int qrcp_truncated(const TM &tm, double *A, int lda, int mrows, int n
 // forms the reflector itself.  (Through global memory a step took 24,000 cycles on a 130-column core, bound
 // by dependent L2 round trips and five cluster barriers.)  R goes to X = R^T directly (rk columns of
 // ncols entries, ld ldx, entry t of column s for pivot order t).  pvt: shared by the cluster.
-constexpr int QRCP_CLUSTER_G = 16;
 __host__ __device__ __forceinline__ int qrcp_cluster_doubles(int mrows, int ncols, int ctas) {
     const int nl = (ncols + ctas - 1) / ctas;
     return mrows * nl + 3 * nl + 2 * mrows + (ncols + 1) / 2 + 6 * ctas + 8;
 }
 
-template <class TM>
+template <int G, class TM>
 __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, int ncols, double stop2, double rel,
                             double *X, int ldx, int *pvt, double *pool) {
-    constexpr int C = TM::ctas, G = QRCP_CLUSTER_G, CPW = 32 / G;
+    constexpr int C = TM::ctas, CPW = 32 / G;
     const Team<TM::cta_threads> ct{(int) threadIdx.x, 1};
     const int warp = ct.warp(), lane = threadIdx.x & 31, nw = ct.nw(), rank = tm.rank;
     const int gl = lane % G, grp = lane / G;
@@ -1084,10 +1160,11 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
         if (warp == 0) {
             const double *x = cluster_map(A, owner) + (size_t) lcol * mrows;
             double t = 0.0;
-            for (int i = s + lane; i < mrows; i += 32) {
+            if (lane == 0) xb[s] = x[s];
+            for (int i = s + 1 + lane; i < mrows; i += 32) {
                 const double v = x[i];
                 xb[i] = v;
-                if (i > s) t = fma(v, v, t);
+                t = fma(v, v, t);
             }
             t = warp_sum(t);
             __syncwarp();
@@ -1290,107 +1367,93 @@ template <int RPL, class TM>
 __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace &ws, const Params &p, int slot,
                             double *sm, double *pool, int pool_doubles, CoreShared &sh);
 
-// Stage key of an update in ws.order (sorted by decreasing key): its stack width k when C is
-// compressed.  Both fields are written by the plan kernel only, so the key is stable while the
-// heavy stages run.
-__device__ __forceinline__ int order_key(const Workspace &ws, int slot) {
-    const int *m = ws.meta + (size_t) slot * META_INTS;
-    return m[META_CKIND] ? m[META_K] : 0;
-}
-
-// Updates of `order` (descending keys) with a key above thr.
-__device__ int count_above(const Workspace &ws, int nup, int thr) {
-    int lo = 0, hi = nup;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (order_key(ws, ws.order[mid]) > thr) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // Doubles of the auxiliary arrays of an update of stack width k at the start of its team's shared memory.
 __device__ __forceinline__ int core_aux_doubles(const Workspace &ws, int slot) {
     const int k = ws.meta[(size_t) slot * META_INTS + META_K];
     return 6 * (k > 0 ? k : 1) + SVD_AUX_FIXED;
 }
 
-// CTA of SVD_THREADS threads, in one of two team layouts chosen by the update's stack width k: light
-// (kthr4 < k <= kthr) — two half-CTA teams of SVD_THREADS / 2 threads, one update each, each with half
+// CTA of SVD_THREADS threads, in one of three team layouts chosen by the update's stack width k: heavy (k > k_heavy:
+// the core needs more than half of the shared memory) — the whole CTA; light
+// (kthr4 < k <= k_heavy) — two half-CTA teams of SVD_THREADS / 2 threads, one update each, each with half
 // of the shared memory and its own named barrier; small (k <= kthr4: the core fits a quarter) — four teams
 // of SVD_THREADS / 4 threads.  Small cores are latency-bound (per-step barriers, dependent FP64 chains), so
 // four of them per SM hide each other's latency.  Wider updates are core_wide_kernel's.  With ws.order
-// (sorted by decreasing k) the classes are contiguous: after the H wide updates, the first ceil(L / 2)
-// CTAs take the L light updates in pairs; the rest take the small ones in fours.  Without an order
+// (sorted by decreasing k) the classes are contiguous: after the wide updates, a CTA takes a heavy one each, the
+// next ceil(L / 2) take the L light updates in pairs, the rest the small ones in fours.  Without an order
 // (one update per CTA) the team size follows the same class rule, so an update's arithmetic never
 // depends on the launch it is part of.
 template <int RPL>
-__global__ void __launch_bounds__(SVD_THREADS, 1) core_svd_kernel(const DevUpdate *ups, int nup, Workspace ws,
-                                                               Params p, int team_doubles, int kthr, int kthr4) {
+__device__ void core_svd_cta(const DevUpdate *ups, int nup, const Workspace &ws, const Params &p, int team_doubles, int kthr4) {
     extern __shared__ double smem_all[];
     __shared__ CoreShared s_sh[4];
-    __shared__ int s_wide, s_nlight;
-    if (threadIdx.x == 0) {
-        s_wide = ws.order ? count_above(ws, nup, kthr) : -1;
-        s_nlight = ws.order ? count_above(ws, nup, kthr4) - s_wide : 0;
-    }
+    __shared__ int s_end[3];  // first index behind the wide, heavy and light updates
+    if (threadIdx.x < 3)
+        s_end[threadIdx.x] = !ws.order ? 0 : (threadIdx.x == 0 ? ws.wide_updates(nup)
+                                                               : ws.count_above(nup, threadIdx.x == 1 ? ws.k_heavy : kthr4));
     __syncthreads();
-    const int H = s_wide, NL = s_nlight;
     constexpr int HALF = SVD_THREADS / 2, QUART = SVD_THREADS / 4;
-    const int quarter_doubles = team_doubles / 2;
-    int idx, part = 0;
-    bool light;
-    if (H < 0) {
+    int idx, part = 0, teams;
+    if (!ws.order) {
         idx = blockIdx.x;
         if (idx >= nup) return;
-        const int key = order_key(ws, idx);
-        if (key > kthr) return;
-        light = key > kthr4;
-        if (threadIdx.x >= (light ? HALF : QUART)) return;
+        const int key = ws.key(idx);
+        if (key > ws.k_heavy) return;  // single updates: heavy ones on a cluster
+        teams = key > kthr4 ? 2 : 4;
+        if ((int) threadIdx.x >= SVD_THREADS / teams) return;
     } else {
-        const int b = blockIdx.x, nlb = (NL + 1) / 2;
-        light = b < nlb;
-        if (light) {
-            part = threadIdx.x / HALF;
-            idx = H + 2 * b + part;
-            if (idx >= H + NL) return;  // the odd light update's partner slot stays idle
+        const int b = blockIdx.x, nh = s_end[1] - s_end[0], nl = s_end[2] - s_end[1], nlb = (nl + 1) / 2;
+        teams = b < nh ? 1 : (b < nh + nlb ? 2 : 4);
+        part = threadIdx.x / (SVD_THREADS / teams);
+        if (teams == 1) {
+            idx = s_end[0] + b;
+        } else if (teams == 2) {
+            idx = s_end[1] + 2 * (b - nh) + part;
+            if (idx >= s_end[2]) return;  // the odd light update's partner slot stays idle
         } else {
-            part = threadIdx.x / QUART;
-            idx = H + NL + 4 * (b - nlb) + part;
+            idx = s_end[2] + 4 * (b - nh - nlb) + part;
         }
     }
     if (idx >= nup) return;
-    const int slot = ws.heavy(idx), doubles = light ? team_doubles : quarter_doubles;
+    const int slot = ws.heavy(idx), doubles = 2 * team_doubles / teams;
     double *sm = smem_all + (size_t) part * doubles;
-    const int aux = core_aux_doubles(ws, slot);
-    if (light)
-        core_update<RPL>(Team<HALF>{(int) threadIdx.x % HALF, 1 + part}, ups, ws, p, slot, sm, sm + aux, doubles - aux,
-                         s_sh[part]);
+    const int aux = core_aux_doubles(ws, slot), tid = threadIdx.x % (SVD_THREADS / teams);
+    if (teams == 1)
+        core_update<RPL>(Team<SVD_THREADS>{tid, 1}, ups, ws, p, slot, sm, sm + aux, doubles - aux, s_sh[0]);
+    else if (teams == 2)
+        core_update<RPL>(Team<HALF>{tid, 1 + part}, ups, ws, p, slot, sm, sm + aux, doubles - aux, s_sh[part]);
     else
-        core_update<RPL>(Team<QUART>{(int) threadIdx.x % QUART, 1 + part}, ups, ws, p, slot, sm, sm + aux,
-                         doubles - aux, s_sh[part]);
+        core_update<RPL>(Team<QUART>{tid, 1 + part}, ups, ws, p, slot, sm, sm + aux, doubles - aux, s_sh[part]);
 }
 
-// The wide updates (k > kthr: the core does not fit half of an SM's shared memory): a cluster of WIDE_CTAS
+template <int RPL>
+__global__ void __launch_bounds__(SVD_THREADS, 1) core_svd_kernel(const DevUpdate *ups, int nup, Workspace ws,
+                                                               Params p, int team_doubles, int kthr4) {
+    core_svd_cta<RPL>(ups, nup, ws, p, team_doubles, kthr4);
+    wait_for_previous_launch();
+}
+
+// The wide updates (Workspace::wide_updates): a cluster of WIDE_CTAS
 // CTAs each, the matrices in global memory (L2), the auxiliary arrays and shared variables in the first
 // CTA's shared memory.  One SM's FP64 pipe took 35 ms for the Jacobi sweeps of a 200-column core and 180 ms for
 // a 340-column one, and a chain of such updates bounds a multiply, however few they are.
 template <int RPL>
 __global__ void __cluster_dims__(WIDE_CTAS, 1, 1) __launch_bounds__(SVD_THREADS, 1)
-    core_wide_kernel(const DevUpdate *ups, int nup, Workspace ws, Params p, int smem_doubles, int kthr) {
+    core_wide_kernel(const DevUpdate *ups, int nup, Workspace ws, Params p, int smem_doubles) {
     extern __shared__ double smem_all[];
     __shared__ CoreShared s_sh;
     __shared__ int s_wide;
+    let_next_launch_start();
     const int rank = cluster_rank();
     const ClusterTeam<SVD_THREADS, WIDE_CTAS> tm{rank * SVD_THREADS + (int) threadIdx.x, rank};
-    if (threadIdx.x == 0) s_wide = ws.order ? count_above(ws, nup, kthr) : nup;
+    if (threadIdx.x == 0) s_wide = ws.order ? ws.wide_updates(nup) : nup;
     __syncthreads();
     const int H = s_wide, ncl = gridDim.x / WIDE_CTAS;
     double *sm = cluster_map(smem_all, 0);
     CoreShared &sh = *cluster_map(&s_sh, 0);
     for (int h = blockIdx.x / WIDE_CTAS; h < H; h += ncl) {
         const int slot = ws.heavy(h);
-        if (order_key(ws, slot) <= kthr) continue;
+        if (ws.key(slot) <= ws.k_heavy) continue;
         const int aux = (core_aux_doubles(ws, slot) + 1) & ~1;
         tm.sync();  // the first CTA's shared memory is the previous update's no more (and exists)
         core_update<RPL>(tm, ups, ws, p, slot, sm, smem_all + aux, smem_doubles - aux, sh);
@@ -1499,7 +1562,7 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
     int rk = 0;
     double *XV = base + ws.off_xv;
     double up = 1.0;  // mixed form: Mw holds float-float values of M / up from here to step 3
-    const bool ff = !CLUSTER && p.mode == 1;  // wide cores are FP64 in every form
+    const bool ff = TM::nth < SVD_THREADS && p.mode == 1;  // heavy and wide cores are FP64 in every form
     if (ff) {
         // Exact power-of-two scaling that brings the largest entry of M near 1 (float range), then
         // the pivoted QR and the Jacobi sweeps in float-float arithmetic on the FP32 pipe.
@@ -1525,7 +1588,11 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         rk = qrcp_truncated_df(tm, Md, ldw, kU, kV, stop2f, (float) (rel * rel), reinterpret_cast<df *>(nrm),
                                reinterpret_cast<df *>(inv), pvt, reinterpret_cast<float *>(red), redi);
     } else if (spread) {
-        if constexpr (CLUSTER) rk = qrcp_cluster(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool);
+        if constexpr (CLUSTER) {  // lanes per column as in qrcp_truncated
+            rk = kU <= 64    ? qrcp_cluster<4>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool)
+                 : kU <= 256 ? qrcp_cluster<8>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool)
+                             : qrcp_cluster<16>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool);
+        }
     } else {
         rk = qrcp_truncated(tm, Mw, ldw, kU, kV, stop2, rel, nrm, inv, pvt, red, redi);
     }
@@ -1558,6 +1625,8 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         bool fits;
         if constexpr (CLUSTER) {
             b.ls4 = x4 + j4;
+            b.blocks = SWEEP_BLOCKS;
+            b.g8 = false;
             b.y = reinterpret_cast<float4 *>(base + ws.off_mixed);
             b.buf = reinterpret_cast<float4 *>(pool);
             b.buf_quads = pool_doubles / 2;
@@ -1568,6 +1637,8 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
             fits = 4 * (size_t) b.ls4 * rk <= (size_t) ws.kmax * (ws.kmax + ws.ld) && 2 * b.ls4 <= b.buf_quads;
         } else {
             b.ls4 = ((x4 + j4 + 3) & ~7) + 4;  // 4 mod 8 quads: two 4-lane groups a quarter-warp, no bank conflicts
+            b.blocks = k > LIGHT_K ? SWEEP_BLOCKS : 0;
+            b.g8 = rk <= (k <= SMALL_K ? 32 : 64);
             const int skip = (int) ((reinterpret_cast<uintptr_t>(pool) >> 3) & 1);
             b.y = reinterpret_cast<float4 *>(pool + skip);
             b.buf = nullptr;
@@ -1580,6 +1651,20 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         }
         b.e64 = base + ws.off_m;
         b.w = base + ws.off_mixed;
+        if constexpr (!CLUSTER) {
+            // E, W and V in shared memory behind y / wh, as far as they fit
+            const long ly = 2L * b.ls4 * rk + 1, lh = (long) b.ldh * rk;
+            long top = ly > lh ? ly : lh;
+            auto place = [&](long doubles) -> double * {
+                if (top + doubles > (long) pool_doubles) return nullptr;
+                double *at = pool + top;
+                top += doubles;
+                return at;
+            };
+            if (double *at = place((long) rk * rk)) b.e64 = at;
+            if (double *at = place((long) kV * rk)) b.w = at;
+            if (double *at = place(((long) rk * rk + 1) / 2)) b.v = reinterpret_cast<float *>(at);
+        }
         if (fits && jacobi_precond(tm, XV, ld, kV, rk, b, reinterpret_cast<df *>(nrm), perm, &s_rot, &s_emax,
                                    &sh.cosine, &sh.tangent, (float) tol64, &sweeps, &converged)) {
             Xs = b.w;
@@ -1720,25 +1805,39 @@ size_t svd_smem_bytes(int kmax) { return 2 * sizeof(double) * (size_t) svd_team_
 // Register tiles of the FP64 sweeps: up to 16 rows a lane (longer columns take the looped sweep).
 constexpr int CORE_RPL = 16;
 
+// A core of k columns takes its aux arrays, 6 k + SVD_AUX_FIXED doubles, and a k x k working copy.  A 110-column core
+// of width 128 takes a cluster of eight 4,300 kcycles and one SM alone 7,900: heavy ones go to clusters only
+// while SMs are idle, wide ones always.
+void core_classes(int kmax, int *whole, int *half, int *quarter) {
+    const int team = svd_team_doubles(kmax);
+    auto widest = [](long doubles) {
+        int k = 0;
+        while ((k + 1L) * (k + 1L) + 6 * (k + 1L) + SVD_AUX_FIXED <= doubles) k++;
+        return k;
+    };
+    *whole = widest(2 * team);
+    *half = widest(team);
+    *quarter = widest(team / 2);
+}
+
+static void launch_core_wide(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {
+    const int aux = 6 * ws.kmax + SVD_AUX_FIXED + 1;
+    const int doubles = std::min(aux + WIDE_POOL_DOUBLES, 2 * svd_team_doubles(ws.kmax));
+    const size_t bytes = sizeof(double) * (size_t) doubles;
+    cudaFuncSetAttribute(core_wide_kernel<CORE_RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
+    const int ctas = std::min(n, WIDE_CLUSTERS) * WIDE_CTAS;
+    { core_wide_kernel<CORE_RPL><<<ctas, SVD_THREADS, bytes, st>>>(ups, n, ws, p, doubles); note_launch(); }
+}
+
 void launch_core_svd(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {
     const int team = svd_team_doubles(ws.kmax);
     const size_t smem = 2 * sizeof(double) * (size_t) team;
-    // Wide: a core of k columns (its aux arrays, 6 k + SVD_AUX_FIXED doubles, and a k x k working
-    // copy) does not fit the half-CTA team's shared memory; small: it fits a quarter-CTA team's.
-    auto fits = [](long k, long doubles) { return k * k + 6 * k + SVD_AUX_FIXED <= doubles; };
-    int kthr = 0, kthr4 = 0;
-    while (fits(kthr + 1, team)) kthr++;
-    while (fits(kthr4 + 1, team / 2)) kthr4++;
-    if (ws.kmax > kthr) {
-        const int aux = 6 * ws.kmax + SVD_AUX_FIXED + 1;
-        const int doubles = std::min(aux + WIDE_POOL_DOUBLES, 2 * team);
-        const size_t bytes = sizeof(double) * (size_t) doubles;
-        cudaFuncSetAttribute(core_wide_kernel<CORE_RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
-        const int ctas = std::min(n, WIDE_CLUSTERS) * WIDE_CTAS;
-        { core_wide_kernel<CORE_RPL><<<ctas, SVD_THREADS, bytes, st>>>(ups, n, ws, p, doubles, kthr); note_launch(); }
-    }
+    int whole, half, quarter;
+    core_classes(ws.kmax, &whole, &half, &quarter);
     cudaFuncSetAttribute(core_svd_kernel<CORE_RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    { core_svd_kernel<CORE_RPL><<<n, SVD_THREADS, smem, st>>>(ups, n, ws, p, team, kthr, kthr4); note_launch(); }
+    const bool wide = ws.kmax > ws.k_heavy;
+    if (wide) launch_core_wide(ups, n, ws, p, st);
+    launch_beside(wide, 1, n, SVD_THREADS, smem, st, core_svd_kernel<CORE_RPL>, ups, n, ws, p, team, quarter);
 }
 
 }  // namespace hcgb
