@@ -159,6 +159,21 @@ __device__ __forceinline__ double job_b(const GemmJob &jb, int k, int j) {
 // Precision of the factor products and of the WY Q-application products in arithmetic form `mode`.
 __host__ __device__ inline int lowp_prec(int mode) { return mode == HCGB_TF32 ? 1 : (mode == HCGB_BF16 ? 2 : 0); }
 
+// The job whose tile w is (sched: exclusive prefix sums of the jobs' tiles, njobs + 1 entries): a 32-way search by
+// the whole warp, two or three dependent loads.
+__device__ __forceinline__ int job_of_tile(const int *sched, int njobs, int w) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, n = njobs;  // sched[lo] <= w < sched[lo + n]
+    while (n > 1) {
+        const int step = (n + 31) >> 5, at = (lane + 1) * step;
+        const unsigned below = __ballot_sync(0xffffffffu, at < n && sched[lo + at] <= w);
+        const int skip = __popc(below) * step;
+        lo += skip;
+        n = n - skip < step ? n - skip : step;
+    }
+    return lo;
+}
+
 // Products worth the split (enough k to amortise the 4 FP64 instructions per output, enough outputs
 // for a tile).
 constexpr int OZ_MIN_OUTPUTS = 2048;

@@ -202,13 +202,16 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     if (tid < OZ_TM) ea[tid] = 0;
     else if (tid < OZ_TM + OZ_TN) eb[tid - OZ_TM] = 0;
     __syncthreads();
-    auto exponents = [&](auto is_a, int count, int groups, int *out) {
+    auto exponents = [&](auto is_a, int count, int *out) {
         constexpr bool IS_A = decltype(is_a)::value;
         const bool kfast = IS_A ? jb.opA != 0 : jb.opB == 0;
+        int groups = 16;  // few rows: more threads each
+        while (groups < count) groups <<= 1;
         const int per = OZ_THREADS / groups;
         const int g = kfast ? tid / per : tid % groups, part = kfast ? tid % per : tid / groups;
         if (g >= count) return;
         int top = 0;
+#pragma unroll 4
         for (int k = 4 * part; k < jb.K; k += 4 * per) {
             double v[4];
             load_run<IS_A, 4>(jb, (IS_A ? m0 : n0) + g, k, v);
@@ -217,8 +220,8 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
         }
         if (top) atomicMax(out + g, top);
     };
-    exponents(std::true_type{}, rows, OZ_TM, ea);
-    exponents(std::false_type{}, cols, OZ_TN, eb);
+    exponents(std::true_type{}, rows, ea);
+    exponents(std::false_type{}, cols, eb);
     __syncthreads();
     if (tid < OZ_TM) ea[tid] = ea[tid] ? ea[tid] - 1022 : OZ_NOGROUP;
     else if (tid < OZ_TM + OZ_TN) eb[tid - OZ_TM] = eb[tid - OZ_TM] ? eb[tid - OZ_TM] - 1022 : OZ_NOGROUP;
@@ -271,12 +274,15 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     const int ra = ka ? tid >> 2 : tid & 127, ca = ka ? tid & 3 : tid >> 7;
     const int rb = (tid & 7) + 8 * (tid >> 6), cb = ((tid >> 4) & 3) * 8 + ((tid >> 3) & 1) * 4;
     const int nchunks = (jb.K + OZ_KC - 1) / OZ_KC;
+    double va[8], vb[4];  // the next chunk's runs, loaded while this one's products are issued and read out
+    auto load = [&](int c) {
+        if (ra < rows) load_run<true, 8>(jb, m0 + ra, c * OZ_KC + 8 * ca, va);
+        if (rb < cols) load_run<false, 4>(jb, n0 + rb, c * OZ_KC + cb, vb);
+    };
+    if (nchunks > 0) load(0);
     for (int c = 0; c < nchunks; c++) {
-        const int buf = c & 1, k0 = c * OZ_KC;
+        const int buf = c & 1;
         unsigned char *sa = stage0 + buf * OZ_STAGE, *sb = sa + OZ_S * OZ_A_PLANE;
-        double va[8], vb[4];
-        if (ra < rows) load_run<true, 8>(jb, m0 + ra, k0 + 8 * ca, va);
-        if (rb < cols) load_run<false, 4>(jb, n0 + rb, k0 + cb, vb);
         if (pending[buf]) {  // the MMAs of chunk c - 2 have read this stage
             ok &= tc::mbar_wait(mbar0 + 8 * buf, phase[buf]);
             phase[buf] ^= 1;
@@ -284,6 +290,7 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
         }
         if (ra < rows) split_run<8>(va, ea[ra], sa + oz_off(ra, 8 * ca), OZ_A_PLANE);
         if (rb < cols) split_run<4>(vb, eb[rb], sb + oz_off(rb, cb), OZ_B_PLANE);
+        if (c + 1 < nchunks) load(c + 1);
         tc::fence_smem_to_async();
         __syncthreads();
         if (tid == OZ_THREADS - 32) {
@@ -360,12 +367,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_jobs_kernel(const GemmJ
     uint32_t phase[2] = {0u, 0u};
     bool pending[2] = {false, false};
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
-        int lo = 0, hi = njobs;  // sched[lo] <= w < sched[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (sched[mid] <= w) lo = mid;
-            else hi = mid;
-        }
+        const int lo = job_of_tile(sched, njobs, w);
         const GemmJob jb = jobs[lo];
         oz_tile(jb, w - sched[lo], stage0, tmem, mbar0, phase, pending, ea, eb);
     }

@@ -166,32 +166,34 @@ __device__ void plan_update(const DevUpdate *ups, int n, double alpha, double be
 }
 
 // dst[j + i*ldd] = scale * src[i + j*lds] for i < rows(src), j < cols(src): a transposed copy
-// through a 32x33 shared tile so that both sides stay coalesced.
+// through a 32x33 shared tile so that both sides stay coalesced; tile `part` of every `parts`.
 __device__ void transpose_scaled(const double *src, int lds, int rows, int cols, double *dst, int ldd,
-                                 double scale, double (*tile)[33]) {
+                                 double scale, double (*tile)[33], int part, int parts) {
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, nty = blockDim.x >> 5;
-    for (int i0 = 0; i0 < rows; i0 += 32)
-        for (int j0 = 0; j0 < cols; j0 += 32) {
-            for (int jj = ty; jj < 32; jj += nty) {
-                int i = i0 + tx, j = j0 + jj;
-                tile[jj][tx] = (i < rows && j < cols) ? src[i + (size_t) j * lds] : 0.0;
-            }
-            __syncthreads();
-            for (int ii = ty; ii < 32; ii += nty) {
-                int i = i0 + ii, j = j0 + tx;
-                if (i < rows && j < cols) dst[j + (size_t) i * ldd] = scale * tile[tx][ii];
-            }
-            __syncthreads();
+    const int nti = (rows + 31) / 32, ntj = (cols + 31) / 32;
+    for (int t = part; t < nti * ntj; t += parts) {
+        const int i0 = t % nti * 32, j0 = t / nti * 32;
+        for (int jj = ty; jj < 32; jj += nty) {
+            int i = i0 + tx, j = j0 + jj;
+            tile[jj][tx] = (i < rows && j < cols) ? src[i + (size_t) j * lds] : 0.0;
         }
+        __syncthreads();
+        for (int ii = ty; ii < 32; ii += nty) {
+            int i = i0 + ii, j = j0 + tx;
+            if (i < rows && j < cols) dst[j + (size_t) i * ldd] = scale * tile[tx][ii];
+        }
+        __syncthreads();
+    }
 }
 
-__device__ void copy_scaled(const double *src, int lds, int rows, int cols, double *dst, int ldd, double scale) {
-    for (int j = 0; j < cols; j++)
+__device__ void copy_scaled(const double *src, int lds, int rows, int cols, double *dst, int ldd, double scale, int part,
+                            int parts) {
+    for (int j = part; j < cols; j += parts)
         for (int i = threadIdx.x; i < rows; i += blockDim.x)
             dst[i + (size_t) j * ldd] = scale * src[i + (size_t) j * lds];
 }
 
-// One CTA per update: the parts of the stacks that are copies of existing factors
+// gridDim.y CTAs per update: the parts of the stacks that are copies of existing factors
 // (LaCpy + MultiplyByAlpha + ProcessVpointer, Compressed.cpp:331-379).
 __global__ void __launch_bounds__(256) stack_kernel(const DevUpdate *ups, double alpha, double beta, Workspace ws) {
     __shared__ double tile[32][33];
@@ -206,15 +208,16 @@ __global__ void __launch_bounds__(256) stack_kernel(const DevUpdate *ups, double
     double *Vs = slot + ws.off_vstack;
     const int ld = ws.ld;
     const double *Cu = u.c.data, *Cv = u.c.v;
-    copy_scaled(Cu, m, m, rC, Us, ld, 1.0);                                      // U[:, :rC] = Cu
-    if (side == 0 && u.a.kind) copy_scaled(u.a.data, m, m, rA, Us + (size_t) rC * ld, ld, alpha);  // alpha Au
+    const int part = blockIdx.y, parts = gridDim.y;
+    copy_scaled(Cu, m, m, rC, Us, ld, 1.0, part, parts);                                      // U[:, :rC] = Cu
+    if (side == 0 && u.a.kind) copy_scaled(u.a.data, m, m, rA, Us + (size_t) rC * ld, ld, alpha, part, parts);  // alpha Au
     // V[:, :rC] = beta Cv^T; a compressed_vt C stores Cv^T itself (ProcessVpointer's Cholesky copy)
-    if (u.c.kind == HCGB_COMPRESSED_VT) copy_scaled(Cv, nn, nn, rC, Vs, ld, beta);
-    else transpose_scaled(Cv, rC, rC, nn, Vs, ld, beta, tile);
+    if (u.c.kind == HCGB_COMPRESSED_VT) copy_scaled(Cv, nn, nn, rC, Vs, ld, beta, part, parts);
+    else transpose_scaled(Cv, rC, rC, nn, Vs, ld, beta, tile, part, parts);
     if (side == 1 && u.b.kind) {
         const double *Bv = u.b.v;
-        if (u.b.kind == HCGB_COMPRESSED_VT) copy_scaled(Bv, nn, nn, rB, Vs + (size_t) rC * ld, ld, 1.0);
-        else transpose_scaled(Bv, rB, rB, nn, Vs + (size_t) rC * ld, ld, 1.0, tile);  // V[:, rC:] = Bv^T
+        if (u.b.kind == HCGB_COMPRESSED_VT) copy_scaled(Bv, nn, nn, rB, Vs + (size_t) rC * ld, ld, 1.0, part, parts);
+        else transpose_scaled(Bv, rB, rB, nn, Vs + (size_t) rC * ld, ld, 1.0, tile, part, parts);  // V[:, rC:] = Bv^T
     }
 }
 
@@ -314,12 +317,7 @@ __global__ void __launch_bounds__(128) gemm_jobs_kernel(const GemmJob *jobs, int
     __shared__ double Bs[GK][BS_LD];
     const int total = sched[njobs];
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
-        int lo = 0, hi = njobs;  // sched[lo] <= w < sched[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (sched[mid] <= w) lo = mid;
-            else hi = mid;
-        }
+        const int lo = job_of_tile(sched, njobs, w);
         const GemmJob jb = jobs[lo];
         gemm_tile(jb, w - sched[lo], As, Bs);
         __syncthreads();
@@ -370,14 +368,14 @@ __global__ void __launch_bounds__(1024) schedule_kernel(const GemmJob *jobs, int
         for (int l = 0; l < NL; l++) sched[l * (njobs + 1) + njobs] = part[l][1023];
 }
 
-// One CTA per update: V (r x n, ld r) = XV^T into the tile buffer, publish rank and record.
+// gridDim.y CTAs per update: V (r x n, ld r) = XV^T into the tile buffer, publish rank and record.
 __global__ void __launch_bounds__(256) finalize_kernel(const DevUpdate *ups, Workspace ws, hcgb_update_info *info) {
     __shared__ double tile[32][33];
     const int s = blockIdx.x;
     const int *meta = ws.meta + (size_t) s * META_INTS;
     const int status = meta[META_STATUS];
     const bool ok = (status == HCGB_OK || status == HCGB_NOT_CONVERGED) && meta[META_CKIND];
-    if (info && threadIdx.x == 0) {
+    if (info && threadIdx.x == 0 && blockIdx.y == 0) {
         hcgb_update_info r;
         r.status = status;
         r.rank_a = meta[META_RA];
@@ -398,9 +396,9 @@ __global__ void __launch_bounds__(256) finalize_kernel(const DevUpdate *ups, Wor
     const int r = meta[META_NEWRANK], nn = meta[META_N];
     const double *XV = ws.slot(s) + ws.off_xv;
     double *Cv = u.c.v;
-    if (u.c.kind == HCGB_COMPRESSED_VT) copy_scaled(XV, ws.ld, nn, r, Cv, nn, 1.0);  // W = XV (n x r, ld n)
-    else transpose_scaled(XV, ws.ld, nn, r, Cv, r, 1.0, tile);
-    if (threadIdx.x == 0) *u.c.rank = r;
+    if (u.c.kind == HCGB_COMPRESSED_VT) copy_scaled(XV, ws.ld, nn, r, Cv, nn, 1.0, blockIdx.y, gridDim.y);  // W = XV (n x r, ld n)
+    else transpose_scaled(XV, ws.ld, nn, r, Cv, r, 1.0, tile, blockIdx.y, gridDim.y);
+    if (threadIdx.x == 0 && blockIdx.y == 0) *u.c.rank = r;
 }
 
 // DDC: W = alpha A B + beta Cu Cv sits in the tmp2 region (ld ws.ld); C <- [U = W | V = I].
@@ -438,7 +436,7 @@ __global__ void __launch_bounds__(1024) order_kernel(int n, Workspace ws) {
 __global__ void __launch_bounds__(256) transpose_kernel(const double *src, int lds, int rows, int cols, double *dst,
                                                       int ldd) {
     __shared__ double tile[32][33];
-    transpose_scaled(src, lds, rows, cols, dst, ldd, 1.0, tile);
+    transpose_scaled(src, lds, rows, cols, dst, ldd, 1.0, tile, blockIdx.x, gridDim.x);
 }
 
 // One thread per update: the six jobs of the WY application of both Q factors (after the core).
@@ -508,7 +506,9 @@ __global__ void __launch_bounds__(256) wy_solve_kernel(Workspace ws) {
     const double *G = base + (side ? ws.off_mcopy : ws.off_m);
     const double *tau = base + (side ? ws.off_tauv : ws.off_tauu);
     const int lk = ws.kmax;
-    const int share = (r + gridDim.y - 1) / gridDim.y, c0 = blockIdx.y * share;
+    int share = (r + gridDim.y - 1) / gridDim.y;
+    if (share < 8) share = 8;
+    const int c0 = blockIdx.y * share;
     const int nc = r - c0 < share ? r - c0 : share;
     if (nc <= 0) return;
     double *W = base + ws.off_w + (size_t) side * lk * lk + (size_t) c0 * lk;
@@ -576,15 +576,16 @@ void launch_plan_wy(const DevUpdate *ups, int n, Workspace ws, Params p, GemmJob
 }
 
 void launch_wy_solve(int n, Workspace ws, cudaStream_t st) {
-    // As many CTAs a side as leave no SM idle (up to one per eight columns): a side's solve on one SM took 3 ms at
-    // 340 reflectors and 170 columns.
+    // As many CTAs a side as leave no SM idle (up to one per eight columns), four at least: a side's solve on one SM
+    // took 3 ms at 340 reflectors and 170 columns.
     const int sms = device_sms(), cols = (ws.kmax + 7) / 8;
-    const int split = std::max(1, std::min(cols, 2 * sms / (2 * n * ws.conc)));
+    const int split = std::min(cols, std::max(4, 2 * sms / (2 * n * ws.conc)));
     { wy_solve_kernel<<<dim3(2 * n, split), 256, 0, st>>>(ws); note_launch(); }
 }
 
 void launch_transpose(const double *src, int lds, int rows, int cols, double *dst, int ldd, cudaStream_t st) {
-    { transpose_kernel<<<1, 256, 0, st>>>(src, lds, rows, cols, dst, ldd); note_launch(); }
+    const int tiles = ((rows + 31) / 32) * ((cols + 31) / 32);
+    { transpose_kernel<<<std::max(1, std::min(tiles, 1024)), 256, 0, st>>>(src, lds, rows, cols, dst, ldd); note_launch(); }
 }
 
 void launch_plan(const DevUpdate *ups, int n, double alpha, double beta, Workspace ws, Params p, GemmJob *jobs,
@@ -601,12 +602,16 @@ void launch_gather_ranks(const int *const *ptrs, int n, int *out, cudaStream_t s
     if (n > 0) { gather_ranks_kernel<<<(n + 255) / 256, 256, 0, st>>>(ptrs, n, out); note_launch(); }
 }
 
+// CTAs per update of the copying kernels: one per update took 330 us for the stacks of 256 updates, the widest of
+// them 200 columns of 512 rows.
+static int copy_split(int n) { return n >= 512 ? 4 : (n >= 64 ? 8 : 16); }
+
 void launch_order(int n, Workspace ws, cudaStream_t st) {
     { order_kernel<<<1, 1024, 0, st>>>(n, ws); note_launch(); }
 }
 
 void launch_stack(const DevUpdate *ups, int n, double alpha, double beta, Workspace ws, cudaStream_t st) {
-    { stack_kernel<<<n, 256, 0, st>>>(ups, alpha, beta, ws); note_launch(); }
+    { stack_kernel<<<dim3(n, copy_split(n)), 256, 0, st>>>(ups, alpha, beta, ws); note_launch(); }
 }
 
 void launch_gemm_jobs(const GemmJob *jobs, int njobs, int *sched, cudaStream_t st, bool has_lowp) {
@@ -621,7 +626,7 @@ void launch_gemm_jobs(const GemmJob *jobs, int njobs, int *sched, cudaStream_t s
 }
 
 void launch_finalize(const DevUpdate *ups, int n, Workspace ws, hcgb_update_info *info, cudaStream_t st) {
-    { finalize_kernel<<<n, 256, 0, st>>>(ups, ws, info); note_launch(); }
+    { finalize_kernel<<<dim3(n, copy_split(n)), 256, 0, st>>>(ups, ws, info); note_launch(); }
 }
 
 void launch_ddc_finalize(const DevUpdate *ups, int n, Workspace ws, cudaStream_t st) {

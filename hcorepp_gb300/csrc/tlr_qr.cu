@@ -152,13 +152,11 @@ __device__ void factor_panel_df(const TM &tm, df *Ps, int ldp, int mr, int nbp, 
     }
 }
 
-// Overwrite the panel with the explicit unit-lower V (zeros above the diagonal, zero padding).
+// Overwrite the panel with the explicit unit-lower V (its columns beyond nbp are zero already).
 __device__ void make_explicit_v(double *Ps, int ldp, int nbp) {
-    for (int e = threadIdx.x; e < NB * ldp; e += blockDim.x) {
-        const int c = e / ldp, r = e % ldp;
-        if (c >= nbp) Ps[e] = 0.0;
-        else if (r < c) Ps[e] = 0.0;
-        else if (r == c) Ps[e] = 1.0;
+    for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
+        const int c = e / NB, r = e % NB;
+        if (c < nbp && r <= c) Ps[r + (size_t) c * ldp] = r == c ? 1.0 : 0.0;
     }
 }
 
@@ -326,19 +324,19 @@ __device__ void qr_side(const Workspace &ws, int slot, int side, int part, doubl
     for (int j0 = 0; j0 < kk; j0 += NB) {
         const int nbp = (kk - j0) < NB ? (kk - j0) : NB;
         const int mr = m - j0;
-        for (int e = threadIdx.x; e < NB * s.ldp; e += blockDim.x) {
-            const int c = e / s.ldp, r = e % s.ldp;
-            s.Ps[e] = (c < nbp && r < mr) ? A[(j0 + r) + (size_t) (j0 + c) * lda] : 0.0;
-        }
+        for (int c = threadIdx.x >> 5; c < NB; c += QR_THREADS / 32)
+#pragma unroll 4
+            for (int r = threadIdx.x & 31; r < s.ldp; r += 32)
+                s.Ps[r + (size_t) c * s.ldp] = (c < nbp && r < mr) ? A[(j0 + r) + (size_t) (j0 + c) * lda] : 0.0;
         __syncthreads();
         if (C > 1) cluster_arrive();  // this CTA has read the panel
         const bool any = factor_panel(s.Ps, s.ldp, mr, nbp, s.tau, s.red);
         if (C > 1) cluster_wait();    // so has every other: it may be written
         if (part == 0) {
-            for (int e = threadIdx.x; e < nbp * mr; e += blockDim.x) {
-                const int c = e / mr, r = e % mr;
-                A[(j0 + r) + (size_t) (j0 + c) * lda] = s.Ps[(size_t) c * s.ldp + r];
-            }
+            for (int c = threadIdx.x >> 5; c < nbp; c += QR_THREADS / 32)
+#pragma unroll 4
+                for (int r = threadIdx.x & 31; r < mr; r += 32)
+                    A[(j0 + r) + (size_t) (j0 + c) * lda] = s.Ps[(size_t) c * s.ldp + r];
             if (threadIdx.x < nbp) tau[j0 + threadIdx.x] = s.tau[threadIdx.x];
         }
         __syncthreads();
@@ -600,12 +598,13 @@ __global__ void __launch_bounds__(QR_THREADS) apply_q_kernel(const DevUpdate *up
         const int j0 = p * NB;
         const int nbp = (kk - j0) < NB ? (kk - j0) : NB;
         const int mr = m - j0;
-        for (int e = threadIdx.x; e < NB * s.ldp; e += blockDim.x) {
-            const int c = e / s.ldp, rr = e % s.ldp;
-            double v = 0.0;
-            if (c < nbp && rr < mr) v = rr > c ? A[(j0 + rr) + (size_t) (j0 + c) * lda] : (rr == c ? 1.0 : 0.0);
-            s.Ps[e] = v;
-        }
+        for (int c = threadIdx.x >> 5; c < NB; c += QR_THREADS / 32)
+#pragma unroll 4
+            for (int rr = threadIdx.x & 31; rr < s.ldp; rr += 32) {
+                double v = 0.0;
+                if (c < nbp && rr < mr) v = rr > c ? A[(j0 + rr) + (size_t) (j0 + c) * lda] : (rr == c ? 1.0 : 0.0);
+                s.Ps[rr + (size_t) c * s.ldp] = v;
+            }
         for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) s.Ts[e] = Tg[(size_t) p * NB * NB + e];
         __syncthreads();
         apply_block_reflector(s.Ps, s.ldp, s.Ts, false, X + j0, ldx, mr, r, s.Ws, s.ldw);

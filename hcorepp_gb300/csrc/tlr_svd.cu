@@ -28,7 +28,8 @@ namespace hcgb {
 namespace {
 
 constexpr int SVD_THREADS = 512;
-constexpr int WIDE_POOL_DOUBLES = 16640;  // shared memory of a CTA for a pair of column blocks (130 KB)
+constexpr int WIDE_POOL_DOUBLES = 16640;  // shared memory of a CTA: 130 KB leave the rest to L1 ...
+constexpr int WIDE_POOL_K = 350;          // ... up to the width whose columns they hold
 constexpr float PRECOND_TOL32 = 1e-6f;  // above the rounding of a single-precision cosine
 constexpr int PRECOND_MAX_SWEEPS = 12;
 constexpr int SVD_RED_DOUBLES = 64, SVD_REDI_INTS = 128;  // reduction area (up to 32 warps)
@@ -346,10 +347,28 @@ __device__ void jacobi_dispatch(const TM &tm, double *X, int ldx, int rows, int 
 // leaves the rest to the FP64 sweeps.
 // ---------------------------------------------------------------------------------------------
 
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Tangent of the rotation angle, zeta = (b - a) / (2 c) (Rutishauser; zeta^2 must not overflow).
 __device__ __forceinline__ float rotation_tangent(float zeta) {
     if (fabsf(zeta) > 1.0e18f) return 0.5f / zeta;
     return copysignf(1.f, zeta) / (fabsf(zeta) + sqrtf(fmaf(zeta, zeta, 1.f)));
+}
+
+// Cosine and sine of the single-precision sweeps.  The chain of two divisions and two square roots was half of a
+// step's latency; approximations do (any tangent gives a rotation), but the cosine gets a Newton step: its
+// error makes the accumulated J32 less orthogonal.
+__device__ __forceinline__ void rotation32(float a, float b, float c, float &cs, float &sn) {
+    const float zeta = __fdividef(b - a, 2.f * c), z = fabsf(zeta);
+    float t = z > 1.0e18f ? __fdividef(0.5f, z) : __fdividef(1.f, z + sqrt_approx(fmaf(z, z, 1.f)));
+    t = copysignf(t, zeta);
+    const float q = fmaf(t, t, 1.f), r = rsqrtf(q);
+    cs = fmaf(0.5f * r, fmaf(-q * r, r, 1.f), r);
+    sn = cs * t;
 }
 
 // Pair `pp` of step t over columns [0, nc_a) and [off_b, off_b + nc_b): round robin over all of them (cross =
@@ -392,9 +411,8 @@ __device__ __forceinline__ int jacobi32_rotate(bool act, float4 *x, float4 *y, i
         c += __shfl_xor_sync(0xffffffffu, c, o);
     }
     if (!(act && a > 0.f && b > 0.f && fabsf(c) * rsqrtf(a) * rsqrtf(b) > tol)) return 0;
-    const float zeta = (b - a) / (2.f * c);
-    const float tt = rotation_tangent(zeta);
-    const float cs = 1.f / sqrtf(fmaf(tt, tt, 1.f)), sn = cs * tt;
+    float cs, sn;
+    rotation32(a, b, c, cs, sn);
 #pragma unroll 4
     for (int r = gl; r < x4 + j4; r += G) {
         const float4 u = x[r], v = y[r];
@@ -467,35 +485,63 @@ __device__ int jacobi32_block_pair(const TM &tm, float4 *Y, int ls4, int x4, int
     return rotations;
 }
 
-// 16 x 8 output tiles of an M x N result, one warp each: lane (li, lj) accumulates rows i0 + li, i0 + li + 8
-// and columns j0 + lj, j0 + lj + 4 over k = 0 .. K - 1.  mac(acc, i, j0.., k) is given the operands by fa / fb
-// (indices clamped into range); fo stores what lies inside.  keep(i0, j0) skips whole tiles.
+// 8 R x 4 R output tiles of an M x N result, one warp each: lane (li, lj) accumulates rows i0 + li + 8 u and columns
+// j0 + lj + 4 v, u, v < R, over k = 0 .. K - 1 (indices clamped into range for the loads; fo stores what lies
+// inside).  keep(i0, j0, rows, cols) skips whole tiles.
+template <int R, class TM, class FA, class FB, class FM, class FI, class FO, class FK>
+__device__ __forceinline__ void warp_tiles_r(const TM &tm, int M, int N, int K, FA fa, FB fb, FM mac, FI init, FO fo,
+                                             FK keep) {
+    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
+    const int li = lane & 7, lj = lane >> 3;
+    constexpr int TI = 8 * R, TJ = 4 * R;
+    const int nti = (M + TI - 1) / TI, ntj = (N + TJ - 1) / TJ;
+    for (int idx = warp; idx < nti * ntj; idx += nw) {
+        const int i0 = (idx % nti) * TI, j0 = (idx / nti) * TJ;
+        if (!keep(i0, j0, TI, TJ)) continue;
+        int ii[R], jj[R];
+        df_acc acc[R][R];
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            ii[u] = i0 + li + 8 * u < M ? i0 + li + 8 * u : M - 1;
+            jj[u] = j0 + lj + 4 * u < N ? j0 + lj + 4 * u : N - 1;
+        }
+#pragma unroll
+        for (int u = 0; u < R; u++)
+#pragma unroll
+            for (int v = 0; v < R; v++) acc[u][v] = init(ii[u], jj[v]);
+#pragma unroll(R == 2 ? 2 : 1)
+        for (int k = 0; k < K; k++) {
+            decltype(fa(0, 0)) a[R];
+            decltype(fb(0, 0)) b[R];
+#pragma unroll
+            for (int u = 0; u < R; u++) {
+                a[u] = fa(ii[u], k);
+                b[u] = fb(k, jj[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < R; u++)
+#pragma unroll
+                for (int v = 0; v < R; v++) mac(acc[u][v], a[u], b[v]);
+        }
+#pragma unroll
+        for (int u = 0; u < R; u++)
+#pragma unroll
+            for (int v = 0; v < R; v++)
+                if (i0 + li + 8 * u < M && j0 + lj + 4 * v < N) fo(ii[u], jj[v], acc[u][v]);
+    }
+}
+
+// R = 2, or 4 on a cluster whose warps all get such a tile (half the loads per product: on a cluster the operands come
+// through L1, 8 bytes a lane).  An element's arithmetic does not depend on R.
 template <class TM, class FA, class FB, class FM, class FI, class FO, class FK>
 __device__ __forceinline__ void warp_tiles(const TM &tm, int M, int N, int K, FA fa, FB fb, FM mac, FI init, FO fo,
                                            FK keep) {
-    const int warp = tm.warp(), lane = threadIdx.x & 31, nw = tm.nw();
-    const int li = lane & 7, lj = lane >> 3;
-    const int nti = (M + 15) >> 4, ntj = (N + 7) >> 3;
-    for (int idx = warp; idx < nti * ntj; idx += nw) {
-        const int i0 = (idx % nti) * 16, j0 = (idx / nti) * 8;
-        if (!keep(i0, j0)) continue;
-        const int ia = i0 + li < M ? i0 + li : M - 1, ib = i0 + li + 8 < M ? i0 + li + 8 : M - 1;
-        const int ja = j0 + lj < N ? j0 + lj : N - 1, jb = j0 + lj + 4 < N ? j0 + lj + 4 : N - 1;
-        df_acc c00 = init(ia, ja), c01 = init(ia, jb), c10 = init(ib, ja), c11 = init(ib, jb);
-#pragma unroll 2
-        for (int k = 0; k < K; k++) {
-            const auto a0 = fa(ia, k), a1 = fa(ib, k);
-            const auto b0 = fb(k, ja), b1 = fb(k, jb);
-            mac(c00, a0, b0);
-            mac(c01, a0, b1);
-            mac(c10, a1, b0);
-            mac(c11, a1, b1);
+    if constexpr (TM::ctas > 1)
+        if ((long) ((M + 31) / 32) * ((N + 15) / 16) >= TM::nw()) {
+            warp_tiles_r<4>(tm, M, N, K, fa, fb, mac, init, fo, keep);
+            return;
         }
-        if (i0 + li < M && j0 + lj < N) fo(i0 + li, j0 + lj, c00);
-        if (i0 + li < M && j0 + lj + 4 < N) fo(i0 + li, j0 + lj + 4, c01);
-        if (i0 + li + 8 < M && j0 + lj < N) fo(i0 + li + 8, j0 + lj, c10);
-        if (i0 + li + 8 < M && j0 + lj + 4 < N) fo(i0 + li + 8, j0 + lj + 4, c11);
-    }
+    warp_tiles_r<2>(tm, M, N, K, fa, fb, mac, init, fo, keep);
 }
 
 // acc += a b for floats, exactly (Ogita, Rump and Oishi's Dot2).
@@ -515,7 +561,7 @@ __device__ void ns_gram(const TM &tm, const float *J, int ldj, int rk, df *E) {
         [&](int k, int j) { return J[k + (size_t) j * ldj]; },
         [](df_acc &c, float a, float b) { acc_exact(c, a, b); },
         [](int i, int j) { return df_acc{i == j ? -1.f : 0.f, 0.f}; },
-        [&](int i, int j, df_acc c) { E[i + (size_t) j * rk] = df_acc_value(c); }, [](int, int) { return true; });
+        [&](int i, int j, df_acc c) { E[i + (size_t) j * rk] = df_acc_value(c); }, [](int, int, int, int) { return true; });
 }
 
 // Largest column sum of |E| (bounds its norm).
@@ -710,7 +756,7 @@ __device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh
                 S[i + (size_t) j * nc] = ldexpf(tt, -d);
                 S[j + (size_t) i * nc] = -ldexpf(tt, d);
             },
-            [](int i0, int j0) { return i0 <= j0 + 7; });
+            [](int i0, int j0, int, int tj) { return i0 <= j0 + tj - 1; });
         for (int o = 16; o > 0; o >>= 1) {
             mcos = fmaxf(mcos, __shfl_xor_sync(0xffffffffu, mcos, o));
             mtan = fmaxf(mtan, __shfl_xor_sync(0xffffffffu, mtan, o));
@@ -731,7 +777,7 @@ __device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh
                 tm, nc, nc, nc, [&](int i, int k) { return S[i + (size_t) k * nc]; },
                 [&](int k, int j) { return S[k + (size_t) j * nc]; },
                 [](df_acc &c, float a, float b) { c.s = fmaf(a, b, c.s); }, [](int, int) { return df_acc{0.f, 0.f}; },
-                [&](int i, int j, df_acc c) { Q[i + (size_t) j * nc] = 0.5f * c.s; }, [](int, int) { return true; });
+                [&](int i, int j, df_acc c) { Q[i + (size_t) j * nc] = 0.5f * c.s; }, [](int, int, int, int) { return true; });
             tm.sync();
         }
         warp_tiles(
@@ -748,7 +794,7 @@ __device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh
                 double *w = W + i + (size_t) j * rows;
                 *w += double_scaled_up(d.h, ex[j]) + double_scaled_up(d.l, ex[j]);  // the inner sum is exact
             },
-            [](int, int) { return true; });
+            [](int, int, int, int) { return true; });
         tm.sync();
         // what is left after the correction: second order in the angles
         if ((float) nc * mtan * mcos < 0.1f * tol) return true;
@@ -757,11 +803,84 @@ __device__ bool jacobi_correct(const TM &tm, double *W, int rows, int nc, df *Wh
 }
 
 
+// The cross steps of a block pair with the first block's columns in registers (RQ quads a lane, CPG columns a group of
+// G lanes): only the second block's columns go through shared memory, once per step.  The steps are bound by
+// shared-memory bandwidth: 3,400 cycles each for 22 + 22 columns of 340 rows when both go through it twice.
+// Same operations as jacobi32_block_pair.
+template <int G, int RQ, int CPG, class TM>
+__device__ int jacobi32_cross(const TM &tm, float4 *Y, int ls4, int x4, int j4, int nc_a, int nc_b, int off_b, float tol) {
+    const int gl = tm.tid % G, grp = tm.tid / G;
+    constexpr int NG = TM::nth / G;
+    const int wide = nc_a > nc_b ? nc_a : nc_b, len = x4 + j4;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x[CPG][RQ];
+#pragma unroll
+    for (int c = 0; c < CPG; c++)
+#pragma unroll
+        for (int u = 0; u < RQ; u++) {
+            const int r = gl + G * u, p = grp + c * NG;
+            x[c][u] = p < nc_a && r < len ? Y[(size_t) p * ls4 + r] : zero;
+        }
+    int rotations = 0;
+    for (int t = 0; t < wide; t++) {
+#pragma unroll
+        for (int c = 0; c < CPG; c++) {
+            const int p = grp + c * NG, q = p + t < wide ? p + t : p + t - wide;
+            const bool act = p < nc_a && q < nc_b;
+            float4 *yc = Y + (size_t) (off_b + (act ? q : 0)) * ls4;
+            float4 y[RQ];
+            float a = 0.f, b = 0.f, d = 0.f;
+#pragma unroll
+            for (int u = 0; u < RQ; u++) {
+                const int r = gl + G * u;
+                y[u] = act && r < len ? yc[r] : zero;
+                if (r < x4) {
+                    const float4 e = x[c][u], f = y[u];
+                    a = fmaf(e.x, e.x, fmaf(e.y, e.y, fmaf(e.z, e.z, fmaf(e.w, e.w, a))));
+                    b = fmaf(f.x, f.x, fmaf(f.y, f.y, fmaf(f.z, f.z, fmaf(f.w, f.w, b))));
+                    d = fmaf(e.x, f.x, fmaf(e.y, f.y, fmaf(e.z, f.z, fmaf(e.w, f.w, d))));
+                }
+            }
+#pragma unroll
+            for (int o = G >> 1; o > 0; o >>= 1) {
+                a += __shfl_xor_sync(0xffffffffu, a, o);
+                b += __shfl_xor_sync(0xffffffffu, b, o);
+                d += __shfl_xor_sync(0xffffffffu, d, o);
+            }
+            if (act && a > 0.f && b > 0.f && fabsf(d) * rsqrtf(a) * rsqrtf(b) > tol) {
+                float cs, sn;
+                rotation32(a, b, d, cs, sn);
+#pragma unroll
+                for (int u = 0; u < RQ; u++) {
+                    const int r = gl + G * u;
+                    const float4 e = x[c][u], f = y[u];
+                    x[c][u] = make_float4(fmaf(cs, e.x, -sn * f.x), fmaf(cs, e.y, -sn * f.y), fmaf(cs, e.z, -sn * f.z),
+                                          fmaf(cs, e.w, -sn * f.w));
+                    if (r < len)
+                        yc[r] = make_float4(fmaf(cs, f.x, sn * e.x), fmaf(cs, f.y, sn * e.y), fmaf(cs, f.z, sn * e.z),
+                                            fmaf(cs, f.w, sn * e.w));
+                }
+                rotations += gl == 0;
+            }
+        }
+        tm.sync();
+    }
+#pragma unroll
+    for (int c = 0; c < CPG; c++)
+#pragma unroll
+        for (int u = 0; u < RQ; u++) {
+            const int r = gl + G * u, p = grp + c * NG;
+            if (p < nc_a && r < len) Y[(size_t) p * ls4 + r] = x[c][u];
+        }
+    tm.sync();
+    return rotations;
+}
+
 // Stack widths up to which a core fits a quarter and half of an SM's shared memory: the sweep's order and lanes per pair
 // go by the width, not by the team that a launch gives the update.
 constexpr int SMALL_K = 82, LIGHT_K = 117;
 constexpr int SWEEP_BLOCKS = 2 * WIDE_CTAS;  // column blocks of a core that a cluster can hold two at a time a CTA
-constexpr int BLOCK_G16_QUADS = 42;          // up to 168 rows
+constexpr int BLOCK_G16_QUADS = 42;          // up to 168 rows (and as many columns, eleven a block)
 
 // Column blocks of the cluster's sweeps: every CTA of the cluster holds one pair of blocks at a time in its
 // shared memory (buf, `quads` float4s) and sweeps the pairs of columns that it gives; the blocks meet in
@@ -788,8 +907,18 @@ __device__ int jacobi32_blocks(const TM &tm, float4 *Y, int x4, int j4, int nc, 
             for (int e = threadIdx.x; e < na * L; e += TM::cta_threads) buf[e] = __ldcg(ya + e);
             for (int e = threadIdx.x; e < nb * L; e += TM::cta_threads) buf[w * L + e] = __ldcg(yb + e);
             ct.sync();
-            if (rows_g16) rot += jacobi32_block_pair<16>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
-            else rot += jacobi32_block_pair<32>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
+            if (rows_g16) {
+                if (t > 0) rot += jacobi32_cross<16, 6, 1>(ct, buf, L, x4, j4, na, nb, w, tol);
+                else rot += jacobi32_block_pair<16>(ct, buf, L, x4, j4, na, nb, w, false, tol);
+            } else if (t > 0 && L <= 6 * 32 && w <= 16) {
+                rot += jacobi32_cross<32, 6, 1>(ct, buf, L, x4, j4, na, nb, w, tol);
+            } else if (t > 0 && L <= 6 * 32 && w <= 32) {
+                rot += jacobi32_cross<32, 6, 2>(ct, buf, L, x4, j4, na, nb, w, tol);
+            } else if (t > 0 && L <= 8 * 32 && w <= 16) {
+                rot += jacobi32_cross<32, 8, 1>(ct, buf, L, x4, j4, na, nb, w, tol);
+            } else {
+                rot += jacobi32_block_pair<32>(ct, buf, L, x4, j4, na, nb, w, t > 0, tol);
+            }
             for (int e = threadIdx.x; e < na * L; e += TM::cta_threads) ya[e] = buf[e];
             for (int e = threadIdx.x; e < nb * L; e += TM::cta_threads) yb[e] = buf[w * L + e];
             ct.sync();
@@ -1086,21 +1215,25 @@ __device__ int qrcp_truncated(const TM &tm, double *A, int lda, int mrows, int n
 // forms the reflector itself.  (Through global memory a step took 24,000 cycles on a 130-column core, bound
 // by dependent L2 round trips and five cluster barriers.)  R goes to X = R^T directly (rk columns of
 // ncols entries, ld ldx, entry t of column s for pivot order t).  pvt: shared by the cluster.
-__host__ __device__ __forceinline__ int qrcp_cluster_doubles(int mrows, int ncols, int ctas) {
+// Doubles beside the columns.
+__device__ __forceinline__ int qrcp_cluster_aux(int mrows, int ncols, int ctas) {
     const int nl = (ncols + ctas - 1) / ctas;
-    return mrows * nl + 3 * nl + 2 * mrows + (ncols + 1) / 2 + 6 * ctas + 8;
+    return 3 * nl + 2 * mrows + (ncols + 1) / 2 + 6 * ctas + 8;
 }
 
 template <int G, class TM>
 __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, int ncols, double stop2, double rel,
-                            double *X, int ldx, int *pvt, double *pool) {
+                            double *X, int ldx, int *pvt, double *pool, int pool_doubles, double *spill, int lds) {
     constexpr int C = TM::ctas, CPW = 32 / G;
     const Team<TM::cta_threads> ct{(int) threadIdx.x, 1};
     const int warp = ct.warp(), lane = threadIdx.x & 31, nw = ct.nw(), rank = tm.rank;
     const int gl = lane % G, grp = lane / G;
     const int nlmax = (ncols + C - 1) / C, nl = rank < ncols ? (ncols - rank + C - 1) / C : 0;
-    double *A = pool;                               // mrows x nlmax: local column q is column rank + q C
-    double *nrm = A + (size_t) mrows * nlmax;
+    // local column q is column rank + q C; the first `fit` in shared memory, the others in place in `spill`
+    double *A = pool;
+    const int room = (pool_doubles - qrcp_cluster_aux(mrows, ncols, C)) / mrows, fit = room < nlmax ? room : nlmax;
+    auto column = [&](int r, int q) { return spill + (size_t) (r + q * C) * lds; };
+    double *nrm = A + (size_t) mrows * fit;
     double *nref = nrm + nlmax;
     double *xb = nref + nlmax;                      // the pivot column
     double *diag = xb + mrows;                      // beta of every step
@@ -1111,10 +1244,11 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
     int *taken = act_list + 2 * nlmax;              // per column: chosen (for the leftovers)
     for (int q = warp; q < nl; q += nw) {
         const double *col = M + (size_t) (rank + q * C) * ldm;
+        double *own = q < fit ? A + (size_t) q * mrows : column(rank, q);
         double t = 0.0;
         for (int i = lane; i < mrows; i += 32) {
             const double v = col[i];
-            A[i + (size_t) q * mrows] = v;
+            own[i] = v;
             t = fma(v, v, t);
         }
         t = warp_sum(t);
@@ -1158,7 +1292,7 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
         }
         const int owner = bi % C, lcol = bi / C;
         if (warp == 0) {
-            const double *x = cluster_map(A, owner) + (size_t) lcol * mrows;
+            const double *x = lcol < fit ? cluster_map(A, owner) + (size_t) lcol * mrows : column(owner, lcol);
             double t = 0.0;
             if (lane == 0) xb[s] = x[s];
             for (int i = s + 1 + lane; i < mrows; i += 32) {
@@ -1189,7 +1323,7 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
         for (int q0 = warp * CPW; q0 < nact; q0 += nw * CPW) {
             const bool act = q0 + grp < nact;
             const int c = act_list[act ? q0 + grp : 0];
-            reflect_column<G>(act, A + (size_t) c * mrows, xb, h, s, mrows, gl, nrm + c, nref + c);
+            reflect_column<G>(act, c < fit ? A + (size_t) c * mrows : column(rank, c), xb, h, s, mrows, gl, nrm + c, nref + c);
         }
         ct.sync();
     }
@@ -1202,7 +1336,7 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
     tm.sync();
     for (int t = tm.warp(); t < ncols; t += tm.nw()) {
         const int j = pvt[t];
-        const double *col = cluster_map(A, j % C) + (size_t) (j / C) * mrows;
+        const double *col = j / C < fit ? cluster_map(A, j % C) + (size_t) (j / C) * mrows : column(j % C, j / C);
         for (int i = lane; i < rk; i += 32) X[t + (size_t) i * ldx] = i < t ? col[i] : (i == t ? diag[i] : 0.0);
         if (rk == 0 && lane == 0) X[t] = M[(size_t) j * ldm];
     }
@@ -1503,8 +1637,9 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         ldw = ldm;
     }
 
-    // A cluster holds the columns of M in its CTAs' shared memory during the pivoted QR, where they fit.
-    const bool spread = CLUSTER && qrcp_cluster_doubles(kU, kV, TM::ctas) <= pool_doubles;
+    // A cluster holds the columns of M in its CTAs' shared memory during the pivoted QR, as far as they fit (the working
+    // copy takes the others).
+    constexpr bool spread = CLUSTER;
 
     const long long t0 = clock64();
     // 1. M = R_U R_V^T on DMMA (R_U = triu of the U stack's top kU rows, likewise R_V), or the tile itself.
@@ -1589,9 +1724,9 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
                                reinterpret_cast<df *>(inv), pvt, reinterpret_cast<float *>(red), redi);
     } else if (spread) {
         if constexpr (CLUSTER) {  // lanes per column as in qrcp_truncated
-            rk = kU <= 64    ? qrcp_cluster<4>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool)
-                 : kU <= 256 ? qrcp_cluster<8>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool)
-                             : qrcp_cluster<16>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool);
+            rk = kU <= 64    ? qrcp_cluster<4>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool, pool_doubles, Mw, ldw)
+                 : kU <= 256 ? qrcp_cluster<8>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool, pool_doubles, Mw, ldw)
+                             : qrcp_cluster<16>(tm, Mc, ldm, kU, kV, stop2, rel, XV, ld, pvt, pool, pool_doubles, Mw, ldw);
         }
     } else {
         rk = qrcp_truncated(tm, Mw, ldw, kU, kV, stop2, rel, nrm, inv, pvt, red, redi);
@@ -1822,7 +1957,9 @@ void core_classes(int kmax, int *whole, int *half, int *quarter) {
 
 static void launch_core_wide(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {
     const int aux = 6 * ws.kmax + SVD_AUX_FIXED + 1;
-    const int doubles = std::min(aux + WIDE_POOL_DOUBLES, 2 * svd_team_doubles(ws.kmax));
+    // a pair of column blocks, or (wider cores) as many columns as there is room for
+    const int most = 2 * svd_team_doubles(ws.kmax);
+    const int doubles = ws.kmax <= WIDE_POOL_K ? std::min(aux + WIDE_POOL_DOUBLES, most) : most;
     const size_t bytes = sizeof(double) * (size_t) doubles;
     cudaFuncSetAttribute(core_wide_kernel<CORE_RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) bytes);
     const int ctas = std::min(n, WIDE_CLUSTERS) * WIDE_CTAS;
