@@ -191,7 +191,7 @@ class Context:
         """hcgb_tlr_gemm as a captured CUDA graph, replayed while the call is unchanged."""
         self.check(lib().hcgb_set_graph(self._h, int(bool(enable))))
 
-    def set_tuning(self, oz_min_outputs: int = 2048, wy_min_reflectors: int = 48):
+    def set_tuning(self, oz_min_outputs: int = 256, wy_min_reflectors: int = 24):
         self.check(lib().hcgb_set_tuning(self._h, int(oz_min_outputs), int(wy_min_reflectors)))
 
     def set_precond(self, min_cols: int = 0):

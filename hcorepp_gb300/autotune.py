@@ -22,8 +22,8 @@ import os
 import numpy as np
 
 CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuning_cache.json")
-DEFAULT = {"groups": 8, "wy_min": 48, "oz_min": 2048, "graph": 0, "precond": 16}
-CANDIDATES = {"groups": [4, 8, 16], "wy_min": [32, 48, 96, 1 << 30], "oz_min": [512, 1024, 2048, 4096],
+DEFAULT = {"groups": 8, "wy_min": 24, "oz_min": 256, "graph": 0, "precond": 16}
+CANDIDATES = {"groups": [4, 8, 16], "wy_min": [16, 24, 48, 96, 1 << 30], "oz_min": [256, 512, 1024, 4096],
               "graph": [0, 1], "precond": [16, 32, 64, 1 << 30]}
 ORDER = ["groups", "wy_min", "oz_min", "graph", "precond"]
 # The float-float form applies Q in float-float panels on every side (no WY form), so wy_min does not act on

@@ -174,9 +174,10 @@ __device__ __forceinline__ int job_of_tile(const int *sched, int njobs, int w) {
     return lo;
 }
 
-// Products worth the split (enough k to amortise the 4 FP64 instructions per output, enough outputs
-// for a tile).
-constexpr int OZ_MIN_OUTPUTS = 2048;
+// Products worth the split: a 16 x 16 product takes both paths about as long (K = 512: 280 and 310 us for 608 of them;
+// K = 64: 85 and 58), a 32 x 32 one is 2 and 1.2 times faster here.  Multiplies 11x11 nb=301, n=16384 and n=8192 at 1e-4:
+// 68.5, 707 and 58.9 ms from 256 outputs and 24 reflectors on, 72.7, 719 and 61.0 from 2048 and 48 on.
+constexpr int OZ_MIN_OUTPUTS = 256;
 __host__ __device__ inline bool oz_shape(int M, int N, int K, int min_outputs = OZ_MIN_OUTPUTS) {
     return K >= 16 && M >= 16 && N >= 8 && (long long) M * N >= min_outputs;
 }
@@ -323,7 +324,7 @@ constexpr int SCHED_INTS_PER_UPDATE = 16;  // >= (3 * 4n + 3) / n: one WY launch
 // with at least WY_MIN_REFLECTORS reflectors (their products run on the tensor cores); the
 // others keep the panel-wise apply_q_kernel, which skips the WY sides.  Plain form only: the mixed
 // form's float-float panels are faster than either.
-constexpr int WY_MIN_REFLECTORS = 48;
+constexpr int WY_MIN_REFLECTORS = 24;
 void launch_plan_wy(const DevUpdate *ups, int n, Workspace ws, Params p, GemmJob *jobs, cudaStream_t st);
 void launch_wy_solve(int n, Workspace ws, cudaStream_t st);
 void launch_qr(Workspace ws, int n, bool mixed, cudaStream_t st);

@@ -18,9 +18,10 @@
 //     accumulators are read out of tensor memory and added into two 64-bit integers (levels 0-3 and
 //     4-7, each shifted to a common scale), which stay exact for k up to 2^16, and the tile ends with
 //     C_ij = 2^(e_i + f_j) (hi 2^-35 + lo 2^-63).
-// Tensor memory holds the eight level accumulators of a 128 x 64 output tile (512 columns); one
-// thread issues the 72 MMAs (36 pairs x 2 k-steps of 16) of a 32-wide K chunk while the others cut
-// the next chunk into digit planes in the second shared-memory stage.
+// Tensor memory holds the eight level accumulators of a 128 x 64 output tile (512 columns).  The sixteen warps cut
+// 32-wide K chunks into digit planes, two shared-memory stages in turn, and read the accumulators out; a thread of the
+// last one issues the 72 MMAs (36 pairs x 2 k-steps of 16) of a chunk when it is filled.  They meet on mbarriers
+// only (every wait bounded).
 //
 // What bounds it is the splitting, not the tensor cores: every operand element becomes eight FP16 digits.  A
 // bias of 64 in every digit makes the balanced digits independent bit fields (no carry from digit to digit),
@@ -102,47 +103,41 @@ __device__ __forceinline__ int oz_off(int r, int kk) {
     return ((r >> 3) * OZ_KB + (kk >> 3)) * 128 + (r & 7) * 16 + (kk & 7) * 2;
 }
 
-// (hi 2^28 + lo) 2^(e - 63) as a double, rounded once (to nearest even), by integer operations.
+// (hi 2^28 + lo) 2^(e - 63) as a double, rounded once (to nearest even), by integer operations without branches
+// (a normal result; the rare others through ldexp).
 __device__ __forceinline__ double oz_value(long long hi, long long lo, int e) {
     long long t = hi + (lo >> 28);
     uint32_t r = (uint32_t) lo & 0xfffffffu;  // the number is t 2^28 + r
     const bool neg = t < 0;
-    if (neg) {
-        t = -t;
-        if (r) {
-            t -= 1;
-            r = 0x10000000u - r;
-        }
-    }
-    const unsigned long long u = (unsigned long long) t;
-    unsigned long long x;
-    int ex;
-    bool sticky = false;
-    if (u) {
-        const int n = __clzll(u);
-        x = u << n;
-        if (n >= 28) {
-            x |= (unsigned long long) r << (n - 28);
-        } else {
-            x |= r >> (28 - n);
-            sticky = (r & ((1u << (28 - n)) - 1u)) != 0;
-        }
-        ex = 28 - n;
-    } else if (r) {
-        const int n = __clzll((unsigned long long) r);
-        x = (unsigned long long) r << n;
-        ex = -n;
-    } else {
-        return 0.0;
-    }
-    ex += e - 63;  // x 2^ex, the leading bit of x set
-    const uint32_t rest = (uint32_t) x & 0x7ffu;
-    unsigned long long m = x >> 11;
-    if (rest > 0x400u || (rest == 0x400u && (sticky || (m & 1)))) m++;
-    const int field = ex + 63 + 1023;
-    double v;
-    if (field > 0 && field < 2046) v = __longlong_as_double((long long) (((unsigned long long) (field - 1) << 52) + m));
-    else v = ldexp((double) m, ex + 11);
+    t = neg ? ~t + (r == 0 ? 1 : 0) : t;
+    r = neg ? (0u - r) & 0xfffffffu : r;
+    // |number| 2^4 as three words, the leading bit shifted to the top
+    uint32_t w2 = (uint32_t) ((unsigned long long) t >> 32), w1 = (uint32_t) t, w0 = r << 4;
+    int n = 0;
+    const bool z2 = w2 == 0;
+    w2 = z2 ? w1 : w2;
+    w1 = z2 ? w0 : w1;
+    w0 = z2 ? 0u : w0;
+    n += z2 ? 32 : 0;
+    const bool z1 = w2 == 0;
+    w2 = z1 ? w1 : w2;
+    w1 = z1 ? w0 : w1;
+    w0 = z1 ? 0u : w0;
+    n += z1 ? 32 : 0;
+    const int c = __clz(w2) & 31;
+    const bool zero = w2 == 0;
+    w2 = __funnelshift_l(w1, w2, c);
+    w1 = __funnelshift_l(w0, w1, c);
+    w0 <<= c;
+    n += c;
+    // the leading bit stands for 2^(91 - n) of the number
+    const uint32_t rest = w1 & 0x7ffu;
+    unsigned long long m = ((unsigned long long) w2 << 21) | (w1 >> 11);
+    m += (rest > 0x400u || (rest == 0x400u && (w0 != 0 || (m & 1)))) ? 1 : 0;
+    const int field = 91 - n + e - 63 + 1023;
+    const unsigned long long bits = ((unsigned long long) (field - 1) << 52) + m;
+    double v = zero ? 0.0 : __longlong_as_double((long long) bits);
+    if (!zero && (field <= 0 || field >= 2046)) v = ldexp((double) m, field - 1023 - 52);
     return neg ? -v : v;
 }
 
@@ -188,9 +183,16 @@ __device__ __forceinline__ void split_run(const double (&v)[NK], int e, unsigned
     plane(std::integral_constant<int, 7>{});
 }
 
-// One 128 x 64 output tile of one job.
-__device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint32_t tmem, uint32_t mbar0,
-                        uint32_t (&phase)[2], bool (&pending)[2], int *ea, int *eb) {
+// Barriers of the CTA: full[2] (the sixteen warps have filled a stage), empty[2] (the MMAs have read it: a commit),
+// read (the sixteen warps have read the accumulators).
+struct OzBarriers {
+    uint32_t full, empty, read;
+};
+
+// One 128 x 64 output tile of one job.  chunks / windows: 32-wide K chunks and read-out windows of the CTA's earlier
+// tiles; chunk t fills stage t & 1 for the (t >> 1)-th time.
+__device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint32_t tmem, const OzBarriers &bars,
+                        int &chunks, int &windows, int *ea, int *eb) {
     const int ntm = (jb.M + OZ_TM - 1) / OZ_TM;
     const int m0 = (tile % ntm) * OZ_TM, n0 = (tile / ntm) * OZ_TN;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -233,17 +235,7 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     unsigned long long hi[16], lo[16];  // levels 0-3 at scale 2^-35, levels 4-7 at scale 2^-63
 #pragma unroll
     for (int j = 0; j < 16; j++) hi[j] = lo[j] = 0;
-    int windows = 0;
     bool ok = true;
-    auto drain = [&]() {  // every committed MMA complete (each commit waited for exactly once)
-        for (int b = 0; b < 2; b++)
-            if (pending[b]) {
-                ok &= tc::mbar_wait(mbar0 + 8 * b, phase[b]);
-                phase[b] ^= 1;
-                pending[b] = false;
-            }
-        tc::fence_after();
-    };
     // A level sum iv appears as the bit pattern 0x4B400000 + iv of iv + 1.5 2^23; the pattern is added with the
     // level's weight, what the constant contributes is taken off at the end.
     auto readout = [&]() {
@@ -264,16 +256,40 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
                 }
             }
         }
-        windows++;
         tc::fence_before();
-        __syncthreads();  // the next MMAs overwrite the accumulators only after every read-out
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bars.read);  // the next window's MMAs may overwrite the accumulators
     };
 
     // this thread's runs: eight K of a row of A, four of a column of B (see oz_off for the layout)
     const bool ka = jb.opA != 0;
     const int ra = ka ? tid >> 2 : tid & 127, ca = ka ? tid & 3 : tid >> 7;
     const int rb = (tid & 7) + 8 * (tid >> 6), cb = ((tid >> 4) & 3) * 8 + ((tid >> 3) & 1) * 4;
-    const int nchunks = (jb.K + OZ_KC - 1) / OZ_KC;
+    const int nchunks = (jb.K + OZ_KC - 1) / OZ_KC, nwindows = (nchunks + OZ_FLUSH - 1) / OZ_FLUSH;
+    // the MMAs of chunk c, by one thread
+    auto issue = [&](int c) {
+        const int t = chunks + c, buf = t & 1, fill = t >> 1, window = windows + c / OZ_FLUSH;
+        const bool first = (c % OZ_FLUSH) == 0;  // accumulators restart after every read-out
+        ok &= tc::mbar_wait(bars.full + 8 * buf, fill & 1);
+        if (first && window > 0) ok &= tc::mbar_wait(bars.read, (window - 1) & 1);
+        tc::fence_after();
+        unsigned char *sa = stage0 + buf * OZ_STAGE, *sb = sa + OZ_S * OZ_A_PLANE;
+        const uint64_t ad = tc::smem_desc(tc::smem_u32(sa), 128, OZ_KB * 128);
+        const uint64_t bd = tc::smem_desc(tc::smem_u32(sb), 128, OZ_KB * 128);
+#pragma unroll
+        for (int ks = 0; ks < OZ_KC / 16; ks++)
+#pragma unroll
+            for (int s = 0; s < OZ_S; s++)
+#pragma unroll
+                for (int u = 0; u < OZ_S - s; u++) {
+                    // The first MMA into level L of a read-out window overwrites it: in this order
+                    // that is the pair (0, L) of the window's first k-step.
+                    const bool overwrite = first && ks == 0 && s == 0;
+                    tc::mma_f16(tmem + (uint32_t) ((s + u) * OZ_TN), ad + ((s * OZ_A_PLANE + ks * 256) >> 4),
+                                bd + ((u * OZ_B_PLANE + ks * 256) >> 4), idesc, overwrite ? 0u : 1u);
+                }
+        tc::commit(bars.empty + 8 * buf);
+    };
     double va[8], vb[4];  // the next chunk's runs, loaded while this one's products are issued and read out
     auto load = [&](int c) {
         if (ra < rows) load_run<true, 8>(jb, m0 + ra, c * OZ_KC + 8 * ca, va);
@@ -281,50 +297,34 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     };
     if (nchunks > 0) load(0);
     for (int c = 0; c < nchunks; c++) {
-        const int buf = c & 1;
+        const int t = chunks + c, buf = t & 1, fill = t >> 1;
         unsigned char *sa = stage0 + buf * OZ_STAGE, *sb = sa + OZ_S * OZ_A_PLANE;
-        if (pending[buf]) {  // the MMAs of chunk c - 2 have read this stage
-            ok &= tc::mbar_wait(mbar0 + 8 * buf, phase[buf]);
-            phase[buf] ^= 1;
-            pending[buf] = false;
-        }
+        if (fill > 0) ok &= tc::mbar_wait(bars.empty + 8 * buf, (fill - 1) & 1);
         if (ra < rows) split_run<8>(va, ea[ra], sa + oz_off(ra, 8 * ca), OZ_A_PLANE);
         if (rb < cols) split_run<4>(vb, eb[rb], sb + oz_off(rb, cb), OZ_B_PLANE);
-        if (c + 1 < nchunks) load(c + 1);
         tc::fence_smem_to_async();
-        __syncthreads();
-        if (tid == OZ_THREADS - 32) {
-            tc::fence_after();
-            const uint64_t ad = tc::smem_desc(tc::smem_u32(sa), 128, OZ_KB * 128);
-            const uint64_t bd = tc::smem_desc(tc::smem_u32(sb), 128, OZ_KB * 128);
-            const bool first = (c % OZ_FLUSH) == 0;  // accumulators restart after every read-out
-#pragma unroll
-            for (int ks = 0; ks < OZ_KC / 16; ks++)
-#pragma unroll
-                for (int s = 0; s < OZ_S; s++)
-#pragma unroll
-                    for (int t = 0; t < OZ_S - s; t++) {
-                        // The first MMA into level L of a read-out window overwrites it: in this order
-                        // that is the pair (0, L) of the window's first k-step.
-                        const bool overwrite = first && ks == 0 && s == 0;
-                        tc::mma_f16(tmem + (uint32_t) ((s + t) * OZ_TN), ad + ((s * OZ_A_PLANE + ks * 256) >> 4),
-                                    bd + ((t * OZ_B_PLANE + ks * 256) >> 4), idesc, overwrite ? 0u : 1u);
-                    }
-            tc::commit(mbar0 + 8 * buf);
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(bars.full + 8 * buf);
+        if (c + 1 < nchunks) load(c + 1);
+        if (__shfl_sync(0xffffffffu, warp, 0) == OZ_THREADS / 32 - 1) {  // uniform, as the MMAs' operands must be
+            if (tc::elect_one()) issue(c);
+            __syncwarp();
         }
-        pending[buf] = true;
         if ((c + 1) % OZ_FLUSH == 0 || c + 1 == nchunks) {
-            drain();
+            ok &= tc::mbar_wait(bars.empty + 8 * buf, fill & 1);  // this commit covers every earlier MMA
+            tc::fence_after();
             readout();
         }
     }
-    if (!ok && tid == 0) atomicAdd(&g_oz_wait_timeouts, 1u);
+    chunks += nchunks;
+    windows += nwindows;
+    if (!ok && lane == 0) atomicAdd(&g_oz_wait_timeouts, 1u);
 
     // Epilogue: C = alpha * product + beta * C, one row per thread, 16 columns.
     const int row_l = q * 32 + lane;
     if (reads && row_l < rows) {
         const unsigned long long constant =
-            (unsigned long long) windows * 0x4B400000ull * ((1ull << 21) + (1ull << 14) + (1ull << 7) + 1ull);
+            (unsigned long long) nwindows * 0x4B400000ull * ((1ull << 21) + (1ull << 14) + (1ull << 7) + 1ull);
         const bool scale = jb.alpha != 1.0 && jb.alpha != -1.0, negate = jb.alpha == -1.0, accum = jb.beta != 0.0;
 #pragma unroll
         for (int j = 0; j < 16; j++) {
@@ -347,7 +347,7 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
 // entries); a grid sized to the GPU strides over them.
 __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_jobs_kernel(const GemmJob *jobs, int njobs, const int *sched) {
     extern __shared__ __align__(1024) unsigned char oz_smem_raw[];
-    __shared__ __align__(8) unsigned long long mbar[2];
+    __shared__ __align__(8) unsigned long long mbar[5];
     __shared__ uint32_t tmem_slot;
     __shared__ int ea[OZ_TM], eb[OZ_TN];
     unsigned char *stage0 = reinterpret_cast<unsigned char *>(
@@ -356,20 +356,23 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_jobs_kernel(const GemmJ
     if (blockIdx.x >= total) return;  // whole CTA leaves before any TMEM or barrier is set up
     const uint32_t mbar0 = tc::smem_u32(&mbar[0]);
     if (threadIdx.x == 0) {
-        tc::mbar_init(mbar0, 1);
-        tc::mbar_init(mbar0 + 8, 1);
+        for (int b = 0; b < 2; b++) {
+            tc::mbar_init(mbar0 + 8 * b, OZ_THREADS / 32);
+            tc::mbar_init(mbar0 + 16 + 8 * b, 1);
+        }
+        tc::mbar_init(mbar0 + 32, OZ_THREADS / 32);
     }
     if ((threadIdx.x >> 5) == 0) tc::tmem_alloc(tc::smem_u32(&tmem_slot), OZ_TMEM_COLS);
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = tmem_slot;
-    uint32_t phase[2] = {0u, 0u};
-    bool pending[2] = {false, false};
+    const OzBarriers bars{mbar0, mbar0 + 16, mbar0 + 32};
+    int chunks = 0, windows = 0;
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int lo = job_of_tile(sched, njobs, w);
         const GemmJob jb = jobs[lo];
-        oz_tile(jb, w - sched[lo], stage0, tmem, mbar0, phase, pending, ea, eb);
+        oz_tile(jb, w - sched[lo], stage0, tmem, bars, chunks, windows, ea, eb);
     }
     __syncthreads();
     if ((threadIdx.x >> 5) == 0) tc::tmem_free(tmem, OZ_TMEM_COLS);

@@ -50,6 +50,13 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b,
         "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 
+// True in one thread of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
 // The mbarrier at `mbar` receives one arrival when every tcgen05 operation issued so far by this
 // thread has completed.
 __device__ __forceinline__ void commit(uint32_t mbar) {
@@ -109,6 +116,10 @@ __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    asm volatile("{\n.reg .b64 t;\nmbarrier.arrive.shared::cta.b64 t, [%0];\n}\n" ::"r"(mbar) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -125,7 +136,7 @@ __device__ __forceinline__ bool mbar_test(uint32_t mbar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
     for (int i = 0; i < (1 << 22); i++) {
         if (mbar_test(mbar, parity)) return true;
-        if (i > 64) __nanosleep(256);
+        if (i > 256) __nanosleep(256);
     }
     return false;
 }

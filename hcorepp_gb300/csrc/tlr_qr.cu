@@ -68,7 +68,8 @@ __device__ bool factor_panel(double *Ps, int ldp, int mr, int nbp, double *tau_s
     for (int j = 0; j + 1 < nbp; j++) {
         const double *x = Ps + (size_t) j * ldp;
         const double scale = red[j], tau = tau_s[j];
-        for (int c = j + 1 + warp; c < nbp; c += nw) {
+        // the first warp has the next column to itself, the others share the rest
+        for (int c = j + 1 + warp; c < nbp; c += warp == 0 ? nbp : nw - 1) {
             double *y = Ps + (size_t) c * ldp;
             double ss = 0.0, alpha = y[c];
             if (tau != 0.0) {

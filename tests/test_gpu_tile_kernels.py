@@ -125,3 +125,21 @@ def test_compression_of_rectangular_tiles(T, m, n, mode):
     o = O.CompressedTile.from_dense(d, O.CompressionParameters(1e-8, truncated_svd=True), max_rank=r)
     assert abs(g.rank - o.rank) <= 1
     assert rel_fro(g.to_dense(), d) <= 2 * max(rel_fro(o.to_dense(), d), 1e-14)
+
+
+@pytest.mark.parametrize("k", [16, 17, 33, 128, 129, 512])
+@pytest.mark.parametrize("m,n", [(16, 16), (17, 31), (129, 8), (40, 70), (300, 24)])
+def test_tensor_core_products_at_tile_edges(T, m, n, k):
+    """One dense update C = A B + C on the tensor cores: 56-bit operands relative to the row and column maxima
+    (rounding 2^-57 each, dropped digit pairs below 2^-56), one rounding of the sum and one of beta C."""
+    rng = np.random.default_rng([m, n, k])
+    a = rng.standard_normal((m, k)) * 2.0 ** rng.integers(-20, 20, (m, 1))
+    b = rng.standard_normal((k, n)) * 2.0 ** rng.integers(-20, 20, (1, n))
+    a[0], b[:, 0] = 0.0, -np.abs(b[:, 0])
+    c = rng.standard_normal((m, n))
+    g = T.DenseTile(m, n, c)
+    T.HCore.Gemm(1.0, T.DenseTile(m, k, a), 0, T.DenseTile(k, n, b), 0, 1.0, g, T.CompressionParameters(1e-8))
+    p = a.astype(np.longdouble) @ b.astype(np.longdouble)
+    scale = np.abs(a).max(1)[:, None] * np.abs(b).max(0)[None, :]
+    bound = 2 * k * 2.0 ** -56 * scale * 2 + EPS * np.abs(p) + EPS * (np.abs(c) + np.abs(p))
+    assert np.all(np.abs(g.to_dense() - (p + c)) <= bound)
