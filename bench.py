@@ -1,14 +1,14 @@
 #!/usr/bin/env python
 """TLR-GEMM tile-updates/s at 1e-8 relative accuracy on GB300.
 
-Headline ("value", "e2e", "roofline"): the plain FP64 form -- the stack QR, the core SVD (pivoted
-QR + one-sided Jacobi) and the Q application in double precision on the FP64 pipe (DFMA / DMMA);
-the factor products FP64-accurate (DMMA, or for the larger ones the 16-bit tensor cores by
+Headline ("value", "e2e", "roofline"): the plain FP64 form -- the stack QR, the core SVD (pivoted QR,
+one-sided Jacobi whose rotations are found in single precision and whose columns are finished to FP64
+working precision) and the Q application in double precision; the factor products FP64-accurate (DMMA, or for the larger ones the 16-bit tensor cores by
 error-free splitting, error below FP64's own worst-case bound).
 
 Other forms, each timed in the same process on the same inputs and reported in "forms" with its
 own value, e2e, product error and speed-up over the plain form:
-  mixed_ff48 : the stack QR, the core's pivoted QR and Jacobi and the Q application in
+  mixed_ff48 : the stack QR, the pivoted QR of cores up to 117 columns and the Q application in
                float-float arithmetic (two floats, 48-bit significand) on the FP32 pipe.
 
 Workload (default): n = 16384, nb = 512 -> 32 x 32 tiles, Morton-sorted 2-D points,
@@ -53,10 +53,10 @@ METRIC = "TLR-GEMM tile-updates/s at 1e-8 rel err: plain FP64 vs batched mixed+l
 UNIT = "tile-updates/s"
 HEADLINE_FORM = "plain_fp64"
 FORM_NOTES = {
-    "plain_fp64": "FP64 throughout: stack QR, core SVD (pivoted QR + one-sided Jacobi) and Q application on the "
-                  "FP64 pipe; factor products FP64-accurate (DMMA, or 16-bit tensor cores by error-free splitting)",
-    "mixed_ff48": "stack QR, core pivoted QR + Jacobi and Q application in float-float (48-bit significand) on the "
-                  "FP32 pipe; core product, new factors, truncation test and factor products as in plain_fp64",
+    "plain_fp64": "FP64 results throughout: stack QR, core SVD (pivoted QR, Jacobi rotations found in FP32, columns "
+                  "formed in FP64 and corrected to its working precision) and Q application; products FP64-accurate (DMMA, or 16-bit tensor cores by error-free splitting)",
+    "mixed_ff48": "stack QR, narrower cores' pivoted QR and Q application in float-float (48-bit significand) on the "
+                  "FP32 pipe; core SVD, core product, new factors, truncation test and factor products as in plain_fp64",
     "learned_ff48": "mixed_ff48 with the learned form: an MLP (trained on plain runs of other seeds, "
                     "hcorepp_gb300/rank_model_weights.npy) sizes a Gaussian sketch of each update; the plain "
                     "recompression runs where the a-posteriori residual test fails",

@@ -14,8 +14,9 @@ constexpr int CT = 1024;
 
 // Blocked right-looking Cholesky.  One launch per 32-column block solves the rows below it, one updates the
 // trailing 32 x 32 tiles over the whole GPU; the CTA of the next diagonal tile factors it on the spot, so a
-// block costs two launches.  (One CTA walking the columns, each a left-looking product from L2, took 55 ms
-// for n = 512: one SM's FP64 pipe and dependent loads.)  L(i, k) stands at A[i rs + k cs]: lower triangle
+// block costs two launches.  (One CTA walked the columns, each a left-looking product from L2, bound by one
+// SM's FP64 pipe and dependent loads: with the panel solve below, five tiles of 512 and ten panel tiles took 285 ms
+// of a tile Cholesky, 10 ms now.)  L(i, k) stands at A[i rs + k cs]: lower triangle
 // rs = 1, cs = lda, upper the other way round.  Every L(i, j) takes its products in ascending k.
 constexpr int PB = 32;
 
@@ -207,7 +208,7 @@ __global__ void fill_triangle_kernel(int uplo, int n, double *A, int lda, double
 // as the tile Cholesky applies it (src/api/HCore.cpp:623-647), the rank read on the device.  One CTA per
 // tile and TRSM_COLS columns, which stay in shared memory: blocks of 32 rows are solved, then taken out of
 // the rows below.  Every element takes the same operations in the same order as in trsm_kernel, so the
-// results are identical.  (One CTA per tile, one row a step through L2: 15 ms for 512 rows and 100 columns.)
+// results are identical.  (One CTA took a tile, one row a step through L2.)
 constexpr int TRSM_COLS = 4, TRSM_THREADS = 256;
 __global__ void __launch_bounds__(TRSM_THREADS) trsm_panel_kernel(const double *L, int nb, int ldl, const DevTile *tiles,
                                                                   int in_smem) {

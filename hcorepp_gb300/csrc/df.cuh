@@ -2,7 +2,8 @@
 // (|l| <= ulp(h) / 2), 48 significant bits, computed on the FP32 pipe (about 70x the FP64 rate of
 // this GPU).  Error-free transformations (Knuth two-sum, FMA two-product; Dekker's double-length
 // arithmetic) with explicitly rounded intrinsics so that nothing is contracted or reassociated.
-// Used by the mixed form of the recompression (core pivoted QR and Jacobi, Householder panels).
+// Used by the mixed form of the recompression (stack QR, pivoted QR of the narrower cores, Q application) and by
+// the corrections that finish every form's core SVD (their products; sums are added to FP64 columns).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -65,18 +66,6 @@ __device__ __forceinline__ df df_f(float v) {
     r.l = 0.f;
     return r;
 }
-// 1 / sqrt(q) for q >= 1 to float-float accuracy: two Newton steps r <- r + r (1 - q r^2) / 2 from
-// the float reciprocal square root (about 22 -> 44 -> 48 correct bits).
-__device__ __forceinline__ df df_rsqrt(df q) {
-    df r = df_f(rsqrtf(q.h));
-#pragma unroll
-    for (int it = 0; it < 2; it++) {
-        const df res = df_add(df_f(1.f), -df_mul(q, df_mul(r, r)));  // 1 - q r^2, small
-        r = df_add(r, df_mul(df_mul(r, res), df_f(0.5f)));
-    }
-    return r;
-}
-
 // Float-float reciprocal and square root (one correction step each from the float result).
 __device__ __forceinline__ df df_div(df a, df b) {
     const float q0 = __fdiv_rn(a.h, b.h);

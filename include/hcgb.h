@@ -68,13 +68,14 @@ typedef struct {
     int mode;           /* hcgb_mode: arithmetic of the recompression core */
 } hcgb_params;
 
-/* HCGB_PLAIN_FP64: the recompression (stack QR, core SVD, Q application) in double precision.
- * HCGB_MIXED: the stack QR, the core SVD's pivoted QR and Jacobi sweeps and the panel-wise Q
+/* HCGB_PLAIN_FP64: the recompression (stack QR, core SVD, Q application) in double precision (the core SVD
+ * finds its rotations in single precision and finishes the columns to FP64 working precision).
+ * HCGB_MIXED: the stack QR, the pivoted QR of cores up to 117 columns and the panel-wise Q
  * application in float-float arithmetic (a value is the unevaluated sum of two floats, 48-bit
  * significand) on the FP32 pipe, each block scaled by an exact power of two first; the core
  * product, the new factors, the truncation test and all factor products stay in double precision.
  * Backward error of the float-float stages ~2^-48 relative: same ranks and product accuracy as the
- * plain form at the accuracies this path is used at (>= 1e-12 relative), about 1.6x as fast.
+ * plain form at the accuracies this path is used at (>= 1e-12 relative), faster.
  * In both forms the larger factor products run on the 16-bit tensor cores by FP64-accurate
  * error-free splitting unless hcgb_set_tensor_products(ctx, 0). */
 typedef enum { HCGB_PLAIN_FP64 = 0, HCGB_MIXED = 1, HCGB_TF32 = 2, HCGB_BF16 = 3 } hcgb_mode;
@@ -102,7 +103,7 @@ typedef struct {
     int rank_c;
     int k;          /* columns of the stacked bases that were recompressed (0 for a dense C) */
     int new_rank;   /* rank of C after the update (0 for a dense C) */
-    int sweeps;     /* Jacobi sweeps the core SVD took */
+    int sweeps;     /* Jacobi sweeps and corrections the core SVD took */
     int side;       /* 0: stacked [Cu | alpha Au]; 1: stacked [Cu | alpha Au (Av Bu)] */
     int core_cols;  /* rows of R the rank-revealing QR of the core kept (columns Jacobi rotated) */
     int core_kcycles[4]; /* core SVD phases in units of 1024 SM cycles: core product, pivoted QR,
