@@ -998,9 +998,10 @@ namespace {
 
 // Whether a compression runs the core on the dense tiles themselves.  The low-precision forms and the learned
 // form (and a feature sink) take the identity-operand update instead: their product precision, sketch
-// and records belong to it.
-bool compress_direct(const hcgb_context *ctx, const hcgb_params *params) {
-    return !ctx->learned && !ctx->feature_sink && !lowp_prec(params ? params->mode : 0);
+// and records belong to it.  So do long tiles, whose stack QR leaves a much smaller core.
+bool compress_direct(const hcgb_context *ctx, const hcgb_params *params, int rows, int cols) {
+    return !ctx->learned && !ctx->feature_sink && !lowp_prec(params ? params->mode : 0) &&
+           std::max(rows, cols) <= 2 * std::min(rows, cols);
 }
 
 // Truncated SVDs of n dense tiles (rows x cols) into out, chunk by chunk; statuses and ranks in dinfo.
@@ -1036,7 +1037,7 @@ extern "C" int hcgb_compress_tile(hcgb_context *ctx, const double *dense, int ro
     if (!dense || !out || rows <= 0 || cols <= 0 || !compressed(out->kind) || out->rows != rows ||
         out->cols != cols || !out->rank || out->max_rank <= 0)
         return fail(ctx, HCGB_BAD_ARG, "hcgb_compress_tile: bad arguments");
-    if (compress_direct(ctx, params)) return hcgb_compress_tiles(ctx, 1, &dense, rows, cols, out, params, rank);
+    if (compress_direct(ctx, params, rows, cols)) return hcgb_compress_tiles(ctx, 1, &dense, rows, cols, out, params, rank);
     HCGB_CUDA(ctx, cudaSetDevice(ctx->device));
     // D = D * I: an update with A = the dense tile, B = I (compressed, U = V = I_cols), C = 0 (rank 0)
     // recompresses exactly the columns of D, i.e. computes its truncated SVD.
@@ -1085,7 +1086,7 @@ extern "C" int hcgb_compress_tiles(hcgb_context *ctx, int count, const double *c
         if (dinfo) cudaFree(dinfo);
         return rc;
     };
-    const bool direct = compress_direct(ctx, params);
+    const bool direct = compress_direct(ctx, params, rows, cols);
     if (!direct) {
         if (cudaMalloc(&ibuf, sizeof(double) * 2 * n * n) != cudaSuccess ||
             cudaMalloc(&irank, sizeof(int)) != cudaSuccess)
