@@ -8,7 +8,7 @@ error-free splitting, error below FP64's own worst-case bound).
 
 Other forms, each timed in the same process on the same inputs and reported in "forms" with its
 own value, e2e, product error and speed-up over the plain form:
-  mixed_ff48 : the stack QR, the pivoted QR of cores up to 117 columns and the Q application in
+  mixed_ff48 : the stack QR, the pivoted QR of cores up to 114 columns and the Q application in
                float-float arithmetic (two floats, 48-bit significand) on the FP32 pipe.
 
 Workload (default): n = 16384, nb = 512 -> 32 x 32 tiles, Morton-sorted 2-D points,

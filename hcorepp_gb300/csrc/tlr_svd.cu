@@ -876,9 +876,13 @@ __device__ int jacobi32_cross(const TM &tm, float4 *Y, int ls4, int x4, int j4, 
     return rotations;
 }
 
-// Stack widths up to which a core fits a quarter and half of an SM's shared memory: the sweep's order and lanes per pair
-// go by the width, not by the team that a launch gives the update.
-constexpr int SMALL_K = 82, LIGHT_K = 117;
+// Columns of the preconditioner's working matrix (x4 quads of X above j4 of J): a length of 4 mod 8 quads, so that two
+// 4-lane groups, a quarter-warp, meet no bank conflict.
+__host__ __device__ constexpr int precond_quads(int x4, int j4) { return ((x4 + j4 + 3) & ~7) + 4; }
+
+// Stack width up to which a core gets eight lanes a pair from 33 columns on, and not from 65: about a quarter of an SM's
+// shared memory.  A width, not the team that a launch gives the update.
+constexpr int SMALL_K = 82;
 constexpr int SWEEP_BLOCKS = 2 * WIDE_CTAS;  // column blocks of a core that a cluster can hold two at a time a CTA
 constexpr int BLOCK_G16_QUADS = 42;          // up to 168 rows (and as many columns, eleven a block)
 
@@ -1508,7 +1512,7 @@ __device__ __forceinline__ int core_aux_doubles(const Workspace &ws, int slot) {
 }
 
 // CTA of SVD_THREADS threads, in one of three team layouts chosen by the update's stack width k: heavy (k > k_heavy:
-// the core needs more than half of the shared memory) — the whole CTA; light
+// more than half of the shared memory, the preconditioner's columns included) — the whole CTA; light
 // (kthr4 < k <= k_heavy) — two half-CTA teams of SVD_THREADS / 2 threads, one update each, each with half
 // of the shared memory and its own named barrier; small (k <= kthr4: the core fits a quarter) — four teams
 // of SVD_THREADS / 4 threads.  Small cores are latency-bound (per-step barriers, dependent FP64 chains), so
@@ -1771,8 +1775,8 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
             b.ldv = 4 * b.ls4;
             fits = 4 * (size_t) b.ls4 * rk <= (size_t) ws.kmax * (ws.kmax + ws.ld) && 2 * b.ls4 <= b.buf_quads;
         } else {
-            b.ls4 = ((x4 + j4 + 3) & ~7) + 4;  // 4 mod 8 quads: two 4-lane groups a quarter-warp, no bank conflicts
-            b.blocks = k > LIGHT_K ? SWEEP_BLOCKS : 0;
+            b.ls4 = precond_quads(x4, j4);
+            b.blocks = k > ws.k_heavy ? SWEEP_BLOCKS : 0;  // as on a cluster
             b.g8 = rk <= (k <= SMALL_K ? 32 : 64);
             const int skip = (int) ((reinterpret_cast<uintptr_t>(pool) >> 3) & 1);
             b.y = reinterpret_cast<float4 *>(pool + skip);
@@ -1815,8 +1819,9 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         sweeps = -sweeps;  // the corrections left orthogonal columns
     } else {
         int more = 0;
+        // on a cluster, a core that one SM could hold takes that SM's lanes per pair
         jacobi_dispatch<RPL>(tm, X, ldx, kV, rk, nrm, &s_rot, &s_amax, &more, &converged, tol64, MAX_JACOBI_SWEEPS, dsc,
-                             ka, Mw == pool);
+                             ka, CLUSTER ? k <= ws.k_wide : Mw == pool);
         sweeps += more;
     }
 
@@ -1940,19 +1945,24 @@ size_t svd_smem_bytes(int kmax) { return 2 * sizeof(double) * (size_t) svd_team_
 // Register tiles of the FP64 sweeps: up to 16 rows a lane (longer columns take the looped sweep).
 constexpr int CORE_RPL = 16;
 
-// A core of k columns takes its aux arrays, 6 k + SVD_AUX_FIXED doubles, and a k x k working copy.  A 110-column core
+// A core of k columns takes its aux arrays, 6 k + SVD_AUX_FIXED doubles, and a k x k working copy; in half an SM and in a
+// whole one, where a cluster may do the same work, the preconditioner's padded columns too (one double aligns
+// them).  A 110-column core
 // of width 128 takes a cluster of eight 4,300 kcycles and one SM alone 7,900: heavy ones go to clusters only
 // while SMs are idle, wide ones always.
 void core_classes(int kmax, int *whole, int *half, int *quarter) {
     const int team = svd_team_doubles(kmax);
-    auto widest = [](long doubles) {
+    auto widest = [](long doubles, bool padded) {
         int k = 0;
-        while ((k + 1L) * (k + 1L) + 6 * (k + 1L) + SVD_AUX_FIXED <= doubles) k++;
-        return k;
+        while (true) {
+            const long c = k + 1, q = (c + 3) / 4;
+            if ((padded ? 2 * precond_quads(q, q) * c + 1 : c * c) + 6 * c + SVD_AUX_FIXED > doubles) return k;
+            k++;
+        }
     };
-    *whole = widest(2 * team);
-    *half = widest(team);
-    *quarter = widest(team / 2);
+    *whole = widest(2 * team, true);
+    *half = widest(team, true);
+    *quarter = widest(team / 2, false);
 }
 
 static void launch_core_wide(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {

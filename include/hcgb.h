@@ -70,7 +70,7 @@ typedef struct {
 
 /* HCGB_PLAIN_FP64: the recompression (stack QR, core SVD, Q application) in double precision (the core SVD
  * finds its rotations in single precision and finishes the columns to FP64 working precision).
- * HCGB_MIXED: the stack QR, the pivoted QR of cores up to 117 columns and the panel-wise Q
+ * HCGB_MIXED: the stack QR, the pivoted QR of cores up to 114 columns and the panel-wise Q
  * application in float-float arithmetic (a value is the unevaluated sum of two floats, 48-bit
  * significand) on the FP32 pipe, each block scaled by an exact power of two first; the core
  * product, the new factors, the truncation test and all factor products stay in double precision.

@@ -115,6 +115,42 @@ def test_results_do_not_depend_on_the_number_of_updates(T, rc, ra):
 
 
 @pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("close", [False, True])
+@pytest.mark.parametrize("k", [113, 114, 115, 116, 117, 118, 165, 166, 167, 168])
+def test_heavy_cores_do_not_depend_on_the_team(T, k, close, mode):
+    """One update, alone and among 19, 20 and 40: heavy cores run on clusters up to 19 updates and on one SM each
+    beyond, at widths around half an SM's shared memory and a whole one's.  With close, groups of nearly equal
+    singular values; without, a core of full rank."""
+    import torch
+    from hcorepp_gb300 import _lib as L
+    rng = np.random.default_rng([k, close, mode])
+    n, ra = 203, k // 2
+    rc = k - ra
+    q = lambda r: np.linalg.qr(rng.standard_normal((n, r)))[0]
+    sigma = lambda r: (np.repeat(np.logspace(0, -9, (r + 4) // 5), 5)[:r] * (1.0 + 1e-7 * np.arange(r)) if close
+                       else np.logspace(0, -6, r))
+    cu, cv = q(rc), sigma(rc)[:, None] * q(rc).T
+    au, av, bu, bv = q(ra), sigma(ra)[:, None] * q(ra).T, q(ra), q(ra).T
+    p, first = T.CompressionParameters(1e-8, truncated_svd=True, mode=mode).c(), None
+    for count in (1, 19, 20, 40):
+        a, b = T.CompressedTile(n, n, au, av, max_rank=k), T.CompressedTile(n, n, bu, bv, max_rank=k)
+        cs = [T.CompressedTile(n, n, cu, cv, max_rank=k) for _ in range(count)]
+        ups = (L.Update * count)(*[L.Update(a.c_tile(), b.c_tile(), c.c_tile()) for c in cs])
+        ctx = T.run_context()
+        ctx.check(L.lib().hcgb_gemm_batch(ctx.handle, 1.0, 1.0, count, ups, C.byref(p), None))
+        torch.cuda.synchronize()
+        got = [(c.rank, c.u(), c.v()) for c in cs]
+        first = first or got[0]
+        for r, u, v in got:
+            assert r == first[0]
+            np.testing.assert_array_equal(u, first[1])
+            np.testing.assert_array_equal(v, first[2])
+    d = cu @ cv + au @ (av @ bu) @ bv
+    # at most k dropped singular values of up to 1e-8 of the largest, and the pivoted QR's share of 1e-2 of that
+    assert rel_fro(first[1] @ first[2], d) <= 1.02e-8 * np.sqrt(k)
+
+
+@pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("m,n", [(1, 1), (5, 40), (40, 5), (100, 100), (131, 90), (90, 131), (300, 257)])
 def test_compression_of_rectangular_tiles(T, m, n, mode):
     rng = np.random.default_rng([m, n])
