@@ -1094,8 +1094,10 @@ __device__ __forceinline__ void reflect_column(bool act, double *y, const double
 }
 
 // (value, index) with the largest value over a warp, ties to the lower index; values are the bits of
-// non-negative doubles, ordered like them (a NaN is never chosen).
-constexpr long long NRM_MAX_BITS = 0x7ff0000000000000LL;
+// non-negative doubles, ordered like them, a NaN above all.  A norm that is not finite is the first pivot, whose
+// reflector makes every column NaN; behind the first step it ends the factorisation (a core with a NaN or
+// an infinity gives a rank-1 tile of NaN).
+constexpr long long NRM_INF_BITS = 0x7ff0000000000000LL, NRM_SIGN_MASK = 0x7fffffffffffffffLL;
 __device__ __forceinline__ void warp_argmax(long long &v, int &i) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1138,8 +1140,7 @@ __device__ int qrcp_steps(const TM &tm, double *A, int lda, int mrows, int ncols
             int bi = ncols, at = s;  // the largest norm's column (ties to the lower one) and its place in pvt
             for (int j = s + lane; j < ncols; j += 32) {
                 const int c = pvt[j];
-                long long v = __double_as_longlong(nrm[c]);
-                if (v > NRM_MAX_BITS) v = -1;
+                const long long v = __double_as_longlong(nrm[c]) & NRM_SIGN_MASK;
                 if (v > bv || (v == bv && c < bi)) {
                     bv = v;
                     bi = c;
@@ -1153,7 +1154,7 @@ __device__ int qrcp_steps(const TM &tm, double *A, int lda, int mrows, int ncols
             }
             const double top = bv < 0 ? 0.0 : __longlong_as_double(bv);
             if (s == 0 && stop2 == 0.0 && rel > 0.0) lim = rel * rel * top;
-            const bool stop = top <= lim || top <= 0.0;
+            const bool stop = bv >= NRM_INF_BITS ? s > 0 : (top <= lim || top <= 0.0);
             if (!stop) {
                 const int cs = bi;
                 __syncwarp();
@@ -1271,8 +1272,7 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
             int bi = ncols;
             for (int q = lane; q < nact; q += 32) {
                 const int c = act_list[q], j = rank + c * C;
-                long long v = __double_as_longlong(nrm[c]);
-                if (v > NRM_MAX_BITS) v = -1;
+                const long long v = __double_as_longlong(nrm[c]) & NRM_SIGN_MASK;
                 if (v > bv || (v == bv && j < bi)) {
                     bv = v;
                     bi = j;
@@ -1290,7 +1290,7 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
         warp_argmax(bv, bi);
         const double top = bv < 0 ? 0.0 : __longlong_as_double(bv);
         if (s == 0 && stop2 == 0.0 && rel > 0.0) lim = rel * rel * top;
-        if (top <= lim || top <= 0.0) {
+        if (bv >= NRM_INF_BITS ? s > 0 : (top <= lim || top <= 0.0)) {
             rk = s;
             break;
         }
@@ -1394,7 +1394,7 @@ __device__ __forceinline__ void qrcp_apply_df(const TM &tm, df *A, int lda, int 
 // near 1: same pivoting, early stop (stop2 on squared norms; stop2 == 0 with rel2 > 0 sets
 // stop2 = rel2 * |r_00|^2 after the first pivot; stop2 < 0 disables it) and norm downdating with
 // exact recomputation when a downdate cancels.  Pivot keys are the float norms' bit patterns
-// (non-negative floats order like their bits).
+// (non-negative floats order like their bits; a NaN above all, as in the FP64 form).
 template <class TM>
 __device__ int qrcp_truncated_df(const TM &tm, df *A, int lda, int mrows, int ncols, float stop2, float rel2, df *nrm, df *nref,
                                  int *pvt, float *red, int *redi) {
@@ -1414,7 +1414,7 @@ __device__ int qrcp_truncated_df(const TM &tm, df *A, int lda, int mrows, int nc
         int bv = -1, bi = s;  // float bits of the largest remaining squared norm (first warp only)
         if (warp == 0) {
             for (int j = s + lane; j < ncols; j += 32) {
-                const int v = __float_as_int(nrm[j].h);
+                const int v = __float_as_int(nrm[j].h) & 0x7fffffff;
                 if (v > bv) {
                     bv = v;
                     bi = j;
@@ -1438,7 +1438,7 @@ __device__ int qrcp_truncated_df(const TM &tm, df *A, int lda, int mrows, int nc
         const float bvf = __int_as_float(redi[64]);
         bi = redi[65];
         const float lim = red[33];
-        if (bvf <= lim || bvf <= 0.f) {
+        if (!isfinite(bvf) ? s > 0 : (bvf <= lim || bvf <= 0.f)) {
             rkeep = s;
             break;
         }
@@ -1832,7 +1832,9 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         double t = 0.0;
         for (int r = lane; r < kV; r += 32) t = fma(col[r], col[r], t);
         t = warp_sum(t);
-        if (lane == 0) inv[j] = sqrt(t);  // unsorted sigma, temporarily in inv[]
+        // unsorted sigma, temporarily in inv[]; -1 for a NaN, so that the order below is total and perm a
+        // permutation whatever the columns hold
+        if (lane == 0) inv[j] = t >= 0.0 ? sqrt(t) : -1.0;
     }
     tm.sync();
     for (int j = tm.tid; j < rk; j += tm.nth) {
@@ -1843,7 +1845,7 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
             pos += (sl > sj) || (sl == sj && l < j);
         }
         perm[pos] = j;
-        sig[pos] = sj;
+        sig[pos] = sj < 0.0 ? __longlong_as_double(NRM_SIGN_MASK) : sj;
     }
     tm.sync();
     if (tm.tid == 0) {

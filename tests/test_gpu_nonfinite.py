@@ -1,0 +1,65 @@
+"""Inputs with a NaN or an infinity: a compressed result is a rank-1 tile of NaN, whatever the core's width and
+form, and the other tiles of the batch do not notice."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def T():
+    import torch
+    assert torch.cuda.is_available()
+    from hcorepp_gb300 import tiles
+    return tiles
+
+
+def _tile(rng, m, n):
+    r = min(m, n)
+    return (np.linalg.qr(rng.standard_normal((m, r)))[0] * np.logspace(0, -4, r)) @ np.linalg.qr(
+        rng.standard_normal((n, r)))[0].T
+
+
+def _compress(T, tiles, mode):
+    import torch
+    m, n = tiles[0].shape
+    out = [T.CompressedTile(m, n, rank=0, max_rank=min(m, n)) for _ in tiles]
+    ranks = T.CompressedTile.compress_batch([torch.from_numpy(t.ravel(order="F").copy()).cuda() for t in tiles], out,
+                                            T.CompressionParameters(1e-8, truncated_svd=True, mode=mode))
+    return [(r, t.u(), t.v()) for r, t in zip(ranks, out)]
+
+
+# Teams of the core: FP64 sweeps alone (12), a quarter and half an SM (40, 100), an SM and a cluster (150 among 20 and
+# among 3), clusters (200), both orders of a rectangle.
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("m,n,count", [(1, 1, 3), (12, 12, 3), (40, 40, 5), (100, 100, 3), (150, 150, 20), (150, 150, 3),
+                                       (200, 200, 3), (60, 100, 3), (200, 130, 3)])
+def test_compression_of_a_tile_with_a_nonfinite_entry(T, m, n, count, value, mode):
+    rng = np.random.default_rng([m, n, count])
+    tiles = [_tile(rng, m, n) for _ in range(count)]
+    want = _compress(T, tiles, mode)
+    tiles[1][(2 * m) // 3, n // 2] = value
+    got = _compress(T, tiles, mode)
+    assert got[1][0] == 1
+    assert np.isnan(got[1][1] @ got[1][2]).all()
+    for i in [0] + list(range(2, count)):
+        assert got[i][0] == want[i][0]
+        np.testing.assert_array_equal(got[i][1], want[i][1])
+        np.testing.assert_array_equal(got[i][2], want[i][2])
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n,r", [(40, 6), (96, 20), (200, 55), (256, 90)])
+def test_update_of_a_tile_with_a_nan(T, n, r, mode):
+    rng = np.random.default_rng([n, r])
+    q = lambda: np.linalg.qr(rng.standard_normal((n, r)))[0]
+    sigma = np.logspace(0, -6, r)[:, None]
+    cu = q()
+    cu[n // 3, r // 2] = np.nan
+    c = T.CompressedTile(n, n, cu, sigma * q().T, max_rank=n)
+    a = T.CompressedTile(n, n, q(), sigma * q().T, max_rank=r)
+    b = T.CompressedTile(n, n, q(), q().T, max_rank=r)
+    T.HCore.Gemm(1.0, a, 0, b, 0, 1.0, c, T.CompressionParameters(1e-8, truncated_svd=True, mode=mode))
+    assert c.rank == 1
+    assert np.isnan(c.to_dense()).all()
