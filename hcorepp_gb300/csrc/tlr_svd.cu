@@ -1036,19 +1036,21 @@ __device__ bool jacobi_precond(const TM &tm, const double *X, int ldx, int rows,
     return true;
 }
 
-// A step's reflector H = I - gamma v v^T for the pivot column x (rows s ..), v = [alpha - beta; x_{s+1}, ..]
-// (dlarfg's beta, v not normalised: only R is kept).  sigma = ||x_{s+1..}||^2.  One reciprocal square root and
-// one reciprocal: every FP64 instruction of this chain holds up the whole team.
+// A step's reflector H = I - tau v v^T for the pivot column x (rows s ..), v = [1; scale x_{s+1}, ..] (dlarfg's
+// beta and tau; x stays as it is: only R is kept).  sigma = ||x_{s+1..}||^2.  One reciprocal square root and one
+// reciprocal: every FP64 instruction of this chain holds up the whole team.  tau and scale stay in range
+// wherever sigma is not zero; 2 / ||x||^2 in one number, an instruction less a column, overflows for columns
+// below 7e-155.
 struct Reflector {
-    double beta, vs, gamma;
+    double beta, tau, scale;
 };
 __device__ __forceinline__ Reflector make_reflector(double alpha, double sigma) {
     Reflector h{alpha, 0.0, 0.0};
     if (sigma != 0.0) {
-        const double q = fma(alpha, alpha, sigma), r = rsqrt(q), nrm = q * r, d = nrm + fabs(alpha);
+        const double q = fma(alpha, alpha, sigma), r = rsqrt(q), nrm = q * r;
         h.beta = -copysign(nrm, alpha);
-        h.vs = copysign(d, alpha);       // alpha - beta
-        h.gamma = r * __drcp_rn(d);      // 2 / ||v||^2 = 1 / (nrm (nrm + |alpha|))
+        h.tau = fma(fabs(alpha), r, 1.0);                            // (beta - alpha) / beta
+        h.scale = copysign(__drcp_rn(nrm + fabs(alpha)), alpha);     // 1 / (alpha - beta)
     }
     return h;
 }
@@ -1060,16 +1062,18 @@ template <int G>
 __device__ __forceinline__ void reflect_column(bool act, double *y, const double *x, const Reflector &h, int s,
                                                int mrows, int gl, double *nrm, double *nref) {
     double w = 0.0;
-    if (act && h.gamma != 0.0) {
-        w = gl == 0 ? h.vs * y[s] : 0.0;
+    if (act && h.tau != 0.0)
         for (int i = s + 1 + gl; i < mrows; i += G) w = fma(x[i], y[i], w);
-    }
-    w = group_sum(w, G) * h.gamma;
+    w = group_sum(w, G);
     double ys = 0.0;
     if (act) {
-        ys = fma(-w, h.vs, y[s]);  // every lane of the group reads the old y[s] before lane 0 writes it
-        if (h.gamma != 0.0)
-            for (int i = s + 1 + gl; i < mrows; i += G) y[i] = fma(-w, x[i], y[i]);
+        ys = y[s];  // every lane of the group reads the old y[s] before lane 0 writes it
+        if (h.tau != 0.0) {
+            w = fma(w, h.scale, ys) * h.tau;
+            ys -= w;
+            const double t = w * h.scale;
+            for (int i = s + 1 + gl; i < mrows; i += G) y[i] = fma(-t, x[i], y[i]);
+        }
     }
     __syncwarp();
     double nn = 0.0;
@@ -1169,8 +1173,8 @@ __device__ int qrcp_steps(const TM &tm, double *A, int lda, int mrows, int ncols
                 const Reflector h = make_reflector(x[s], t);
                 __syncwarp();
                 if (lane == 0) {
-                    red[0] = h.vs;
-                    red[1] = h.gamma;
+                    red[0] = h.tau;
+                    red[1] = h.scale;
                     x[s] = h.beta;
                     redi[1] = cs;
                 }
@@ -1242,7 +1246,7 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
     double *nref = nrm + nlmax;
     double *xb = nref + nlmax;                      // the pivot column
     double *diag = xb + mrows;                      // beta of every step
-    double *red = diag + mrows;                     // vs, gamma
+    double *red = diag + mrows;                     // tau, scale
     long long *cv = reinterpret_cast<long long *>(red + 4);  // candidates of the CTAs, two steps' worth
     int *ci = reinterpret_cast<int *>(cv + 2 * C);
     int *act_list = ci + 2 * C;                     // local columns not chosen yet
@@ -1308,8 +1312,8 @@ __device__ int qrcp_cluster(const TM &tm, const double *M, int ldm, int mrows, i
             __syncwarp();
             const Reflector h = make_reflector(xb[s], t);
             if (lane == 0) {
-                red[0] = h.vs;
-                red[1] = h.gamma;
+                red[0] = h.tau;
+                red[1] = h.scale;
                 diag[s] = h.beta;
                 taken[bi] = 1;
                 if (rank == 0) pvt[s] = bi;

@@ -63,3 +63,15 @@ def test_update_of_a_tile_with_a_nan(T, n, r, mode):
     T.HCore.Gemm(1.0, a, 0, b, 0, 1.0, c, T.CompressionParameters(1e-8, truncated_svd=True, mode=mode))
     assert c.rank == 1
     assert np.isnan(c.to_dense()).all()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [12, 40, 100, 200])
+@pytest.mark.parametrize("e", [-505, -512, -530])
+def test_compression_of_tiny_tiles_stays_finite(T, n, e, mode):
+    """Squared column norms in the subnormal range.  Singular values of at most 1e-150 (2^-498) count as zero: such a
+    tile is dropped, to the last bit."""
+    d = _tile(np.random.default_rng([n, -e]), n, n) * 2.0 ** e
+    t = T.CompressedTile.from_dense(d, T.CompressionParameters(1e-5, truncated_svd=True, mode=mode), max_rank=n)
+    assert np.isfinite(t.u()).all() and np.isfinite(t.v()).all()
+    assert not t.to_dense().any()
