@@ -1603,6 +1603,36 @@ __global__ void __cluster_dims__(WIDE_CTAS, 1, 1) __launch_bounds__(SVD_THREADS,
     if ((int) (blockIdx.x / WIDE_CTAS) < H) tm.sync();  // no CTA leaves while another reads its shared memory
 }
 
+// Exponent of the largest entry of X (rows x cols), within +-1000 so that 2^e and 2^-e are normal (0 for a zero X).
+template <class TM>
+__device__ int core_exponent(const TM &tm, const double *X, int ldx, int rows, int cols, int *s_emax) {
+    if (tm.tid == 0) *s_emax = 0;
+    tm.sync();
+    int em = 0;
+    for (int j = tm.warp(); j < cols; j += tm.nw())
+        for (int r = threadIdx.x & 31; r < rows; r += 32) {
+            const int f = (int) ((__double_as_longlong(X[r + (size_t) j * ldx]) >> 52) & 0x7ff);
+            em = em > f ? em : f;
+        }
+    for (int o = 16; o > 0; o >>= 1) {
+        const int f = __shfl_xor_sync(0xffffffffu, em, o);
+        em = em > f ? em : f;
+    }
+    if ((threadIdx.x & 31) == 0) atomicMax(s_emax, em);
+    tm.sync();
+    const int e = *s_emax ? *s_emax - 1023 : 0;
+    return e < -1000 ? -1000 : (e > 1000 ? 1000 : e);
+}
+
+// X (rows x cols) <- X 2^e.
+template <class TM>
+__device__ void scale_columns(const TM &tm, double *X, int ldx, int rows, int cols, int e) {
+    const double f = __hiloint2double((1023 + e) << 20, 0);
+    for (int j = tm.warp(); j < cols; j += tm.nw())
+        for (int r = threadIdx.x & 31; r < rows; r += 32) X[r + (size_t) j * ldx] *= f;
+    tm.sync();
+}
+
 // The recompression core of one update (slot) by one team: auxiliary arrays at sm, `pool_doubles` of shared
 // memory at pool (a cluster: of every CTA's own).
 template <int RPL, class TM>
@@ -1823,9 +1853,15 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
         sweeps = -sweeps;  // the corrections left orthogonal columns
     } else {
         int more = 0;
+        // The sweeps' tests multiply squared norms with one another: columns far from 1 (a^2 below ~1e-300 or above
+        // 1e300, with the factors tol^2 and noise^2 between them) are scaled by an exact power of two for them.
+        const int e = core_exponent(tm, X, ldx, kV, rk, &s_emax);
+        const bool scaled = e < -150 || e > 150;
+        if (scaled) scale_columns(tm, X, ldx, kV, rk, -e);
         // on a cluster, a core that one SM could hold takes that SM's lanes per pair
         jacobi_dispatch<RPL>(tm, X, ldx, kV, rk, nrm, &s_rot, &s_amax, &more, &converged, tol64, MAX_JACOBI_SWEEPS, dsc,
                              ka, CLUSTER ? k <= ws.k_wide : Mw == pool);
+        if (scaled) scale_columns(tm, X, ldx, kV, rk, e);
         sweeps += more;
     }
 

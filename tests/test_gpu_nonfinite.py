@@ -75,3 +75,19 @@ def test_compression_of_tiny_tiles_stays_finite(T, n, e, mode):
     t = T.CompressedTile.from_dense(d, T.CompressionParameters(1e-5, truncated_svd=True, mode=mode), max_rank=n)
     assert np.isfinite(t.u()).all() and np.isfinite(t.v()).all()
     assert not t.to_dense().any()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [5, 12, 15, 40, 100, 200])
+@pytest.mark.parametrize("e", [-470, -300, -250, 300])
+def test_compression_does_not_depend_on_the_scale(T, n, e, mode):
+    """Far from 1 (the squares of squared norms leave the range) as near it: a power of two changes no digit of the
+    sweeps.  Smaller squared norms than 2^-960 (e = -470, entries down to 1e-8 of the top) may lose digits in the
+    subnormal range, which moves singular values by at most 1e-150 each."""
+    d = _tile(np.random.default_rng([n, 1]), n, n)
+    p = T.CompressionParameters(1e-5, truncated_svd=True, mode=mode)
+    near = T.CompressedTile.from_dense(d, p, max_rank=n)
+    far = T.CompressedTile.from_dense(d * 2.0 ** e, p, max_rank=n)
+    assert far.rank == near.rank
+    err = np.linalg.norm(far.to_dense() * 2.0 ** -e - d) / np.linalg.norm(d)
+    assert err <= 1.02e-5 * np.sqrt(n) + n * max(1e-150 * 2.0 ** -e, 1e-13) / np.linalg.norm(d)
