@@ -17,7 +17,8 @@
 //     max|A_i| max|B_j| per k, under FP64's own worst-case bound); every 128 k the eight level
 //     accumulators are read out of tensor memory and added into two 64-bit integers (levels 0-3 and
 //     4-7, each shifted to a common scale), which stay exact for k up to 2^16, and the tile ends with
-//     C_ij = 2^(e_i + f_j) (hi 2^-35 + lo 2^-63).
+//     C_ij = 2^(e_i + f_j) (hi 2^-35 + lo 2^-63);
+//   * outputs of a row or column that holds a NaN or an infinity are FP64 products.
 // Tensor memory holds the eight level accumulators of a 128 x 64 output tile (512 columns).  The sixteen warps cut
 // 32-wide K chunks into digit planes, two shared-memory stages in turn, and read the accumulators out; a thread of the
 // last one issues the 72 MMAs (36 pairs x 2 k-steps of 16) of a chunk when it is filled.  They meet on mbarriers
@@ -58,6 +59,7 @@ constexpr int OZ_STAGE = OZ_S * (OZ_A_PLANE + OZ_B_PLANE);  // 96 KB
 constexpr int OZ_SMEM = 2 * OZ_STAGE + 1024;
 constexpr int OZ_TMEM_COLS = OZ_S * OZ_TN;  // 512: one 64-column accumulator per level
 constexpr int OZ_NOGROUP = -1100;       // exponent of an all-zero group
+constexpr int OZ_NONFINITE = 1 << 20;   // exponent of a group with a NaN or an infinity (cut to zeros)
 
 __device__ unsigned int g_oz_wait_timeouts = 0;
 
@@ -225,9 +227,13 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     exponents(std::true_type{}, rows, ea);
     exponents(std::false_type{}, cols, eb);
     __syncthreads();
-    if (tid < OZ_TM) ea[tid] = ea[tid] ? ea[tid] - 1022 : OZ_NOGROUP;
-    else if (tid < OZ_TM + OZ_TN) eb[tid - OZ_TM] = eb[tid - OZ_TM] ? eb[tid - OZ_TM] - 1022 : OZ_NOGROUP;
-    __syncthreads();
+    bool special = false;
+    if (tid < OZ_TM + OZ_TN) {
+        int &e = tid < OZ_TM ? ea[tid] : eb[tid - OZ_TM];
+        special = e == 0x7ff;
+        e = special ? OZ_NONFINITE : (e ? e - 1022 : OZ_NOGROUP);
+    }
+    const bool nonfinite = __syncthreads_or(special);
 
     // This thread's share of the read-out: TMEM lanes 32 (warp % 4) .. (rows), columns 16 (warp / 4) ..
     const int q = warp & 3, h = warp >> 2;
@@ -329,10 +335,11 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
 #pragma unroll
         for (int j = 0; j < 16; j++) {
             const int cl = h * 16 + j;
-            if (cl < cols) {
+            const int eab = cl < cols ? ea[row_l] + eb[cl] : OZ_NONFINITE;
+            if (eab < OZ_NONFINITE / 2) {
                 double *cp = jb.C + m0 + row_l + (size_t) (n0 + cl) * jb.ldc;
                 double v = 0.0;
-                if (jb.K > 0) v = oz_value((long long) (hi[j] - constant), (long long) (lo[j] - constant), ea[row_l] + eb[cl]);
+                if (jb.K > 0) v = oz_value((long long) (hi[j] - constant), (long long) (lo[j] - constant), eab);
                 if (negate) v = -v;
                 if (scale) v *= jb.alpha;
                 if (accum) v = fma(jb.beta, *cp, v);
@@ -340,6 +347,18 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
             }
         }
     }
+    // Outputs of a row or column with a NaN or an infinity, as an FP64 product gives them.
+    if (nonfinite)
+        for (int e = tid; e < rows * cols; e += OZ_THREADS) {
+            const int r = e % rows, c = e / rows;
+            if (ea[r] + eb[c] < OZ_NONFINITE / 2) continue;
+            double v = 0.0;
+            for (int k = 0; k < jb.K; k++) v = fma(job_a(jb, m0 + r, k), job_b(jb, k, n0 + c), v);
+            double *cp = jb.C + m0 + r + (size_t) (n0 + c) * jb.ldc;
+            v *= jb.alpha;
+            if (jb.beta != 0.0) v = fma(jb.beta, *cp, v);
+            *cp = v;
+        }
     __syncthreads();  // ea / eb are rewritten by the next tile
 }
 

@@ -91,3 +91,49 @@ def test_compression_does_not_depend_on_the_scale(T, n, e, mode):
     assert far.rank == near.rank
     err = np.linalg.norm(far.to_dense() * 2.0 ** -e - d) / np.linalg.norm(d)
     assert err <= 1.02e-5 * np.sqrt(n) + n * max(1e-150 * 2.0 ** -e, 1e-13) / np.linalg.norm(d)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1)])
+@pytest.mark.parametrize("m,n,k", [(8, 8, 8), (16, 16, 16), (40, 30, 33), (45, 45, 200), (130, 70, 129)])
+def test_products_carry_nonfinite_entries(T, m, n, k, ta, tb):
+    """A NaN reaches its row and column of the product, an infinity too (NaN where it meets a zero); every other
+    output is that of the same product without them."""
+    import torch
+    rng = np.random.default_rng([m, n, k])
+    a, b, c = rng.standard_normal((m, k)), rng.standard_normal((k, n)), rng.standard_normal((m, n))
+    b[k // 2, n // 3] = 0.0
+
+    def gemm(a, b):
+        ta_, tb_ = a.T if ta else a, b.T if tb else b
+        g = T.DenseTile(m, n, c)
+        T.HCore.Gemm(-1.5, T.DenseTile(*ta_.shape, ta_), ta, T.DenseTile(*tb_.shape, tb_), tb, 0.5, g,
+                     T.CompressionParameters(1e-8))
+        return g.to_dense()
+
+    want = gemm(a, b)
+    a2, b2 = a.copy(), b.copy()
+    a2[m // 2, k // 2] = np.inf
+    a2[0, k - 1] = np.nan
+    b2[0, n - 1] = -np.inf
+    with np.errstate(invalid="ignore"):
+        special = -1.5 * (a2 @ b2) + 0.5 * c
+    got = gemm(a2, b2)
+    finite = np.isfinite(special)
+    np.testing.assert_array_equal(got[finite], want[finite])
+    np.testing.assert_array_equal(got[~finite], special[~finite])
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n,r", [(64, 17), (128, 40)])
+def test_update_with_a_nan_in_a_factor_of_a(T, n, r, mode):
+    """The NaN enters by the factor products."""
+    rng = np.random.default_rng([n, r])
+    q = lambda: np.linalg.qr(rng.standard_normal((n, r)))[0]
+    av = np.logspace(0, -6, r)[:, None] * q().T
+    av[r // 2, n // 3] = np.nan
+    a = T.CompressedTile(n, n, q(), av, max_rank=r)
+    b = T.CompressedTile(n, n, q(), q().T, max_rank=r)
+    c = T.CompressedTile(n, n, q(), q().T, max_rank=n)
+    T.HCore.Gemm(1.0, a, 0, b, 0, 1.0, c, T.CompressionParameters(1e-8, truncated_svd=True, mode=mode))
+    assert c.rank == 1
+    assert np.isnan(c.to_dense()).all()
