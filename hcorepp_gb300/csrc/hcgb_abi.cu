@@ -1514,7 +1514,7 @@ extern "C" int hcgb_dgemm(hcgb_context *ctx, int transa, int transb, int m, int 
     j.opB = transb;
     j.alpha = alpha;
     j.beta = beta;
-    j.oz = (ctx->oz && oz_shape(m, n, k, ctx->oz_min)) ? 1 : 0;
+    j.oz = (ctx->oz && oz_shape(m, n, k, std::max(ctx->oz_min, OZ_MIN_OUTPUTS_DENSE))) ? 1 : 0;
     const size_t jb = (sizeof(GemmJob) + 255) / 256 * 256;
     int rc = ensure_device(ctx, &ctx->desc, &ctx->desc_bytes, jb + sizeof(int) * 16);
     if (rc) return rc;

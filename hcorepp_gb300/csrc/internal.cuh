@@ -178,6 +178,10 @@ __device__ __forceinline__ int job_of_tile(const int *sched, int njobs, int w) {
 // K = 64: 85 and 58), a 32 x 32 one is 2 and 1.2 times faster here.  Multiplies 11x11 nb=301, n=16384 and n=8192 at 1e-4:
 // 68.5, 707 and 58.9 ms from 256 outputs and 24 reflectors on, 72.7, 719 and 61.0 from 2048 and 48 on.
 constexpr int OZ_MIN_OUTPUTS = 256;
+// The least for the products of an update with a dense C and for hcgb_dgemm: the split's error is relative to the
+// row's and the column's maximum, an FP64 product's to the terms of each output.  Recompression truncates relative to
+// the tile's norm; these results are the caller's as they are.
+constexpr int OZ_MIN_OUTPUTS_DENSE = 2048;
 __host__ __device__ inline bool oz_shape(int M, int N, int K, int min_outputs = OZ_MIN_OUTPUTS) {
     return K >= 16 && M >= 16 && N >= 8 && (long long) M * N >= min_outputs;
 }

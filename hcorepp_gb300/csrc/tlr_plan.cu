@@ -45,10 +45,11 @@ __global__ void plan_kernel(const DevUpdate *ups, int n, double alpha, double be
     // Low-precision forms: every product on tcgen05 in TF32 / BF16; otherwise the large products go
     // to the FP64-accurate tensor-core path.
     const int lp = lowp_prec(p.mode);
+    const int oz_min = !ups[s].c.kind && p.oz_min < OZ_MIN_OUTPUTS_DENSE ? OZ_MIN_OUTPUTS_DENSE : p.oz_min;
     for (int ph = 0; ph < 3; ph++) {
         GemmJob &j = jobs[(size_t) ph * n + s];
         j.prec = (lp && j.M > 0 && j.N > 0) ? lp : 0;
-        j.oz = (!j.prec && p.oz && j.M > 0 && j.N > 0 && oz_shape(j.M, j.N, j.K, p.oz_min)) ? 1 : 0;
+        j.oz = (!j.prec && p.oz && j.M > 0 && j.N > 0 && oz_shape(j.M, j.N, j.K, oz_min)) ? 1 : 0;
     }
 }
 

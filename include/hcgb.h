@@ -177,10 +177,12 @@ int hcgb_set_k_order(hcgb_context *ctx, int policy);
 int hcgb_set_graph(hcgb_context *ctx, int enable);
 
 /* Tuning knobs of the batched pipeline (chosen by hcorepp_gb300/autotune.py per tile size and
- * stack-width class; results do not depend on them beyond rounding): a factor product goes to the
- * FP64-accurate tensor-core path when it has at least oz_min_outputs outputs (default 256, with
- * K >= 16, M >= 16, N >= 8), and in the plain form a side's Q is applied in WY form when it has at
- * least wy_min_reflectors reflectors (default 24). */
+ * stack-width class): a factor product goes to the FP64-accurate tensor-core path when it has at
+ * least oz_min_outputs outputs (default 256, with K >= 16, M >= 16, N >= 8; the products of an update
+ * with a dense C and hcgb_dgemm: at least 2048 whatever the knob), and in the plain form a side's Q
+ * is applied in WY form when it has at least wy_min_reflectors reflectors (default 24).  Results
+ * depend on them by the rounding of the path taken: relative to each output's terms on the FP64 pipe,
+ * to the maxima of its row and column on the tensor cores (hcgb_set_tensor_products). */
 int hcgb_set_tuning(hcgb_context *ctx, int oz_min_outputs, int wy_min_reflectors);
 
 /* A core SVD with at least min_cols Jacobi columns finds its rotations in FP32 sweeps (accumulated, made
@@ -195,10 +197,12 @@ int hcgb_set_precond(hcgb_context *ctx, int min_cols);
  * sketches every update whose sketch is narrower than its stacks. */
 int hcgb_set_sketch_limit(hcgb_context *ctx, int percent);
 
-/* Factor products of k >= 16 with at least 256 outputs run on the 16-bit tensor cores by
- * error-free splitting (each FP64 operand cut into eight 7-bit integer digit planes relative to its
- * row / column maximum, plane products accumulated exactly in FP32 and combined in FP64; result
- * error below 2^-44 max|A_i| max|B_j|, the order of an FP64 product's worst-case bound).
+/* Factor products of k >= 16 with at least 256 outputs (dense results: 2048) run on the 16-bit tensor
+ * cores by error-free splitting (each FP64 operand cut into eight 7-bit integer digit planes relative to
+ * its row / column maximum, plane products accumulated exactly in FP32 and combined in FP64; result
+ * error below 2^-44 max|A_i| max|B_j|, the order of an FP64 product's worst-case bound; operands below
+ * 2^-57 of that maximum, and subnormals, count as zero; outputs of a row or column with a NaN or an
+ * infinity are FP64 products).
  * enable = 0 keeps every product on the FP64 DMMA path.  Default 1.  Schedule-independent. */
 int hcgb_set_tensor_products(hcgb_context *ctx, int enable);
 

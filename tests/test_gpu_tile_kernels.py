@@ -179,3 +179,20 @@ def test_tensor_core_products_at_tile_edges(T, m, n, k):
     scale = np.abs(a).max(1)[:, None] * np.abs(b).max(0)[None, :]
     bound = 2 * k * 2.0 ** -56 * scale * 2 + EPS * np.abs(p) + EPS * (np.abs(c) + np.abs(p))
     assert np.all(np.abs(g.to_dense() - (p + c)) <= bound)
+
+
+@pytest.mark.parametrize("m,n", [(16, 16), (17, 31), (45, 45), (129, 8)])
+def test_dense_products_below_2048_outputs_are_componentwise(T, m, n):
+    """C = A B + C of a small dense update: each output's error is relative to its own terms (an FP64 sum of k + 1
+    terms), also where the row's and the column's largest entries meet a zero."""
+    rng = np.random.default_rng([m, n])
+    k = 40
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((k, n))
+    a[:, k // 2:] *= 2.0 ** -80
+    b[:k // 2] = 0.0
+    c = rng.standard_normal((m, n)) * 2.0 ** -80
+    g = T.DenseTile(m, n, c)
+    T.HCore.Gemm(1.0, T.DenseTile(m, k, a), 0, T.DenseTile(k, n, b), 0, 1.0, g, T.CompressionParameters(1e-8))
+    p = a.astype(np.longdouble) @ b.astype(np.longdouble) + c
+    bound = (k + 2) * EPS * (np.abs(a) @ np.abs(b) + np.abs(c))
+    assert np.all(np.abs(g.to_dense() - p) <= bound)
