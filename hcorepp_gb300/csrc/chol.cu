@@ -18,6 +18,8 @@ constexpr int CT = 1024;
 // SM's FP64 pipe and dependent loads: with the panel solve below, five tiles of 512 and ten panel tiles took 285 ms
 // of a tile Cholesky, 10 ms now.)  L(i, k) stands at A[i rs + k cs]: lower triangle
 // rs = 1, cs = lda, upper the other way round.  Every L(i, j) takes its products in ascending k.
+// A launch acts on failures of earlier launches alone (*info at most the last column it depends on), so that
+// all its threads decide alike whenever they read the word that one of its own CTAs may write.
 constexpr int PB = 32;
 
 // Factors the leading nb x nb block held in shared memory (lower part); returns the failing column + 1 or 0.
@@ -56,10 +58,12 @@ __global__ void __launch_bounds__(256) potrf_first_kernel(double *A, int n, int 
     if (threadIdx.x == 0) *info = bad;
 }
 
-// Rows below block column j0 (width PB): 32 rows a CTA, four threads a row, each with every fourth column.
+// Rows below block column j0 (width PB; the columns before a failing one): 32 rows a CTA, four threads a row, each with
+// every fourth column.
 __global__ void __launch_bounds__(128) potrf_panel_kernel(double *A, int n, int j0, int rs, int cs, const int *info) {
     __shared__ double D[PB][PB + 1];
-    if (*info) return;
+    const int bad = *info, cols = bad ? bad - 1 - j0 : PB;
+    if (cols <= 0) return;
     for (int e = threadIdx.x; e < PB * PB; e += blockDim.x) {
         const int i = e % PB, k = e / PB;
         D[i][k] = i >= k ? A[(size_t) (j0 + i) * rs + (size_t) (j0 + k) * cs] : 0.0;
@@ -84,13 +88,15 @@ __global__ void __launch_bounds__(128) potrf_panel_kernel(double *A, int n, int 
     }
     if (in)
 #pragma unroll
-        for (int u = 0; u < PB / 4; u++) r[(size_t) (4 * u + q) * cs] = t[u];
+        for (int u = 0; u < PB / 4; u++)
+            if (4 * u + q < cols) r[(size_t) (4 * u + q) * cs] = t[u];
 }
 
 // Trailing tiles (ti, tj), ti >= tj, behind block column j0: A -= L_i L_j^T; tile (0, 0) is factored too.
 __global__ void __launch_bounds__(256) potrf_update_kernel(double *A, int n, int j0, int rs, int cs, int *info) {
     __shared__ double Li[PB][PB + 1], Lj[PB][PB + 1];
-    if (*info) return;  // written by tile (0, 0) alone, after every earlier launch
+    const int bad_before = *info;
+    if (bad_before && bad_before <= j0 + PB) return;  // tile (0, 0) of this launch writes j0 + PB + 1 or more
     int ti = 0, base = 0;
     while (base + ti + 1 <= (int) blockIdx.x) {
         base += ti + 1;
@@ -142,6 +148,14 @@ __global__ void __launch_bounds__(256) potrf_update_kernel(double *A, int n, int
         if (i >= k) A[(size_t) (i0 + i) * rs + (size_t) (i0 + k) * cs] = Li[i][k];
     }
     if (threadIdx.x == 0 && bad) *info = i0 + bad;
+}
+
+// Columns k >= from of the triangle (L(i, k), i >= k) copied between A (ld lda) and keep (ld n); a CTA a stored column.
+__global__ void __launch_bounds__(256) potrf_copy_kernel(int uplo, int n, int from, const double *src, int lds, double *dst,
+                                                         int ldd) {
+    const int c = blockIdx.x, r0 = uplo == 0 ? c : from, r1 = uplo == 0 ? n : c + 1;
+    if (uplo == 0 && c < from) return;
+    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) dst[r + (size_t) c * ldd] = src[r + (size_t) c * lds];
 }
 
 // op(A) X = alpha B (side 0) or X op(A) = alpha B (side 1); X overwrites B (m x n, ld ldb).
@@ -278,8 +292,13 @@ void launch_fill_triangle(int uplo, int n, double *A, int lda, double value, cud
     { fill_triangle_kernel<<<grid, blk, 0, st>>>(uplo, n, A, lda, value); note_launch(); }
 }
 
-void launch_potrf(double *A, int n, int lda, int uplo, int *info_dev, cudaStream_t st) {
+void launch_potrf_restore(double *A, int n, int lda, int uplo, int failed, const double *keep, cudaStream_t st) {
+    { potrf_copy_kernel<<<n, 256, 0, st>>>(uplo, n, failed - 1, keep, n, A, lda); note_launch(); }
+}
+
+void launch_potrf(double *A, int n, int lda, int uplo, int *info_dev, double *keep, cudaStream_t st) {
     const int rs = uplo == 0 ? 1 : lda, cs = uplo == 0 ? lda : 1;
+    if (keep) { potrf_copy_kernel<<<n, 256, 0, st>>>(uplo, n, 0, A, lda, keep, n); note_launch(); }
     { potrf_first_kernel<<<1, 256, 0, st>>>(A, n, rs, cs, info_dev); note_launch(); }
     for (int j0 = 0; j0 + PB < n; j0 += PB) {
         const int rest = (n - j0 - 1) / PB;  // row blocks below

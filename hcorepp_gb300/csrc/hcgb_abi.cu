@@ -1152,13 +1152,19 @@ extern "C" int hcgb_potrf(hcgb_context *ctx, int uplo, int n, double *A, int lda
         if (info) *info = 0;
         return HCGB_OK;
     }
-    int *dinfo = nullptr;
-    HCGB_CUDA(ctx, cudaMalloc(&dinfo, sizeof(int)));
-    launch_potrf(A, n, lda, uplo, dinfo, ctx->stream);
+    const size_t keep_bytes = sizeof(double) * (size_t) n * n;
+    int rc = ensure_device(ctx, &ctx->be_scratch, &ctx->be_scratch_bytes, keep_bytes + sizeof(int));
+    if (rc) return rc;
+    auto *keep = static_cast<double *>(ctx->be_scratch);
+    int *dinfo = reinterpret_cast<int *>(static_cast<char *>(ctx->be_scratch) + keep_bytes);
+    launch_potrf(A, n, lda, uplo, dinfo, keep, ctx->stream);
     int h = 0;
     cudaError_t e = cudaMemcpyAsync(&h, dinfo, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(dinfo);
+    if (e == cudaSuccess && h) {
+        launch_potrf_restore(A, n, lda, uplo, h, keep, ctx->stream);
+        e = cudaStreamSynchronize(ctx->stream);
+    }
     if (e != cudaSuccess) return fail(ctx, HCGB_CUDA_ERROR, std::string("hcgb_potrf: ") + cudaGetErrorString(e));
     if (info) *info = h;
     return HCGB_OK;
@@ -1265,17 +1271,18 @@ extern "C" int hcgb_tile_cholesky(hcgb_context *ctx, int nt, const hcgb_tile *gr
     if (info) *info = 0;
     int *dinfo = nullptr;
     DevTile *dpanel = nullptr;
-    HCGB_CUDA(ctx, cudaMalloc(&dinfo, sizeof(int) * (size_t) nt));
-    if (cudaMalloc(&dpanel, sizeof(DevTile) * (size_t) nt) != cudaSuccess) {
-        cudaFree(dinfo);
-        return fail(ctx, HCGB_CUDA_ERROR, "hcgb_tile_cholesky: cudaMalloc failed");
-    }
+    double *keep = nullptr;  // the diagonal tile, in case it is not positive definite
     auto done = [&](int rc) {
         cudaStreamSynchronize(ctx->stream);
         cudaFree(dinfo);
         cudaFree(dpanel);
+        cudaFree(keep);
         return rc;
     };
+    if (cudaMalloc(&dinfo, sizeof(int) * (size_t) nt) != cudaSuccess ||
+        cudaMalloc(&dpanel, sizeof(DevTile) * (size_t) nt) != cudaSuccess ||
+        cudaMalloc(&keep, sizeof(double) * (size_t) nb * nb) != cudaSuccess)
+        return done(fail(ctx, HCGB_CUDA_ERROR, "hcgb_tile_cholesky: cudaMalloc failed"));
     const Params p = to_params(params, ctx);
     const int max_chunk = 1024;  // updates per pipeline launch (bounds the workspace)
     int uid = 0;
@@ -1283,7 +1290,7 @@ extern "C" int hcgb_tile_cholesky(hcgb_context *ctx, int nt, const hcgb_tile *gr
     for (int k = 0; k < nt; k++) {
         // Syrk leaves the strict upper triangle of a diagonal tile zero (HCore.cpp:555-563).
         if (k > 0) launch_fill_triangle(HCGB_UPPER, nb, tile(k, k).data, nb, 0.0, ctx->stream);
-        launch_potrf(tile(k, k).data, nb, nb, HCGB_LOWER, dinfo + k, ctx->stream);
+        launch_potrf(tile(k, k).data, nb, nb, HCGB_LOWER, dinfo + k, keep, ctx->stream);
         int h = 0;
         cudaError_t e = cudaMemcpyAsync(&h, dinfo + k, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -1291,6 +1298,7 @@ extern "C" int hcgb_tile_cholesky(hcgb_context *ctx, int nt, const hcgb_tile *gr
                                                                      cudaGetErrorString(e)));
         if (h) {
             if (info) *info = k * nb + h;
+            launch_potrf_restore(tile(k, k).data, nb, nb, HCGB_LOWER, h, keep, ctx->stream);
             return done(HCGB_OK);
         }
         if (k == nt - 1) break;

@@ -347,7 +347,10 @@ void launch_transpose(const double *src, int lds, int rows, int cols, double *ds
 // Dense tile building blocks of a tile Cholesky (chol.cu).
 void launch_trsm_panel(const double *L, int nb, int ldl, const DevTile *tiles, int count, int max_rank, cudaStream_t st);
 void launch_fill_triangle(int uplo, int n, double *A, int lda, double value, cudaStream_t st);
-void launch_potrf(double *A, int n, int lda, int uplo, int *info_dev, cudaStream_t st);
+// keep (n x n, or null): a copy of the triangle, from which launch_potrf_restore takes the columns from the failing
+// one on (*info_dev = failed) back; without it they are left partly updated.
+void launch_potrf(double *A, int n, int lda, int uplo, int *info_dev, double *keep, cudaStream_t st);
+void launch_potrf_restore(double *A, int n, int lda, int uplo, int failed, const double *keep, cudaStream_t st);
 void launch_trsm(int side, int uplo, int trans, int diag, int m, int n, double alpha, const double *A, int lda,
                  double *B, int ldb, cudaStream_t st);
 void launch_syrk(int uplo, int trans, int n, int k, double alpha, const double *A, int lda, double beta, double *C,

@@ -196,3 +196,27 @@ def test_dense_products_below_2048_outputs_are_componentwise(T, m, n):
     p = a.astype(np.longdouble) @ b.astype(np.longdouble) + c
     bound = (k + 2) * EPS * (np.abs(a) @ np.abs(b) + np.abs(c))
     assert np.all(np.abs(g.to_dense() - p) <= bound)
+
+
+@pytest.mark.parametrize("uplo", [0, 1])
+@pytest.mark.parametrize("n,bad", [(20, 7), (70, 0), (300, 31), (300, 32), (300, 45), (300, 150), (300, 299)])
+def test_potrf_stops_at_the_failing_column(T, n, bad, uplo):
+    """A matrix whose leading minor of order bad + 1 is not positive: the columns before are those of the factor, the
+    rest is as given, in every run alike."""
+    rng = np.random.default_rng([n, bad])
+    g = rng.standard_normal((n, n + 3))
+    a = g @ g.T + n * np.eye(n)
+    a[bad, bad] = -1.0
+    stored = np.tril(a) if uplo == 0 else np.triu(a)
+    first = None
+    for _ in range(4):
+        info, out = _potrf(T, stored, uplo)
+        assert info == bad + 1
+        first = out if first is None else first
+        np.testing.assert_array_equal(out, first)
+    f = np.tril(first) if uplo == 0 else np.triu(first).T
+    np.testing.assert_array_equal(f[:, bad:], np.tril(a)[:, bad:])
+    l = f[:, :bad]
+    low = np.tril(np.ones((n, bad), dtype=bool))
+    err = np.abs(l @ l[:bad].T - a[:, :bad])
+    assert np.all(err[low] <= 2 * (n + 2) * EPS * (np.abs(l) @ np.abs(l[:bad]).T)[low])
