@@ -1987,24 +1987,24 @@ size_t svd_smem_bytes(int kmax) { return 2 * sizeof(double) * (size_t) svd_team_
 // Register tiles of the FP64 sweeps: up to 16 rows a lane (longer columns take the looped sweep).
 constexpr int CORE_RPL = 16;
 
-// A core of k columns takes its aux arrays, 6 k + SVD_AUX_FIXED doubles, and a k x k working copy; in half an SM and in a
-// whole one, where a cluster may do the same work, the preconditioner's padded columns too (one double aligns
-// them).  A 110-column core
+// A core of k columns takes its aux arrays, 6 k + SVD_AUX_FIXED doubles, a k x k working copy and the preconditioner's
+// padded columns (one double aligns them), whatever its team: one that they did not fit would fall back to
+// the FP64 sweeps, twice the time at 25 columns.  A 110-column core
 // of width 128 takes a cluster of eight 4,300 kcycles and one SM alone 7,900: heavy ones go to clusters only
 // while SMs are idle, wide ones always.
 void core_classes(int kmax, int *whole, int *half, int *quarter) {
     const int team = svd_team_doubles(kmax);
-    auto widest = [](long doubles, bool padded) {
+    auto widest = [](long doubles) {
         int k = 0;
         while (true) {
             const long c = k + 1, q = (c + 3) / 4;
-            if ((padded ? 2 * precond_quads(q, q) * c + 1 : c * c) + 6 * c + SVD_AUX_FIXED > doubles) return k;
+            if (std::max(2 * precond_quads(q, q) * c + 1, c * c) + 6 * c + SVD_AUX_FIXED > doubles) return k;
             k++;
         }
     };
-    *whole = widest(2 * team, true);
-    *half = widest(team, true);
-    *quarter = widest(team / 2, false);
+    *whole = widest(2 * team);
+    *half = widest(team);
+    *quarter = widest(team / 2);
 }
 
 static void launch_core_wide(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {

@@ -68,3 +68,40 @@ def test_recompression_at_class_edges(T, n, rc, ra, kind, mode):
     # U = M XV Sigma^-2: orthonormal up to rounding relative to the smallest kept singular value
     u = np.asarray(gc.u(), dtype=np.float64)
     assert np.abs(u.T @ u - np.eye(u.shape[1])).max() <= 64 * k * unit * norms.max() / norms.min()
+
+
+def _update_in_capacities(T, k, kind, mode, extras):
+    """(rank, U, V) of one update of stack width k in tiles of capacity sum k + extra.  A lies below the threshold but not
+    below the pivoted QR's stop: all k columns are swept, C's own rank is the result's in every capacity."""
+    rng = np.random.default_rng([k, len(kind)])
+    n, ra = max(120, k), k // 2
+    rc = k - ra
+    sc = np.logspace(0, -6, rc) if kind == "decay" else np.repeat(np.logspace(0, -6, (rc + 2) // 3), 3)[:rc]
+    cu, cv = _factor(rng, n, n, sc)
+    au, av = _factor(rng, n, n, np.linspace(3e-9, 2e-9, ra))
+    bv = np.linalg.qr(rng.standard_normal((n, ra)))[0].T
+    bu = av.T / np.linalg.norm(av, axis=1)  # A B = Au Sigma Bv
+    out = []
+    for extra in extras:
+        c = T.CompressedTile(n, n, cu, cv, max_rank=rc + extra)
+        a = T.CompressedTile(n, n, au, av, max_rank=ra)
+        b = T.CompressedTile(n, n, bu, bv, max_rank=ra)
+        T.HCore.Gemm(1.0, a, 0, b, 0, 1.0, c, T.CompressionParameters(1e-8, truncated_svd=True, mode=mode))
+        out.append((c.rank, c.u(), c.v()))
+    return out
+
+
+def _assert_same(results):
+    for r, u, v in results[1:]:
+        assert r == results[0][0]
+        np.testing.assert_array_equal(u, results[0][1])
+        np.testing.assert_array_equal(v, results[0][2])
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("kind", ["decay", "triples"])
+@pytest.mark.parametrize("k", [30, 41, 45, 73, 75, 76, 80, 81, 82])
+def test_preconditioned_cores_in_every_team(T, k, kind, mode):
+    """Widths around the quarter team's, in tiles whose capacities put them there and in the next larger team: a core
+    is preconditioned in either, with the same bits."""
+    _assert_same(_update_in_capacities(T, k, kind, mode, (4, 19, 30, 60, 200)))
