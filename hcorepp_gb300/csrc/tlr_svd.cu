@@ -1962,19 +1962,36 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
 
 namespace {
 
-// Doubles of shared memory per half-CTA team: everything a core of kmax columns could use, capped at
-// half of the per-block opt-in limit (less a reserve for the kernel's static shared variables), and
-// never below the aux arrays.
-int svd_team_doubles(int kmax) {
+// Half of the per-block opt-in limit of shared memory (less a reserve for the kernel's static shared variables), in
+// doubles.
+long svd_half_sm_doubles() {
     static const int optin = [] {  // thread-safe one-time initialisation
         int dev = 0, v = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         return v > 0 ? v : 48 * 1024;
     }();
-    const long aux = 6L * kmax + SVD_AUX_FIXED;
-    const long want = aux + (long) kmax * kmax + 14L * kmax;  // the square, or the preconditioner's padded columns
-    const long cap = (optin - 256) / 2 / (long) sizeof(double);
+    return (optin - 256) / 2 / (long) sizeof(double);
+}
+
+// Doubles a core of k columns takes: its aux arrays, the k x k working copy and the preconditioner's padded columns (one
+// double aligns them).
+long core_doubles(long k) {
+    const long q = (k + 3) / 4;
+    return 6 * k + SVD_AUX_FIXED + std::max(k * k, 2L * precond_quads((int) q, (int) q) * k + 1);
+}
+
+int widest_core(long doubles) {
+    int k = 0;
+    while (core_doubles(k + 1) <= doubles) k++;
+    return k;
+}
+
+// Doubles of shared memory per half-CTA team: what a core of kmax columns takes, capped at half of an SM's, and never
+// below the aux arrays.
+int svd_team_doubles(int kmax) {
+    const long aux = 6L * kmax + SVD_AUX_FIXED, cap = svd_half_sm_doubles();
+    const long want = std::max(aux + (long) kmax * kmax + 14L * kmax, core_doubles(kmax));
     long t = want < cap ? want : cap;
     if (t < aux) t = aux;  // checked against the device limit by the caller
     return (int) t;
@@ -1987,24 +2004,15 @@ size_t svd_smem_bytes(int kmax) { return 2 * sizeof(double) * (size_t) svd_team_
 // Register tiles of the FP64 sweeps: up to 16 rows a lane (longer columns take the looped sweep).
 constexpr int CORE_RPL = 16;
 
-// A core of k columns takes its aux arrays, 6 k + SVD_AUX_FIXED doubles, a k x k working copy and the preconditioner's
-// padded columns (one double aligns them), whatever its team: one that they did not fit would fall back to
-// the FP64 sweeps, twice the time at 25 columns.  A 110-column core
-// of width 128 takes a cluster of eight 4,300 kcycles and one SM alone 7,900: heavy ones go to clusters only
-// while SMs are idle, wide ones always.
+// Widths up to which a core fits its team (one that the preconditioner's columns did not fit would fall back to the FP64
+// sweeps, twice the time at 25 columns).  A whole and half an SM decide the order of the sweeps and the form of the
+// pivoted QR, so they follow from the SM alone and not from the capacities of a launch's tiles; a quarter only decides
+// which team takes the core.  A 110-column core of width 128 takes a cluster of eight 4,300 kcycles and one SM
+// alone 7,900: heavy ones go to clusters only while SMs are idle, wide ones always.
 void core_classes(int kmax, int *whole, int *half, int *quarter) {
-    const int team = svd_team_doubles(kmax);
-    auto widest = [](long doubles) {
-        int k = 0;
-        while (true) {
-            const long c = k + 1, q = (c + 3) / 4;
-            if (std::max(2 * precond_quads(q, q) * c + 1, c * c) + 6 * c + SVD_AUX_FIXED > doubles) return k;
-            k++;
-        }
-    };
-    *whole = widest(2 * team);
-    *half = widest(team);
-    *quarter = widest(team / 2);
+    *whole = widest_core(2 * svd_half_sm_doubles());
+    *half = widest_core(svd_half_sm_doubles());
+    *quarter = widest_core(svd_team_doubles(kmax) / 2);
 }
 
 static void launch_core_wide(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {

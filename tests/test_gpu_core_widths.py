@@ -105,3 +105,11 @@ def test_preconditioned_cores_in_every_team(T, k, kind, mode):
     """Widths around the quarter team's, in tiles whose capacities put them there and in the next larger team: a core
     is preconditioned in either, with the same bits."""
     _assert_same(_update_in_capacities(T, k, kind, mode, (4, 19, 30, 60, 200)))
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("kind", ["decay", "triples"])
+@pytest.mark.parametrize("k", [9, 10, 25, 26, 41, 58, 74, 90, 105, 106, 114, 115])
+def test_results_do_not_depend_on_the_capacity(T, k, kind, mode):
+    """A full stack of k columns, in tiles that hold no more and in larger ones."""
+    _assert_same(_update_in_capacities(T, k, kind, mode, (0, 1, 16, 60, 200)))
