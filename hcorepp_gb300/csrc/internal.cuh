@@ -244,6 +244,7 @@ struct Workspace {
     int k_wide, k_heavy;  // stack widths above which a core does not fit an SM's / half an SM's shared memory
     size_t off_ustack, off_vstack, off_tmp1, off_tmp2, off_tauu, off_tauv, off_tu, off_tv;
     size_t off_m, off_mcopy, off_xv, off_sigma, off_mixed;
+    size_t mixed_floats;  // of the region at off_mixed: the preconditioner's columns of X and J, W
     size_t off_w;  // WY application: W_U, W_V (kmax x kmax each), present when built with wy
     size_t off_sk1, off_sk2, off_skaux;  // learned form: sketch stacks (ld x kmax each), residual estimate
     float *feat;   // learned form / feature sink: MLP_IN features per update (n x MLP_IN), or null

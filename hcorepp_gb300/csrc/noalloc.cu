@@ -93,13 +93,19 @@ extern "C" int hcgb_tile_gemm_noalloc(double alpha, const hcgb_tile *a, const hc
     if (kmax < 8) kmax = 8;
     Workspace ws = make_workspace_layout(ld, kmax, rmax, false);
     ws.order = nullptr;  // a single update: no ordering
-    const size_t slot_bytes = round_up_bytes(sizeof(double) * ws.slot_doubles);
     const size_t meta_bytes = round_up_bytes(sizeof(int) * META_INTS);
     const size_t desc_bytes = round_up_bytes(sizeof(DevUpdate));
     const size_t job_bytes = round_up_bytes(sizeof(GemmJob) * 3);
     const size_t sched_bytes = round_up_bytes(sizeof(int) * 8);  // three tile lists of one job
-    if (slot_bytes + meta_bytes + desc_bytes + job_bytes + sched_bytes > sizeof(double) * HCGB_NOALLOC_SCRATCH_DOUBLES)
-        return HCGB_POOL_TOO_SMALL;
+    const size_t rest = meta_bytes + desc_bytes + job_bytes + sched_bytes;
+    if (round_up_bytes(sizeof(double) * ws.slot_doubles) + rest > sizeof(double) * HCGB_NOALLOC_SCRATCH_DOUBLES) {
+        // The last region without the padding that only a full-rank core of kmax columns asks for (it then takes
+        // the FP64 sweeps): a handful of shapes at the scratch's limit fit that way.
+        ws.mixed_floats = (size_t) kmax * (kmax + ld);
+        ws.slot_doubles = ws.off_mixed + ((ws.mixed_floats + 1) / 2 + 31) / 32 * 32;
+    }
+    const size_t slot_bytes = round_up_bytes(sizeof(double) * ws.slot_doubles);
+    if (slot_bytes + rest > sizeof(double) * HCGB_NOALLOC_SCRATCH_DOUBLES) return HCGB_POOL_TOO_SMALL;
     // The QR panels and the core's bookkeeping live in shared memory: the same per-CTA limit as the
     // allocating entry points, checked before anything is launched so that C stays untouched.
     const size_t smem_limit = 227 * 1024;

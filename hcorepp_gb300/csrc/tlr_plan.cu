@@ -656,7 +656,10 @@ Workspace make_workspace_layout(int ld, int kmax, int rmax, bool ddc_scratch, bo
     w.off_mcopy = off;  off += round((size_t) kmax * kmax);
     w.off_xv = off;     off += round((size_t) ld * kmax);
     w.off_sigma = off;  off += round(kmax);
-    w.off_mixed = off;  off += round(((size_t) kmax * (size_t) (kmax + ld) + 1) / 2);  // float X32 + J32
+    // X32 and J32, each column padded to quads (the second form: a full-rank core of kmax columns and nearly as many rows)
+    const size_t full = ld < kmax ? ld : kmax;
+    w.mixed_floats = std::max((size_t) kmax * (size_t) (kmax + ld), 8 * ((full + 3) / 4) * full);
+    w.off_mixed = off;  off += round((w.mixed_floats + 1) / 2);
     w.off_w = wy ? off : 0;  // 0: absent (no region starts at 0 but the U stack)
     off += wy ? round(2 * (size_t) kmax * kmax) : 0;
     w.off_sk1 = learned ? off : 0;

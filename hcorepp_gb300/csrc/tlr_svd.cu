@@ -1807,7 +1807,7 @@ __device__ void core_update(const TM &tm, const DevUpdate *ups, const Workspace 
             b.ldh = ld;
             b.v = reinterpret_cast<float *>(b.y);
             b.ldv = 4 * b.ls4;
-            fits = 4 * (size_t) b.ls4 * rk <= (size_t) ws.kmax * (ws.kmax + ws.ld) && 2 * b.ls4 <= b.buf_quads;
+            fits = 4 * (size_t) b.ls4 * rk <= ws.mixed_floats && 2 * b.ls4 <= b.buf_quads;
         } else {
             b.ls4 = precond_quads(x4, j4);
             b.blocks = k > ws.k_heavy ? SWEEP_BLOCKS : 0;  // as on a cluster

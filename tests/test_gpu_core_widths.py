@@ -113,3 +113,48 @@ def test_preconditioned_cores_in_every_team(T, k, kind, mode):
 def test_results_do_not_depend_on_the_capacity(T, k, kind, mode):
     """A full stack of k columns, in tiles that hold no more and in larger ones."""
     _assert_same(_update_in_capacities(T, k, kind, mode, (0, 1, 16, 60, 200)))
+
+
+def _full_rank_core(T, n, extras, mode):
+    """An update whose core has full rank n = k and nothing to truncate before the threshold, in several capacities."""
+    rng = np.random.default_rng(n)
+    rc = n - n // 2
+    orth = lambda m: np.linalg.qr(rng.standard_normal((m, m)))[0]
+    qu, qv, gc, ga = orth(n), orth(n), orth(rc), orth(n - rc)  # gc, ga: the sweeps have something to turn
+    sa = np.linspace(3e-9, 2e-9, n - rc)
+    out = []
+    for extra in extras:
+        c = T.CompressedTile(n, n, (qu[:, :rc] * np.logspace(0, -6, rc)) @ gc, qv[:, :rc].T, max_rank=rc + extra)
+        a = T.CompressedTile(n, n, (qu[:, rc:] * sa) @ ga, qv[:, rc:].T, max_rank=n - rc)
+        b = T.CompressedTile(n, n, qv[:, rc:], qv[:, rc:].T, max_rank=n - rc)
+        T.HCore.Gemm(1.0, a, 0, b, 0, 1.0, c, T.CompressionParameters(1e-8, truncated_svd=True, mode=mode))
+        out.append((c.rank, c.u(), c.v()))
+    return out
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [197, 199, 301, 302, 303, 304])
+def test_wide_full_rank_cores_do_not_depend_on_the_capacity(T, n, mode):
+    """As many rows as columns, and no multiple of 4: the padded columns of X and J at their longest."""
+    _assert_same(_full_rank_core(T, n, (0, 1, 16, 100), mode))
+
+
+def test_noalloc_shapes_at_the_limit_of_its_scratch(T):
+    """A shape that fits the 8 MiB only without those columns' padding is still taken."""
+    import ctypes as C
+    import torch
+    from hcorepp_gb300 import _lib as L
+    rng = np.random.default_rng(1)
+    n, rmax, rc = 400, 152, 245
+    cu, cv = _factor(rng, n, n, np.logspace(0, -6, 12))
+    au, av = _factor(rng, n, n, np.logspace(0, -6, 10))
+    tiles = [T.CompressedTile(n, n, au, av, max_rank=rmax), T.CompressedTile(n, n, av.T, au.T, max_rank=rmax),
+             T.CompressedTile(n, n, cu, cv, max_rank=rc)]
+    a, b, c = (t.c_tile() for t in tiles)
+    p = T.CompressionParameters(1e-8, truncated_svd=True).c()
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert L.lib().hcgb_tile_gemm_noalloc(1.0, C.byref(a), C.byref(b), 1.0, C.byref(c), C.byref(p), stream,
+                                          C.c_void_p(0)) == L.HCGB_OK
+    torch.cuda.synchronize()
+    exact = au @ av @ av.T @ au.T + cu @ cv
+    assert rel_fro(tiles[2].to_dense(), exact) <= 1.02e-8 * np.sqrt(22)
