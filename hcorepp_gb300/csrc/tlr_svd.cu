@@ -1527,7 +1527,7 @@ __device__ __forceinline__ int core_aux_doubles(const Workspace &ws, int slot) {
 // depends on the launch it is part of.
 template <int RPL>
 __device__ void core_svd_cta(const DevUpdate *ups, int nup, const Workspace &ws, const Params &p, int team_doubles, int kthr4) {
-    extern __shared__ double smem_all[];
+    extern __shared__ __align__(16) double smem_all[];  // read as float4 at even offsets
     __shared__ CoreShared s_sh[4];
     __shared__ int s_end[3];  // first index behind the wide, heavy and light updates
     if (threadIdx.x < 3)
@@ -1582,7 +1582,7 @@ __global__ void __launch_bounds__(SVD_THREADS, 1) core_svd_kernel(const DevUpdat
 template <int RPL>
 __global__ void __cluster_dims__(WIDE_CTAS, 1, 1) __launch_bounds__(SVD_THREADS, 1)
     core_wide_kernel(const DevUpdate *ups, int nup, Workspace ws, Params p, int smem_doubles) {
-    extern __shared__ double smem_all[];
+    extern __shared__ __align__(16) double smem_all[];  // read as float4 at even offsets
     __shared__ CoreShared s_sh;
     __shared__ int s_wide;
     let_next_launch_start();

@@ -84,3 +84,20 @@ def test_rank_trimmed_host_pack_layout():
             want += [arena[o:o + nb * r], arena[o + nb * mr:o + nb * mr + r * nb]]
     np.testing.assert_array_equal(got, np.concatenate(want))
     assert got.size == 2 * nb * nb + 2 * nb * (2 + 3 + 1 + 1)  # two dense tiles; compressed ranks 2, 3, 1, 1
+
+
+def test_shared_arrays_read_as_vectors_state_their_alignment():
+    """Dynamic shared memory of a file that reads 16-byte vectors is declared 16-byte aligned (or more)."""
+    import glob
+    import os
+    import re
+    seen = 0
+    for path in glob.glob(os.path.join(os.path.dirname(L.__file__), "csrc", "*.cu")):
+        text = open(path).read()
+        if not re.search(r"reinterpret_cast<(?:const )?(?:float4|double2|uint4|int4) \*>", text):
+            continue
+        for decl in re.findall(r"extern __shared__[^;]*;", text):
+            seen += 1
+            align = re.search(r"__align__\((\d+)\)", decl)
+            assert align and int(align.group(1)) >= 16, (path, decl)
+    assert seen
