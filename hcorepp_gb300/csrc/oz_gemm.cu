@@ -324,7 +324,7 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     }
     chunks += nchunks;
     windows += nwindows;
-    if (!ok && lane == 0) atomicAdd(&g_oz_wait_timeouts, 1u);
+    if (!__all_sync(0xffffffffu, ok) && lane == 0) atomicAdd(&g_oz_wait_timeouts, 1u);  // the MMAs' waits are one lane's
 
     // Epilogue: C = alpha * product + beta * C, one row per thread, 16 columns.
     const int row_l = q * 32 + lane;
