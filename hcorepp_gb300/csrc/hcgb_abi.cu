@@ -348,6 +348,7 @@ int prepare_workspace(hcgb_context *ctx, const BatchShape &sh, int n, bool ddc, 
     if (int refused = check_shared_memory(ctx, sh)) return refused;
     const bool learned = ctx->learned, features = learned || ctx->feature_sink;
     Workspace w = make_workspace_layout(sh.ld, sh.kmax, sh.rmax, ddc, ctx->oz != 0 || lowp_prec(mode) != 0, learned);
+    set_core_classes(&w);
     size_t need = workspace_bytes_for(w, n, features);
     int rc = ensure_device(ctx, &ctx->ws, &ctx->ws_bytes, need);
     if (rc) return rc;

@@ -279,7 +279,8 @@ struct Workspace {
 };
 
 // Layout of one workspace slot for stacks of up to `ld` rows and `kmax` columns; factor ranks
-// up to `rmax`.  ddc_scratch reserves an ld x ld product for the DDC combination.
+// up to `rmax`.  ddc_scratch reserves an ld x ld product for the DDC combination.  Host arithmetic alone (sizing needs no
+// device); what launches on the workspace needs set_core_classes too.
 Workspace make_workspace_layout(int ld, int kmax, int rmax, bool ddc_scratch, bool wy = false, bool learned = false);
 
 struct Params {
@@ -334,8 +335,10 @@ void launch_plan_wy(const DevUpdate *ups, int n, Workspace ws, Params p, GemmJob
 void launch_wy_solve(int n, Workspace ws, cudaStream_t st);
 void launch_qr(Workspace ws, int n, bool mixed, cudaStream_t st);
 void launch_core_svd(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st);
-// Stack widths up to which a core fits a whole, half and a quarter of an SM's shared memory in launches of kmax.
+// Stack widths up to which a core fits a whole, half and a quarter of an SM's shared memory in launches of kmax (asks the
+// device); set_core_classes fills the workspace's k_wide and k_heavy with the first two.
 void core_classes(int kmax, int *whole, int *half, int *quarter);
+void set_core_classes(Workspace *ws);
 void launch_apply_q(const DevUpdate *ups, int n, Workspace ws, bool mixed, cudaStream_t st);
 void launch_finalize(const DevUpdate *ups, int n, Workspace ws, hcgb_update_info *info, cudaStream_t st);
 // FP64 throughput probes (TFLOP/s): tensor-core DMMA and SIMT DFMA.

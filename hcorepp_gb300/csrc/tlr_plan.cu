@@ -639,8 +639,6 @@ Workspace make_workspace_layout(int ld, int kmax, int rmax, bool ddc_scratch, bo
     w.ld = ld;
     w.kmax = kmax;
     w.rmax = rmax;
-    int quarter;
-    core_classes(kmax, &w.k_wide, &w.k_heavy, &quarter);
     auto round = [](size_t x) { return (x + 31) & ~size_t(31); };  // 256-byte aligned sub-buffers
     size_t off = 0;
     const int npan = (kmax + QR_NB - 1) / QR_NB;

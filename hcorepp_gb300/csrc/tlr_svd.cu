@@ -2015,6 +2015,11 @@ void core_classes(int kmax, int *whole, int *half, int *quarter) {
     *quarter = widest_core(svd_team_doubles(kmax) / 2);
 }
 
+void set_core_classes(Workspace *ws) {
+    int quarter;
+    core_classes(ws->kmax, &ws->k_wide, &ws->k_heavy, &quarter);
+}
+
 static void launch_core_wide(const DevUpdate *ups, int n, Workspace ws, Params p, cudaStream_t st) {
     const int aux = 6 * ws.kmax + SVD_AUX_FIXED + 1;
     // a pair of column blocks, or (wider cores) as many columns as there is room for

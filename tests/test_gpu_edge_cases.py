@@ -134,3 +134,18 @@ def test_rectangular_tile_grid(T, mode):
     g = C.to_dense()
     o = np.block([[t.to_dense() for t in row] for row in oc])
     assert rel_fro(g, exact) <= 2 * max(rel_fro(o, exact), ACC)
+
+
+def test_workspace_sizing_does_not_start_cuda():
+    """hcgb_workspace_bytes is host arithmetic: a process that only sizes (and may fork afterwards) loads no driver."""
+    import subprocess
+    import sys
+    from hcorepp_gb300 import _lib as L
+    code = ("import ctypes as C\n"
+            f"lib = C.CDLL({L.LIB_PATH!r})\n"
+            "lib.hcgb_workspace_bytes.restype = C.c_size_t\n"
+            "assert lib.hcgb_workspace_bytes(4, 512, 512, 170, 170) > 0\n"
+            "print('libcuda.so' in open('/proc/self/maps').read())\n")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.strip() == "False"
