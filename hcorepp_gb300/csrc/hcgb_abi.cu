@@ -1141,6 +1141,7 @@ extern "C" int hcgb_compress_tiles(hcgb_context *ctx, int count, const double *c
             if (ranks) ranks[off + i] = hinfo[i].new_rank;
         }
     }
+    if (not_converged) ctx->last_error = "hcgb_compress_tiles: Jacobi sweep limit reached";
     return done(not_converged ? HCGB_NOT_CONVERGED : HCGB_OK);
 }
 
