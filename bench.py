@@ -19,7 +19,8 @@ every k step, as the reference driver does), starting from the same C every step
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--forms a,b]
 
-Prints one JSON line (rank 0).  Inputs (A, B, C: ~1.4 GB each) exceed L2, so no flush is
+Prints one JSON line (rank 0) of at most LINE_CHARS characters, so that a reader who keeps only the end of the output
+still has all of it; the blocks named here in full go to --details (bench_details.json).  Inputs (A, B, C: ~1.4 GB each) exceed L2, so no flush is
 needed between steps.  "value" times the multiply on device-resident tiles; "e2e" times the same
 multiply with the host's pinned A and C copied in and C copied out every step, in the
 rank-trimmed transfer format (hcgb_pack_tiles: only the factor columns the ranks use), and
@@ -49,6 +50,7 @@ if ROOT not in sys.path:
 from hcorepp_gb300.problems import WORKLOADS, build_tiles  # noqa: E402
 from hcorepp_gb300.replicas import job_throughput  # noqa: E402
 
+LINE_CHARS = 1400
 METRIC = "TLR-GEMM tile-updates/s at 1e-8 rel err: plain FP64 vs batched mixed+learned"
 UNIT = "tile-updates/s"
 HEADLINE_FORM = "plain_fp64"
@@ -86,6 +88,8 @@ def parse():
     ap.add_argument("--no-config4", action="store_true",
                     help="skip the n = 32768, nb = 1024 multiply (plain, float-float and learned forms; "
                          "hcorepp_gb300/learned_bench.py)")
+    ap.add_argument("--details", default=os.path.join(ROOT, "bench_details.json"),
+                    help="file for the full result (stages, every form, low-precision and nb = 1024 blocks); '' for none")
     ap.add_argument("--no-tuning", action="store_true",
                     help="default launch shapes instead of the autotuner's cache (hcorepp_gb300/tuning_cache.json)")
     return ap.parse_args()
@@ -616,6 +620,49 @@ def parity_block(wb, cpu_results, args, exact):
                    "product <= 2 x max(oracle's error, accuracy)"}
 
 
+def short_line(full):
+    """The printed line: the contract's keys and the figures a reader looks for first, of the full block."""
+    def sig(v, digits=6):
+        return float(f"{v:.{digits}g}") if isinstance(v, float) else v
+
+    cfg = full["config"]
+    line = {k: full[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                                 "higher_is_better", "scaling", "vs_baseline", "dtype", "data")}
+    line["config"] = {k: cfg[k] for k in ("workload", "n", "nb", "tiles", "updates_per_step", "accuracy", "form",
+                                          "parallelism", "l2")}
+    line["e2e"] = {k: full["e2e"][k] for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step")}
+    line["roofline"] = {k: sig(full["roofline"][k]) for k in ("bound", "kernel", "achieved", "peak", "unit", "frac")}
+    line["gpu_launches"] = full["gpu_launches"]
+    line["rel_err"] = sig(full["check"]["rel_fro_err_vs_fp64_dense_product"])
+    if full.get("parity"):
+        line["rank_violations"] = full["parity"]["rank_violations"]
+    line["forms"] = {f: [sig(b["value"]), sig(b["e2e"]["value"]) if "e2e" in b else None]
+                     for f, b in full["forms"].items()}
+    if full.get("cpu_baseline"):
+        line["cpu_baseline"] = {k: sig(full["cpu_baseline"][k]) for k in ("value", "cores", "kind")}
+    line["clocks"] = {k: full["clocks"].get(k) for k in ("sm_mhz", "sm_max_mhz", "reasons")}
+    return line
+
+
+def emit(full, details):
+    """Write the full block to the file `details` and print the short line."""
+    if details:
+        try:
+            with open(details, "w") as f:
+                json.dump(full, f, indent=1)
+        except OSError as e:
+            print(f"bench.py: no details file: {e}", file=sys.stderr)
+    text = json.dumps(short_line(full))
+    if len(text) > LINE_CHARS:  # the contract's keys come first: drop what is only convenient
+        line = short_line(full)
+        for k in ("forms", "cpu_baseline", "roofline"):
+            line.pop(k, None)
+            text = json.dumps(line)
+            if len(text) <= LINE_CHARS:
+                break
+    print(text, flush=True)
+
+
 def gpu_arm(args, rank, world, local):
     import torch
     if world > 1:
@@ -778,7 +825,7 @@ def gpu_arm(args, rank, world, local):
         torch.cuda.empty_cache()
         c4_forms = ["plain_fp64", "mixed_ff48"] + (["learned_ff48"] if os.path.exists(RM.WEIGHTS) else [])
         line["config4"] = learned_bench.run(steps=1, warmup=1, forms=c4_forms)
-    print(json.dumps(line), flush=True)
+    emit(line, args.details)
     return 0
 
 
