@@ -56,6 +56,7 @@ constexpr int OZ_THREADS = 512;         // 16 warps
 constexpr int OZ_A_PLANE = OZ_TM * OZ_KC * 2;   // 8 KB
 constexpr int OZ_B_PLANE = OZ_TN * OZ_KC * 2;   // 4 KB
 constexpr int OZ_STAGE = OZ_S * (OZ_A_PLANE + OZ_B_PLANE);  // 96 KB
+static_assert(OZ_TM * OZ_TN * 8 <= 2 * OZ_STAGE, "a tile's outputs fit the stages");
 constexpr int OZ_SMEM = 2 * OZ_STAGE + 1024;
 constexpr int OZ_TMEM_COLS = OZ_S * OZ_TN;  // 512: one 64-column accumulator per level
 constexpr int OZ_NOGROUP = -1100;       // exponent of an all-zero group
@@ -194,7 +195,7 @@ struct OzBarriers {
 // One 128 x 64 output tile of one job.  chunks / windows: 32-wide K chunks and read-out windows of the CTA's earlier
 // tiles; chunk t fills stage t & 1 for the (t >> 1)-th time.
 __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint32_t tmem, const OzBarriers &bars,
-                        int &chunks, int &windows, int *ea, int *eb) {
+                        int &chunks, int &windows, int *ea, int *eb, int *special) {
     const int ntm = (jb.M + OZ_TM - 1) / OZ_TM;
     const int m0 = (tile % ntm) * OZ_TM, n0 = (tile / ntm) * OZ_TN;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -203,6 +204,7 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
 
     // 1. Group exponents over all of K, largest exponent field per row of op(A) and column of op(B); the
     //    threads of a group are laid out so that consecutive lanes read consecutive addresses.
+    if (tid == 0) *special = 0;
     if (tid < OZ_TM) ea[tid] = 0;
     else if (tid < OZ_TM + OZ_TN) eb[tid - OZ_TM] = 0;
     __syncthreads();
@@ -227,13 +229,13 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     exponents(std::true_type{}, rows, ea);
     exponents(std::false_type{}, cols, eb);
     __syncthreads();
-    bool special = false;
     if (tid < OZ_TM + OZ_TN) {
-        int &e = tid < OZ_TM ? ea[tid] : eb[tid - OZ_TM];
-        special = e == 0x7ff;
-        e = special ? OZ_NONFINITE : (e ? e - 1022 : OZ_NOGROUP);
+        int *e = tid < OZ_TM ? ea + tid : eb + (tid - OZ_TM);
+        const int top = *e;
+        *e = top == 0x7ff ? OZ_NONFINITE : (top ? top - 1022 : OZ_NOGROUP);
+        if (top == 0x7ff) *special = 1;
     }
-    const bool nonfinite = __syncthreads_or(special);
+    __syncthreads();
 
     // This thread's share of the read-out: TMEM lanes 32 (warp % 4) .. (rows), columns 16 (warp / 4) ..
     const int q = warp & 3, h = warp >> 2;
@@ -326,6 +328,23 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
     windows += nwindows;
     if (!__all_sync(0xffffffffu, ok) && lane == 0) atomicAdd(&g_oz_wait_timeouts, 1u);  // the MMAs' waits are one lane's
 
+    // Outputs of a row or column with a NaN or an infinity, as an FP64 product gives them: put aside in the stages, which the
+    // MMAs have read, and stored over what the epilogue makes of them.  (A test an output in the epilogue cost the
+    // products 2 %.)
+    double *stash = reinterpret_cast<double *>(stage0);
+    if (*special) {
+        for (int e = tid; e < rows * cols; e += OZ_THREADS) {
+            const int r = e % rows, c = e / rows;
+            if (ea[r] + eb[c] < OZ_NONFINITE / 2) continue;
+            double v = 0.0;
+            for (int k = 0; k < jb.K; k++) v = fma(job_a(jb, m0 + r, k), job_b(jb, k, n0 + c), v);
+            v *= jb.alpha;
+            if (jb.beta != 0.0) v = fma(jb.beta, jb.C[m0 + r + (size_t) (n0 + c) * jb.ldc], v);
+            stash[e] = v;
+        }
+        __syncthreads();
+    }
+
     // Epilogue: C = alpha * product + beta * C, one row per thread, 16 columns.
     const int row_l = q * 32 + lane;
     if (reads && row_l < rows) {
@@ -335,11 +354,10 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
 #pragma unroll
         for (int j = 0; j < 16; j++) {
             const int cl = h * 16 + j;
-            const int eab = cl < cols ? ea[row_l] + eb[cl] : OZ_NONFINITE;
-            if (eab < OZ_NONFINITE / 2) {
+            if (cl < cols) {
                 double *cp = jb.C + m0 + row_l + (size_t) (n0 + cl) * jb.ldc;
                 double v = 0.0;
-                if (jb.K > 0) v = oz_value((long long) (hi[j] - constant), (long long) (lo[j] - constant), eab);
+                if (jb.K > 0) v = oz_value((long long) (hi[j] - constant), (long long) (lo[j] - constant), ea[row_l] + eb[cl]);
                 if (negate) v = -v;
                 if (scale) v *= jb.alpha;
                 if (accum) v = fma(jb.beta, *cp, v);
@@ -347,18 +365,12 @@ __device__ void oz_tile(const GemmJob &jb, int tile, unsigned char *stage0, uint
             }
         }
     }
-    // Outputs of a row or column with a NaN or an infinity, as an FP64 product gives them.
-    if (nonfinite)
-        for (int e = tid; e < rows * cols; e += OZ_THREADS) {
-            const int r = e % rows, c = e / rows;
-            if (ea[r] + eb[c] < OZ_NONFINITE / 2) continue;
-            double v = 0.0;
-            for (int k = 0; k < jb.K; k++) v = fma(job_a(jb, m0 + r, k), job_b(jb, k, n0 + c), v);
-            double *cp = jb.C + m0 + r + (size_t) (n0 + c) * jb.ldc;
-            v *= jb.alpha;
-            if (jb.beta != 0.0) v = fma(jb.beta, *cp, v);
-            *cp = v;
-        }
+    if (*special) {
+        __syncthreads();
+        for (int e = tid; e < rows * cols; e += OZ_THREADS)
+            if (ea[e % rows] + eb[e / rows] >= OZ_NONFINITE / 2)
+                jb.C[m0 + e % rows + (size_t) (n0 + e / rows) * jb.ldc] = stash[e];
+    }
     __syncthreads();  // ea / eb are rewritten by the next tile
 }
 
@@ -368,7 +380,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_jobs_kernel(const GemmJ
     extern __shared__ __align__(1024) unsigned char oz_smem_raw[];
     __shared__ __align__(8) unsigned long long mbar[5];
     __shared__ uint32_t tmem_slot;
-    __shared__ int ea[OZ_TM], eb[OZ_TN];
+    __shared__ int ea[OZ_TM], eb[OZ_TN], special;
     unsigned char *stage0 = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(oz_smem_raw) + 1023) & ~uintptr_t(1023));
     const int total = sched[njobs];
@@ -391,7 +403,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) oz_gemm_jobs_kernel(const GemmJ
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int lo = job_of_tile(sched, njobs, w);
         const GemmJob jb = jobs[lo];
-        oz_tile(jb, w - sched[lo], stage0, tmem, bars, chunks, windows, ea, eb);
+        oz_tile(jb, w - sched[lo], stage0, tmem, bars, chunks, windows, ea, eb, &special);
     }
     __syncthreads();
     if ((threadIdx.x >> 5) == 0) tc::tmem_free(tmem, OZ_TMEM_COLS);
