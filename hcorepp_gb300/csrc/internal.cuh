@@ -254,8 +254,9 @@ struct Workspace {
     // Update processed by CTA `b` of the QR / core / Q-application launches: largest first, so the
     // long updates of a launch start at once instead of after the short ones.
     __device__ int heavy(int b) const { return order ? order[b] : b; }
-    // Key of an update in `order` (descending): its stack width when C is compressed.  Both fields are written by
-    // the plan kernel only, so the key is stable while the heavy stages run.
+    // Key of an update in `order` (descending): its stack width when C is compressed.  The searches below hold only while
+    // META_K and META_CKIND stand still: from launch_order to the end of that recompression.  The sketch passes of
+    // the learned form rewrite both in between, and launch_order runs again before each of their recompressions.
     __device__ int key(int slot) const {
         const int *m = meta + (size_t) slot * META_INTS;
         return m[META_CKIND] ? m[META_K] : 0;
@@ -303,7 +304,7 @@ struct Params {
 constexpr int SKETCH_MAX_PCT = 50;
 
 // Default of Params::precond_min: a 16-column core is about where the single-precision sweeps and the corrections
-// cost what the FP64 sweeps do (25 columns: 400 kcycles against 930; 15 columns: 250 either way).
+// cost what the FP64 sweeps do (25 columns: 348 kcycles against 930; 15 columns: 250 either way).
 constexpr int PRECOND_MIN_COLS = 16;
 
 // ---- launchers (stream-ordered, asynchronous) ----
@@ -311,7 +312,8 @@ void launch_plan(const DevUpdate *ups, int n, double alpha, double beta, Workspa
                  cudaStream_t st);
 void launch_stack(const DevUpdate *ups, int n, double alpha, double beta, Workspace ws, cudaStream_t st);
 // ws.order <- updates sorted by decreasing stack width k (0 for a dense C; ties by index); needs
-// ws.order != nullptr.  The key ignores the status, so it cannot change while the heavy stages run.
+// ws.order != nullptr.  Run before every recompression (Workspace::key); the key ignores the status, which
+// the core may change.
 void launch_order(int n, Workspace ws, cudaStream_t st);
 // out[i] = *ptrs[i] (device rank ints gathered for one host read).
 void launch_gather_ranks(const int *const *ptrs, int n, int *out, cudaStream_t st);

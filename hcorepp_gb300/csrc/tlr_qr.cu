@@ -4,8 +4,8 @@
 // (src/operators/concrete/Compressed.cpp:353, :384, :551, :611; LAPACK dgeqrf/dorgqr semantics:
 // R on and above the diagonal, unit-lower reflectors below it, tau_j = 2 / (v_j^T v_j)).
 //
-// Plain form: one CTA per matrix, or a cluster of up to eight while SMs are idle and for the wide updates.  The matrix stays in device memory (L2-resident working
-// set); each panel of QR_NB columns is staged in shared memory and factored there with SIMT FP64
+// Plain form: one CTA per matrix, or a cluster of up to eight while SMs are idle and for the wide updates.  The matrix
+// stays in device memory (L2-resident working set); each panel of QR_NB columns is staged in shared memory and factored there with SIMT FP64
 // and warp-shuffle norms; the compact-WY factor T (Q_panel = I - V T V^T, LAPACK dlarft) is kept
 // for the later Q application; the trailing update A <- (I - V T^T V^T) A is two FP64
 // tensor-core (DMMA) products with V and W = V^T A staged in shared memory.

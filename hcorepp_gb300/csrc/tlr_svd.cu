@@ -15,8 +15,8 @@
 // reference's (omp/kernels.cpp:82-104) applied to the sorted sigma.
 //
 // Measured (1.06 TFLOP/s FP64 pipe): the sweeps of a 200-column core of stack width 215 took 72,500 kcycles
-// on one SM, 4,970 on its cluster of eight; of a 25-column core 930, now 400, four to an SM; the pivoted QR
-// 9,970 -> 2,140 and 274 -> 229.
+// on one SM, 4,970 on its cluster of eight; of a 25-column core 930, now 348, four to an SM; the pivoted QR
+// 9,970 -> 2,140 and 274 -> 236.
 #include <algorithm>
 #include <cfloat>
 
@@ -1516,7 +1516,7 @@ __device__ __forceinline__ int core_aux_doubles(const Workspace &ws, int slot) {
 }
 
 // CTA of SVD_THREADS threads, in one of three team layouts chosen by the update's stack width k: heavy (k > k_heavy:
-// more than half of the shared memory, the preconditioner's columns included) — the whole CTA; light
+// more than half of the shared memory, the preconditioner's columns included: 115 to 166) — the whole CTA; light
 // (kthr4 < k <= k_heavy) — two half-CTA teams of SVD_THREADS / 2 threads, one update each, each with half
 // of the shared memory and its own named barrier; small (k <= kthr4: the core fits a quarter) — four teams
 // of SVD_THREADS / 4 threads.  Small cores are latency-bound (per-step barriers, dependent FP64 chains), so
