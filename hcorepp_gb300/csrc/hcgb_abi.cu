@@ -61,6 +61,8 @@ struct hcgb_context {
     // per-matrix operations (hcgb_d*)
     void *be_scratch = nullptr;
     size_t be_scratch_bytes = 0;
+    void *potrf_keep = nullptr;  // hcgb_potrf's alone: it returns with nothing in flight, on whatever stream
+    size_t potrf_keep_bytes = 0;
     // CUDA graph of the last hcgb_tlr_gemm (hcgb_set_graph)
     bool graph_mode = false;
     cudaGraphExec_t graph_exec = nullptr;
@@ -429,6 +431,7 @@ int hcgb_context_destroy(hcgb_context *ctx) {
     if (ctx->pack_desc) cudaFree(ctx->pack_desc);
     if (ctx->tile_info) cudaFree(ctx->tile_info);
     if (ctx->be_scratch) cudaFree(ctx->be_scratch);
+    if (ctx->potrf_keep) cudaFree(ctx->potrf_keep);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->capture_stream) cudaStreamDestroy(ctx->capture_stream);
     if (ctx->graph_desc) cudaFree(ctx->graph_desc);
@@ -1154,19 +1157,30 @@ extern "C" int hcgb_potrf(hcgb_context *ctx, int uplo, int n, double *A, int lda
         if (info) *info = 0;
         return HCGB_OK;
     }
-    const size_t keep_bytes = sizeof(double) * (size_t) n * n;
-    int rc = ensure_device(ctx, &ctx->be_scratch, &ctx->be_scratch_bytes, keep_bytes + sizeof(int));
+    // The copy of the triangle: tiles' in the context, that of a large matrix for this call alone (and without one, if
+    // memory is that short, a failure leaves the columns from the failing one on partly updated).
+    constexpr size_t most_kept = size_t(64) << 20;
+    const size_t bytes = sizeof(double) * (size_t) n * n, kept = bytes <= most_kept ? bytes : 0;
+    int rc = ensure_device(ctx, &ctx->potrf_keep, &ctx->potrf_keep_bytes, kept + sizeof(int));
     if (rc) return rc;
-    auto *keep = static_cast<double *>(ctx->be_scratch);
-    int *dinfo = reinterpret_cast<int *>(static_cast<char *>(ctx->be_scratch) + keep_bytes);
+    double *keep = static_cast<double *>(ctx->potrf_keep), *large = nullptr;
+    int *dinfo = reinterpret_cast<int *>(static_cast<char *>(ctx->potrf_keep) + kept);
+    if (!kept) {
+        if (cudaMalloc(&large, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            large = nullptr;
+        }
+        keep = large;
+    }
     launch_potrf(A, n, lda, uplo, dinfo, keep, ctx->stream);
     int h = 0;
     cudaError_t e = cudaMemcpyAsync(&h, dinfo, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess && h) {
+    if (e == cudaSuccess && h && keep) {
         launch_potrf_restore(A, n, lda, uplo, h, keep, ctx->stream);
         e = cudaStreamSynchronize(ctx->stream);
     }
+    if (large) cudaFree(large);
     if (e != cudaSuccess) return fail(ctx, HCGB_CUDA_ERROR, std::string("hcgb_potrf: ") + cudaGetErrorString(e));
     if (info) *info = h;
     return HCGB_OK;

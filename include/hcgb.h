@@ -247,7 +247,8 @@ typedef enum { HCGB_NONUNIT = 0, HCGB_UNIT = 1 } hcgb_diag;
  * replaces HCoreKernels::potrf (src/kernels/cuda/CudaKernels.cu:1019-1049, omp/kernels.cpp:234-243).
  * Synchronous; *info (if not NULL) receives 0 or the order j of the first non-positive minor, when the
  * first j - 1 columns of the factor are finished and the rest of the triangle is as it was given.
- * Keeps a copy of the triangle in the context's scratch (n * n doubles). */
+ * Takes a copy of the triangle for that (n * n doubles, kept in the context up to 64 MiB); where no memory
+ * for it is left, the rest is partly updated. */
 int hcgb_potrf(hcgb_context *ctx, int uplo, int n, double *A, int lda, int *info);
 /* op(A) X = alpha B (HCGB_LEFT) or X op(A) = alpha B (HCGB_RIGHT), X overwriting B (m x n);
  * BLAS dtrsm semantics; replaces HCoreKernels::trsm (src/kernels/cuda/kernels.cpp:290-298).

@@ -220,3 +220,25 @@ def test_potrf_stops_at_the_failing_column(T, n, bad, uplo):
     low = np.tril(np.ones((n, bad), dtype=bool))
     err = np.abs(l @ l[:bad].T - a[:, :bad])
     assert np.all(err[low] <= 2 * (n + 2) * EPS * (np.abs(l) @ np.abs(l[:bad]).T)[low])
+
+
+def test_potrf_of_a_large_matrix_stops_at_the_failing_column(T):
+    """Beyond the copy that a context keeps (64 MiB): the same after a failure, and no memory is held afterwards."""
+    import torch
+    n, bad = 3100, 2500
+    a = np.eye(n) * 4.0 + 1.0
+    a[bad, bad] = -5.0
+    _potrf(T, np.eye(8), 0)
+    torch.cuda.synchronize()
+    info, out = _potrf(T, np.tril(a), 0)
+    assert info == bad + 1
+    np.testing.assert_array_equal(out[:, bad:], np.tril(a)[:, bad:])
+    l = np.tril(out[:, :bad])
+    low = np.tril(np.ones((n, bad), dtype=bool))
+    err = np.abs(l @ l[:bad].T - a[:, :bad])
+    assert np.all(err[low] <= 2 * (n + 2) * EPS * (np.abs(l) @ np.abs(l[:bad]).T)[low])
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    _potrf(T, np.tril(a), 0)
+    torch.cuda.empty_cache()
+    assert torch.cuda.mem_get_info()[0] >= free - (16 << 20)
